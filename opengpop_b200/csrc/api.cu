@@ -267,6 +267,7 @@ gpop_status gpop_create(const gpop_config* cfg_in, gpop_ctx** out)
     std::string err;
     if (!load_model(ctx->data_dir, cfg.gravity_degree, ctx->md, err))
         return fail(ctx, GPOP_ERR_DATA, err);
+    ctx->corr = corrector_model(ctx->md);
     if (const char* spl = std::getenv("GPOP_STEPS_PER_LAUNCH"))
         ctx->steps_per_launch = std::max(1, atoi(spl));
     if (const char* wm = std::getenv("GPOP_WALK_MODE"))

@@ -8,6 +8,7 @@
 // its steps) from a global queue ordered longest first, so the grid stays busy until the end.
 #include "batch.cuh"
 #include "common.cuh"
+#include "corrector.cuh"
 #include "frames.cuh"
 #include "gravity.cuh"
 #include "integrator.cuh"
@@ -19,9 +20,11 @@ namespace gpop {
 
 // Force model of one request (startup kernel, one lane per object).
 template <bool MIXED> struct ForceReq {
+    static constexpr bool kPositionOnly = true;
     GravSmem g;
     const double* gen_m;
     const double* prop_m;
+    __device__ __forceinline__ unsigned agree(unsigned bits) const { return bits; }
     __device__ __forceinline__ void prop(const double* r, const double*, int idx, double* a) const
     {
         gravity_gcrs1<MIXED>(g, prop_m + (size_t)idx * 9, r, a);
@@ -95,7 +98,7 @@ __global__ void __launch_bounds__(256) batch_startup_kernel(TableSrc ts, BatchAr
 #define GPOP_BATCH_PAIRS 1
 #endif
 constexpr bool kBatchPairs = GPOP_BATCH_PAIRS != 0;
-// Two-object items park the corrector's constants (s1, s2, prev, a7: 12 doubles per object) in
+// Two-object items park the corrector's constants (as in gj8_kernel: 12 doubles per object) in
 // shared memory while the gravity walk runs, as gj8_kernel does, when that fits beside the table.
 #ifndef GPOP_BATCH_STAGE
 #define GPOP_BATCH_STAGE 1
@@ -112,11 +115,11 @@ constexpr bool kBatchPlain = GPOP_BATCH_PLAIN != 0;
 // One work item on one warp: K = 2 objects per lane for single-lane items (up to 64 objects),
 // else one object per group of P lanes (up to 32 / P objects).
 template <bool MIXED, int K, bool STAGE, bool PAIRS>
-__device__ __forceinline__ void run_item(const GravSmem& g0, const BatchArgs& a, const BatchItem& it,
+__device__ __forceinline__ void run_item(const GravSmem& g0, const CorrModel& cm, const BatchArgs& a, const BatchItem& it,
     const BatchReq& rq, int lane, double* stage)
 {
     constexpr bool kStage = K == 2 && STAGE;
-    // staged value q (0..3: s1, s2, prev, a7) of object k, axis j
+    // staged value q (0..3: s2, last, prev, s1) of object k, axis j
     auto slot = [&](int q, int k, int j) { return stage + (size_t)((q * K + k) * 3 + j) * blockDim.x; };
     const int64_t n = a.n_obj;
     double* st = a.state;
@@ -156,7 +159,7 @@ __device__ __forceinline__ void run_item(const GravSmem& g0, const BatchArgs& a,
             continue;
         }
         const int ring0 = (step - 5) % 9;
-        double s1[K][3], s2[K][3], prev[K][3], a7[K][3], a8[K][3];
+        double s1[K][3], s2[K][3], prev[K][3], a7[K][3], last[K][3], a8[K][3]; // as gj8_kernel
 #pragma unroll
         for (int k = 0; k < K; ++k) {
             double hist[9][3];
@@ -189,16 +192,18 @@ __device__ __forceinline__ void run_item(const GravSmem& g0, const BatchArgs& a,
                 s2[k][j] = c2;
                 prev[k][j] = s[k][j];
                 a7[k][j] = hist[8][j];
+                last[k][j] = r[k][j];
                 if constexpr (kStage) {
-                    st_stage(slot(0, k, j), s1[k][j]);
-                    st_stage(slot(1, k, j), s2[k][j]);
+                    st_stage(slot(0, k, j), s2[k][j]);
+                    st_stage(slot(1, k, j), last[k][j]);
                     st_stage(slot(2, k, j), prev[k][j]);
-                    st_stage(slot(3, k, j), a7[k][j]);
+                    st_stage(slot(3, k, j), s1[k][j]);
                 }
             }
         }
         const double* M = rq.prop_m + (size_t)(step + 4) * 9;
-        for (int itc = 0; itc < a.ncorr; ++itc) {
+        bool done[K] = {}, fast[K] = {};
+        for (int itc = 0; itc < a.ncorr; ++itc) { // as gj8_kernel
             if constexpr (K == 2 && PAIRS && kBatchPlain) {
                 gravity_gcrs<MIXED, 2>(g, M, r, a8); // the plain table: gj8_kernel's walk
             } else if constexpr (K == 2 && PAIRS) {
@@ -211,21 +216,50 @@ __device__ __forceinline__ void run_item(const GravSmem& g0, const BatchArgs& a,
             } else {
                 gravity_gcrs_lk<MIXED, K>(g, sl, P, M, r, a8, 0xffffffffu);
             }
+            bool all = true;
 #pragma unroll
-            for (int k = 0; k < K; ++k)
+            for (int k = 0; k < K; ++k) {
+                if (!done[k]) {
 #pragma unroll
-                for (int j = 0; j < 3; ++j) {
-                    if constexpr (kStage) {
-                        s1[k][j] = ld_stage(slot(0, k, j));
-                        s2[k][j] = ld_stage(slot(1, k, j));
-                        prev[k][j] = ld_stage(slot(2, k, j));
-                        a7[k][j] = ld_stage(slot(3, k, j));
+                    for (int j = 0; j < 3; ++j) {
+                        if constexpr (kStage) {
+                            s2[k][j] = ld_stage(slot(0, k, j));
+                            last[k][j] = ld_stage(slot(1, k, j));
+                        }
                     }
-                    s[k][j] = prev[k][j] + (a8[k][j] + a7[k][j]) / 2;
-                    v[k][j] = h * (s1[k][j] + a8[k][j] * c_SA[8][8] + s[k][j]);
-                    r[k][j] = h * h * (s2[k][j] + a8[k][j] * c_GJ[8][8] + S[k][j]);
+                    done[k] = correct_position(cm, h, itc, a.ncorr, s2[k], S[k], a8[k], last[k], fast[k]);
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) {
+                        if constexpr (kStage) {
+                            st_stage(slot(1, k, j), last[k][j]);
+                            if (done[k])
+                                st_stage(slot(0, k, j), a8[k][j]);
+                        } else if (done[k]) {
+                            s2[k][j] = a8[k][j];
+                        }
+                    }
                 }
+                all = all && done[k];
+#pragma unroll
+                for (int j = 0; j < 3; ++j)
+                    r[k][j] = kStage ? ld_stage(slot(1, k, j)) : last[k][j];
+            }
+            if (__all_sync(0xffffffffu, all)) // the lane walk's shuffles name the whole warp
+                break;
         }
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                a8[k][j] = kStage ? ld_stage(slot(0, k, j)) : s2[k][j];
+                if constexpr (kStage) {
+                    prev[k][j] = ld_stage(slot(2, k, j));
+                    s1[k][j] = ld_stage(slot(3, k, j));
+                    a7[k][j] = __ldcg(st + (kHist + (ring0 + 8 - (ring0 > 0 ? 9 : 0)) * 3 + j) * n + o[k]);
+                }
+                s[k][j] = prev[k][j] + (a8[k][j] + a7[k][j]) / 2;
+                v[k][j] = h * (s1[k][j] + a8[k][j] * c_SA[8][8] + s[k][j]);
+            }
 #pragma unroll
         for (int k = 0; k < K; ++k)
             if (lead && valid[k])
@@ -273,12 +307,12 @@ __global__ void __launch_bounds__(256, 1) batch_gj8_kernel(TableSrc ts, BatchArg
         const BatchItem it = a.items[item];
         const BatchReq rq = a.reqs[it.req];
         if constexpr (kPlain) { // every item has one lane per object
-            run_item<MIXED, 2, STAGE, PAIRS>(g0, a, it, rq, lane, stage);
+            run_item<MIXED, 2, STAGE, PAIRS>(g0, ts.corr, a, it, rq, lane, stage);
         } else {
             if (rq.lpo == 1)
-                run_item<MIXED, 2, STAGE, PAIRS>(g0, a, it, rq, lane, stage);
+                run_item<MIXED, 2, STAGE, PAIRS>(g0, ts.corr, a, it, rq, lane, stage);
             else
-                run_item<MIXED, 1, false, false>(g0, a, it, rq, lane, stage);
+                run_item<MIXED, 1, false, false>(g0, ts.corr, a, it, rq, lane, stage);
         }
     }
 }

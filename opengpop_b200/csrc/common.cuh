@@ -94,4 +94,10 @@ __device__ __forceinline__ double ld_stage(const double* p)
     return v;
 }
 
+// Whether two values have the same bit pattern (NaN equals itself, +0 differs from -0).
+__device__ __forceinline__ bool same_bits(double a, double b)
+{
+    return __double_as_longlong(a) == __double_as_longlong(b);
+}
+
 } // namespace gpop

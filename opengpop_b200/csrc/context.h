@@ -75,6 +75,7 @@ struct gpop_ctx {
     std::string data_dir;
     std::string err;
     gpop::ModelData md;
+    gpop::CorrModel corr;
     int num_sms = 148;
     int steps_per_launch = 64;
     int block_override = 0; // GJ8 block size chosen by the tuner (0 = default policy)
@@ -118,6 +119,7 @@ struct gpop_ctx {
         ts.bytes = mixed_mode ? lane_mixed_bytes : lane64_bytes;
         ts.off32 = mixed_mode ? lane_mixed_off32 : lane64_off32;
         ts.wait_spins = first_wait_spins;
+        ts.corr = corr;
         return ts;
     }
 
@@ -138,6 +140,7 @@ struct gpop_ctx {
             ts.off32 = 0;
         }
         ts.wait_spins = first_wait_spins;
+        ts.corr = corr;
         return ts;
     }
 };

@@ -2,10 +2,13 @@
 // shared by the single-request, batched and variational kernels. A force model F provides
 //   gen(r, v, step, k, a)  -- acceleration at RK8 stage k of startup step `step` (+-1..4)
 //   prop(r, v, idx, a)     -- acceleration at propagation epoch index idx (t = (idx - 4) h)
+//   kPositionOnly          -- whether a depends on r (and the epoch) alone
+//   agree(bits)            -- bits set for any of the threads that evaluate together
 // The state type T is double, or a value with a tangent (variational equations): the startup is
 // linear in the state apart from the force evaluations, so only + - and scaling by constants are
 // applied to T.
 #pragma once
+#include "common.cuh"
 #include "gj8_tables.cuh"
 
 namespace gpop {
@@ -92,12 +95,16 @@ template <class T> __device__ inline void corrector_all_s(StartupMatsT<T>& m)
         }
 }
 
-// StartupCorrector::Correct (gpu_startup.cu:247-294)
-template <class F, class T> __device__ void corrector_correct(const F& f, double h, StartupMatsT<T>& m)
+// StartupCorrector::Correct (gpu_startup.cu:247-294). Under a force that depends on the position
+// alone, a column whose new position has the old one's bits keeps its acceleration (an evaluation
+// there would return the same bits). Returns whether any column moved: if none did, every further
+// pass returns this pass's bits.
+template <class F, class T> __device__ bool corrector_correct(const F& f, double h, StartupMatsT<T>& m)
 {
     corrector_s0(h, m);
     corrector_all_s(m);
     const double h2 = h * h;
+    unsigned moved = 0;
     for (int c = 0; c < 9; ++c) {
         if (c == 4)
             continue; // the epoch column is restored
@@ -108,10 +115,17 @@ template <class F, class T> __device__ void corrector_correct(const F& f, double
                 sr = fma(m.a[k][j], c_GJ[c][k], sr);
             }
             m.v[c][j] = h * (sv + m.s[c][j]);
-            m.r[c][j] = h2 * (sr + m.S[c][j]);
+            const T rn = h2 * (sr + m.S[c][j]);
+            if (!F::kPositionOnly || !same_bits(rn, m.r[c][j]))
+                moved |= 1u << c;
+            m.r[c][j] = rn;
         }
     }
-    corrector_accel(f, m, false);
+    moved = f.agree(moved);
+    for (int c = 0; c < 9; ++c)
+        if (moved >> c & 1)
+            f.prop(m.r[c], m.v[c], c, m.a[c]);
+    return moved != 0;
 }
 
 template <class F, class T>
@@ -132,13 +146,15 @@ __device__ void run_startup(const F& f, double h, int ncorr, const T* r0, const 
         return;
     corrector_accel(f, m, true);
     for (int i = 0; i < ncorr; ++i)
-        corrector_correct(f, h, m);
+        if (!corrector_correct(f, h, m))
+            break;
 }
 
 // ---- the same startup for two objects in lockstep (the split block's startup kernel) ----
 // F2 provides gen2(r, v, step, k, a) and prop2(r, v, idx, a) over both objects at once
-// ([2][3] arrays); those may hold block-wide barriers, so every thread of a block makes the same
-// calls in the same order (the control flow below depends on no data). Per object the arithmetic
+// ([2][3] arrays), and any2(x), whether x holds for any thread; those may hold block-wide barriers,
+// so every thread of a block makes the same calls in the same order (the control flow below depends
+// on any2's answers and on no other data). Per object the arithmetic
 // is that of rk8_step, corrector_correct and run_startup. A thread that carries no objects
 // (active false) makes the same force calls and skips the arithmetic around them.
 template <class F2>
@@ -194,28 +210,26 @@ __device__ void rk8_step2(const F2& f, double h, int step, StartupMats (&m)[2], 
 }
 
 template <class F2>
-__device__ void corrector_accel2(const F2& f, StartupMats (&m)[2], bool epoch, bool active)
+__device__ void corrector_accel2(const F2& f, StartupMats (&m)[2], int i, bool active)
 {
-    for (int i = 0; i < 9; ++i) {
-        if (i == 4 && !epoch)
-            continue; // the same for every thread: no evaluation, no barrier
-        double r[2][3] = {}, v[2][3] = {}, acc[2][3];
-        for (int o = 0; o < 2 && active; ++o)
-            for (int j = 0; j < 3; ++j) {
-                r[o][j] = m[o].r[i][j];
-                v[o][j] = m[o].v[i][j];
-            }
-        f.prop2(r, v, i, acc);
-        for (int o = 0; o < 2 && active; ++o)
-            for (int j = 0; j < 3; ++j)
-                m[o].a[i][j] = acc[o][j];
-    }
+    double r[2][3] = {}, v[2][3] = {}, acc[2][3];
+    for (int o = 0; o < 2 && active; ++o)
+        for (int j = 0; j < 3; ++j) {
+            r[o][j] = m[o].r[i][j];
+            v[o][j] = m[o].v[i][j];
+        }
+    f.prop2(r, v, i, acc);
+    for (int o = 0; o < 2 && active; ++o)
+        for (int j = 0; j < 3; ++j)
+            m[o].a[i][j] = acc[o][j];
 }
 
+// As corrector_correct: a column is evaluated where it moved for any object of the block (any2).
 template <class F2>
-__device__ void corrector_correct2(const F2& f, double h, StartupMats (&m)[2], bool active)
+__device__ bool corrector_correct2(const F2& f, double h, StartupMats (&m)[2], bool active)
 {
     const double h2 = h * h;
+    unsigned moved = 0;
     for (int o = 0; o < 2 && active; ++o) {
         corrector_s0(h, m[o]);
         corrector_all_s(m[o]);
@@ -229,11 +243,21 @@ __device__ void corrector_correct2(const F2& f, double h, StartupMats (&m)[2], b
                     sr = fma(m[o].a[k][j], c_GJ[c][k], sr);
                 }
                 m[o].v[c][j] = h * (sv + m[o].s[c][j]);
-                m[o].r[c][j] = h2 * (sr + m[o].S[c][j]);
+                const double rn = h2 * (sr + m[o].S[c][j]);
+                if (!same_bits(rn, m[o].r[c][j]))
+                    moved |= 1u << c;
+                m[o].r[c][j] = rn;
             }
         }
     }
-    corrector_accel2(f, m, false, active);
+    bool any = false;
+    for (int c = 0; c < 9; ++c) {
+        if (c == 4 || !f.any2(moved >> c & 1)) // the same for every thread of the block
+            continue;
+        any = true;
+        corrector_accel2(f, m, c, active);
+    }
+    return any;
 }
 
 template <class F2>
@@ -255,9 +279,11 @@ __device__ void run_startup2(const F2& f, double h, int ncorr, const double (&r0
     }
     if (ncorr <= 0)
         return;
-    corrector_accel2(f, m, true, active);
+    for (int i = 0; i < 9; ++i)
+        corrector_accel2(f, m, i, active);
     for (int i = 0; i < ncorr; ++i)
-        corrector_correct2(f, h, m, active);
+        if (!corrector_correct2(f, h, m, active)) // the same for every thread of the block
+            break;
 }
 
 } // namespace gpop

@@ -18,6 +18,7 @@ struct TableSrc {
     // spins of the first bounded wait on the staging copy (2^22, about a second; a test setting
     // lowers it to make the wait give up on purpose)
     uint32_t wait_spins = 1u << 22;
+    CorrModel corr;
 };
 
 // Byte offset, in a kernel's dynamic shared memory, of what follows a staged table (the 128-byte

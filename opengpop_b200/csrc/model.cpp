@@ -1,9 +1,9 @@
 // model.cpp -- model data loaders and gravity-table builder (host side of the product).
 #include "model.h"
 
-#include <cstring>
-
+#include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <fstream>
 #include <sstream>
 
@@ -196,6 +196,29 @@ bool load_model(const std::string& dir, int degree, ModelData& out, std::string&
         && load_nutation(base + "IAU2000_R06_NutObl.txt", out.obl0, out.obl1, err)
         && load_eop(base + "IAU2000A_EOP.txt", out.eop, err)
         && load_leap(base + "leap-seconds.list", out.leap_mjd, out.leap_val, err);
+}
+
+CorrModel corrector_model(const ModelData& md)
+{
+    CorrModel c;
+    c.gm = (float)md.gm;
+    const double j2 = md.degree >= 2 ? -std::sqrt(5.0) * md.C[tri(2, 0)] : 0.0;
+    c.j2 = (float)(1.5 * j2 * md.radius * md.radius);
+    // Gradient of the terms left out over that of GM/r (2 GM/r^3), at 1.02 R: the root mean square of
+    // a normalised degree-n term's gradient is about (n+1)(n+2)/2 of its coefficients', taken four
+    // times. (JGM3 to 70x70: 5.8e-4 at 1.02 R, 1.9e-4 at 1.1 R.)
+    double sum = 0.0;
+    for (int n = 2; n <= md.degree; ++n)
+        for (int m = n == 2 ? 1 : 0; m <= n; ++m) {
+            const double f = 0.5 * (n + 1) * (n + 2) * std::pow(1.02, -n);
+            sum += f * f * (md.C[tri(n, m)] * md.C[tri(n, m)] + md.S[tri(n, m)] * md.S[tri(n, m)]);
+        }
+    const double kappa = std::max(4.0 * std::sqrt(sum), 1e-5);
+    // kappa 2 GM/r^3 near r <= a tenth of a last bit of GM/r^2
+    const bool usable = kappa < 0.02 && std::fabs(j2) < 0.01;
+    c.near = usable ? (float)(0.05 * std::ldexp(1.0, -53) / kappa) : 0.f;
+    c.low = usable ? (float)(1.02 * md.radius) : INFINITY;
+    return c;
 }
 
 void build_gravity_tables(const ModelData& md, std::vector<GravEntry64>& t64, std::vector<GravEntry32>& t32)

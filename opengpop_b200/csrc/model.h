@@ -38,6 +38,13 @@ struct ModelData {
 // fills `err` on failure (missing file, malformed header, non-static model).
 bool load_model(const std::string& dir, int degree, ModelData& out, std::string& err);
 
+// What the corrector's end (corrector.cuh) needs of the field: GM, 1.5 J2 R^2, the radius from which
+// it may use the Jacobian of these two terms, and the largest step it may end with, relative to r.
+struct CorrModel {
+    float gm = 0, j2 = 0, low = 0, near = 0;
+};
+CorrModel corrector_model(const ModelData& md);
+
 // Gravity table entry, one per (n, m) with n >= m, stored column by column (m outer, n = m..L).
 // With the rescaled derived-Legendre recursion
 //   Q(m,m) = q^m, Q(m+1,m) = u Q(m,m), Q(n,m) = u Q(n-1,m) - c(n,m) w Q(n-2,m)

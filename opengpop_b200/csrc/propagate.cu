@@ -4,6 +4,7 @@
 // many steps with no grid-wide synchronisation. The GJ8 acceleration history lives in a 9-slot
 // ring in global memory (SoA, coalesced); the working state of a step stays in registers.
 #include "common.cuh"
+#include "corrector.cuh"
 #include "gravity.cuh"
 #include "gj8_tables.cuh"
 #include "integrator.cuh"
@@ -18,11 +19,13 @@ namespace gpop {
 // COMP: mixed precision with compensated FP32 sums (GPOP_MIXED_COMPENSATED).
 template <bool MIXED, bool COMP = false> struct ForceGravity {
     static constexpr bool kTable = true;
+    static constexpr bool kPositionOnly = true; // the acceleration depends on r (and the epoch) alone
     static constexpr bool kMixed = MIXED;
     static constexpr bool kComp = COMP;
     GravSmem g;
     const double* gen_m;
     const double* prop_m;
+    __device__ __forceinline__ unsigned agree(unsigned bits) const { return bits; }
     // ForceModel::ComputePropagationAcceleration (force_model.cu:91-109): epoch index idx
     __device__ __forceinline__ void prop(const double* r, const double*, int idx, double* a) const
     {
@@ -46,9 +49,11 @@ template <bool MIXED, bool COMP = false> struct ForceGravity {
 // mock's time rules (unit_tests/include/mock_force_model.cuh:65-106).
 struct ForceAnalytic {
     static constexpr bool kTable = false;
+    static constexpr bool kPositionOnly = false;
     static constexpr bool kMixed = false;
     int kind;
     double h;
+    __device__ __forceinline__ unsigned agree(unsigned bits) const { return bits; }
     __device__ void eval(const double* p, const double* v, double t, double* a) const
     {
         double val = 0.0;
@@ -182,8 +187,10 @@ __global__ void __launch_bounds__(256) startup_kernel(F f, TableSrc ts, PropArgs
 // K objects per thread: object k of thread g is g + k * (threads in the grid); every gravity
 // evaluation of a step runs the K objects in lockstep on the same table entries.
 //
-// With a gravity table, the corrector's constants of a step (s1, s2, prev, a7: 12 doubles per
-// object) and S wait in shared memory while the gravity walk runs, which leaves the walk the
+// Under gravity the corrector passes end as correct_position (corrector.cuh) says.
+//
+// With a gravity table, the corrector's constants of a step (s1, s2, prev and the position: 12 doubles
+// per object) and S wait in shared memory while the gravity walk runs, which leaves the walk the
 // registers they would hold (two objects, 65,536 objects at 70x70 on B200, with the paired column
 // walks: mixed 125.5 -> 131.5 M object-steps/s, FP64 72.3 -> 73.8 M).
 // Largest block of the one-object-per-thread kernel (its register budget is 65,536 / this; at 256
@@ -199,7 +206,7 @@ constexpr int kOneObjectBlock = GPOP_ONE_OBJECT_BLOCK;
 #ifndef GPOP_STAGE_FP64
 #define GPOP_STAGE_FP64 1
 #endif
-constexpr int kStageDoubles = 15; // per object: s1, s2, prev, a7, S (3 each)
+constexpr int kStageDoubles = 15; // per object: s2, last, prev, s1, S (3 each)
 template <class F> constexpr bool stage_corrector()
 {
     return F::kTable && (F::kMixed || GPOP_STAGE_FP64 != 0) && GPOP_STAGE_CORRECTOR != 0;
@@ -409,7 +416,7 @@ __global__ void __launch_bounds__(K == 1 ? kOneObjectBlock : 256, 1) gj8_kernel(
             return;
         stage = reinterpret_cast<double*>(smem + stage_offset(ts)) + threadIdx.x;
     }
-    // staged value q (0..4: s1, s2, prev, a7, S) of object k, axis j
+    // staged value q (0..4: s2, last, prev, s1, S) of object k, axis j
     auto slot = [&](int q, int k, int j) { return stage + (size_t)((q * K + k) * 3 + j) * blockDim.x; };
     const int64_t n = a.n; // the state's stride; this launch runs objects [lo, lo + cnt)
     const int64_t lo = a.obj_lo, cnt = (a.obj_hi < 0 ? n : a.obj_hi) - lo;
@@ -468,6 +475,7 @@ __global__ void __launch_bounds__(K == 1 ? kOneObjectBlock : 256, 1) gj8_kernel(
         } else {
             const int ring0 = (step - 5) % 9;
             double s1[K][3], s2[K][3], prev[K][3], a7[K][3], a8[K][3];
+            double last[K][3]; // the position an object's next evaluation takes
 #pragma unroll
             for (int k = 0; k < K; ++k) {
                 double hist[9][3];
@@ -502,46 +510,96 @@ __global__ void __launch_bounds__(K == 1 ? kOneObjectBlock : 256, 1) gj8_kernel(
                     s2[k][j] = c2;
                     prev[k][j] = s[k][j];
                     a7[k][j] = hist[8][j];
+                    last[k][j] = r[k][j];
                     if constexpr (kStage) {
-                        st_stage(slot(0, k, j), s1[k][j]);
-                        st_stage(slot(1, k, j), s2[k][j]);
+                        st_stage(slot(0, k, j), s2[k][j]);
+                        st_stage(slot(1, k, j), last[k][j]);
                         st_stage(slot(2, k, j), prev[k][j]);
-                        st_stage(slot(3, k, j), a7[k][j]);
+                        st_stage(slot(3, k, j), s1[k][j]);
                         st_stage(slot(4, k, j), S[k][j]);
                     }
                 }
             }
             const int idx = step + 4;
-            if constexpr (SPLIT != kSplitNone)
-                split_eval<F::kMixed, SPLIT>(f.g, f.prop_m + (size_t)idx * 9, a, owner, live, obj, r,
-                    a8, xsmem);
-            else
-                f.template prop_k<K>(r, v, idx, a8);
-            // Corrector: the first pass reuses the predictor's evaluation at the unchanged
-            // position (bit-identical to the reference's repeated call).
-            for (int it = 0; it < a.ncorr; ++it) {
-                if (it > 0) {
+            if constexpr (F::kTable) {
+                // Evaluate and correct until every object of the thread (split block: of the block)
+                // is done; s and v follow from the last acceleration. A finished object keeps its
+                // position and acceleration, whatever its neighbours still do.
+                bool done[K], fast[K];
+#pragma unroll
+                for (int k = 0; k < K; ++k)
+                    done[k] = fast[k] = SPLIT != kSplitNone && !live[k];
+                for (int it = 0; it < a.ncorr; ++it) {
                     if constexpr (SPLIT != kSplitNone)
                         split_eval<F::kMixed, SPLIT>(f.g, f.prop_m + (size_t)idx * 9, a, owner, live,
                             obj, r, a8, xsmem);
                     else
                         f.template prop_k<K>(r, v, idx, a8);
+                    bool all = true;
+#pragma unroll
+                    for (int k = 0; k < K; ++k) {
+                        if (!done[k]) {
+#pragma unroll
+                            for (int j = 0; j < 3; ++j) {
+                                if constexpr (kStage) {
+                                    s2[k][j] = ld_stage(slot(0, k, j));
+                                    last[k][j] = ld_stage(slot(1, k, j));
+                                    S[k][j] = ld_stage(slot(4, k, j));
+                                }
+                            }
+                            done[k] = correct_position(ts.corr, h, it, a.ncorr, s2[k], S[k], a8[k],
+                                last[k], fast[k]);
+#pragma unroll
+                            for (int j = 0; j < 3; ++j) {
+                                if constexpr (kStage) {
+                                    st_stage(slot(1, k, j), last[k][j]);
+                                    if (done[k])
+                                        st_stage(slot(0, k, j), a8[k][j]);
+                                } else if (done[k]) {
+                                    s2[k][j] = a8[k][j]; // (not needed any more)
+                                }
+                            }
+                        }
+                        all = all && done[k];
+#pragma unroll
+                        for (int j = 0; j < 3; ++j) // read back: no position lives through the walk
+                            r[k][j] = kStage ? ld_stage(slot(1, k, j)) : last[k][j];
+                    }
+                    if constexpr (SPLIT != kSplitNone)
+                        all = __syncthreads_and(all);
+                    if (all)
+                        break;
                 }
 #pragma unroll
                 for (int k = 0; k < K; ++k)
 #pragma unroll
                     for (int j = 0; j < 3; ++j) {
-                        if constexpr (kStage) {
-                            s1[k][j] = ld_stage(slot(0, k, j));
-                            s2[k][j] = ld_stage(slot(1, k, j));
+                        a8[k][j] = kStage ? ld_stage(slot(0, k, j)) : s2[k][j];
+                        if constexpr (kStage) { // a7 is read from the ring again
                             prev[k][j] = ld_stage(slot(2, k, j));
-                            a7[k][j] = ld_stage(slot(3, k, j));
+                            s1[k][j] = ld_stage(slot(3, k, j));
                             S[k][j] = ld_stage(slot(4, k, j));
+                            a7[k][j] = __ldcg(st + (kHist + (ring0 + 8 - (ring0 > 0 ? 9 : 0)) * 3 + j) * n + obj[k]);
                         }
                         s[k][j] = prev[k][j] + (a8[k][j] + a7[k][j]) / 2;
                         v[k][j] = h * (s1[k][j] + a8[k][j] * c_SA[8][8] + s[k][j]);
-                        r[k][j] = h * h * (s2[k][j] + a8[k][j] * c_GJ[8][8] + S[k][j]);
                     }
+            } else {
+                f.template prop_k<K>(r, v, idx, a8);
+                // Corrector: the first pass reuses the predictor's evaluation at the unchanged
+                // position (bit-identical to the reference's repeated call).
+                for (int it = 0; it < a.ncorr; ++it) {
+                    if (it > 0)
+                        f.template prop_k<K>(r, v, idx, a8);
+#pragma unroll
+                    for (int k = 0; k < K; ++k)
+#pragma unroll
+                        for (int j = 0; j < 3; ++j) {
+                            s[k][j] = prev[k][j] + (a8[k][j] + a7[k][j]) / 2;
+                            v[k][j] = h * (s1[k][j] + a8[k][j] * c_SA[8][8] + s[k][j]);
+                            r[k][j] = h * h * (s2[k][j] + a8[k][j] * c_GJ[8][8] + S[k][j]);
+                        }
+                }
             }
 #pragma unroll
             for (int k = 0; k < K; ++k)
@@ -609,6 +667,8 @@ template <bool MIXED, int SPLIT> struct SplitForce2 {
     {
         split_eval<MIXED, SPLIT>(f.g, f.prop_m + (size_t)idx * 9, a, owner, live, obj, r, acc, xsmem);
     }
+    // the block evaluates together, so it decides together
+    __device__ __forceinline__ bool any2(bool need) const { return __syncthreads_or(need && owner); }
 };
 
 template <bool MIXED, int SPLIT>
@@ -691,7 +751,7 @@ __global__ void __launch_bounds__(kSplitBlock, 1) startup_split_kernel(ForceGrav
 // of group g is g + k * (groups in the grid). Used when the objects alone leave most warp slots of
 // the GPU empty. MAXT bounds the block (and so the registers a thread may hold): 512 for the many
 // lanes of few objects, 384 for two lanes per object, which then keeps its table loads in flight.
-// STAGE: the corrector's constants of a step (s1, s2, prev, a7, S) wait in shared memory during
+// STAGE: the corrector's constants of a step (as in gj8_kernel) wait in shared memory during
 // the gravity walks, one copy per lane group written by its lead lane, as in gj8_kernel (two
 // objects per lane group, FP64, 18,944 objects at four lanes: the walk at 254 registers waited on
 // its table loads, short_scoreboard 1.43 per issued instruction, FP64 pipe 59 % busy).
@@ -705,7 +765,7 @@ __global__ void __launch_bounds__(MAXT, 1) gj8_lanes_kernel(TableSrc ts, PropArg
     double* stage = nullptr;
     if constexpr (STAGE)
         stage = reinterpret_cast<double*>(smem + stage_offset(ts)) + threadIdx.x / P;
-    // staged value q (0..4: s1, s2, prev, a7, S) of object k, axis j, of this lane's group
+    // staged value q (0..4: s2, last, prev, s1, S) of object k, axis j, of this lane's group
     auto slot = [&](int q, int k, int j) { return stage + (size_t)((q * K + k) * 3 + j) * (blockDim.x / P); };
     const int64_t grp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / P;
     const int64_t groups = ((int64_t)gridDim.x * blockDim.x) / P;
@@ -713,6 +773,9 @@ __global__ void __launch_bounds__(MAXT, 1) gj8_lanes_kernel(TableSrc ts, PropArg
     const int l = lane & (P - 1);
     const int64_t n = a.n; // the state's stride; this launch runs objects [lo, hi)
     const int64_t lo = a.obj_lo, hi = a.obj_hi < 0 ? n : a.obj_hi;
+    const int in_warp = (int)blockDim.x - (int)(threadIdx.x & ~31u); // the block's last warp may be partial
+    const unsigned warp = __ballot_sync(in_warp >= 32 ? 0xffffffffu : (1u << in_warp) - 1u,
+        grp < hi - lo); // lanes that stay
     if (grp >= hi - lo)
         return; // whole groups leave: shuffles name the group only
     const unsigned mask = P == 32 ? 0xffffffffu : ((1u << P) - 1u) << (lane & ~(P - 1));
@@ -750,7 +813,7 @@ __global__ void __launch_bounds__(MAXT, 1) gj8_lanes_kernel(TableSrc ts, PropArg
                 }
         } else {
             const int ring0 = (step - 5) % 9;
-            double s1[K][3], s2[K][3], prev[K][3], a7[K][3], a8[K][3];
+            double s1[K][3], s2[K][3], prev[K][3], a7[K][3], last[K][3], a8[K][3]; // as gj8_kernel
 #pragma unroll
             for (int k = 0; k < K; ++k) {
                 double hist[9][3];
@@ -783,12 +846,13 @@ __global__ void __launch_bounds__(MAXT, 1) gj8_lanes_kernel(TableSrc ts, PropArg
                     s2[k][j] = c2;
                     prev[k][j] = s[k][j];
                     a7[k][j] = hist[8][j];
+                    last[k][j] = r[k][j];
                     if constexpr (STAGE) {
                         if (lead) {
-                            st_stage(slot(0, k, j), s1[k][j]);
-                            st_stage(slot(1, k, j), s2[k][j]);
+                            st_stage(slot(0, k, j), s2[k][j]);
+                            st_stage(slot(1, k, j), last[k][j]);
                             st_stage(slot(2, k, j), prev[k][j]);
-                            st_stage(slot(3, k, j), a7[k][j]);
+                            st_stage(slot(3, k, j), s1[k][j]);
                             st_stage(slot(4, k, j), S[k][j]);
                         }
                     }
@@ -797,27 +861,70 @@ __global__ void __launch_bounds__(MAXT, 1) gj8_lanes_kernel(TableSrc ts, PropArg
             if constexpr (STAGE)
                 __syncwarp(mask); // the lead's stores precede the group's loads
             const double* M = a.prop_m + (size_t)(step + 4) * 9;
-            for (int it = 0; it < a.ncorr; ++it) {
+            bool done[K] = {}, fast[K] = {};
+            for (int it = 0; it < a.ncorr; ++it) { // as gj8_kernel
                 // two columns at a time for one object per group at up to 384 threads a block (FP64
                 // 1,024 objects: 18.8 against 17.4 M object-steps/s); with two objects per group,
                 // or the 128 registers of 512-thread blocks, that spills (-9 %)
                 gravity_gcrs_lk<MIXED, K, K == 1 && MAXT <= 384>(g, l, P, M, r, a8, mask);
+                bool all = true;
+#pragma unroll
+                for (int k = 0; k < K; ++k) {
+                    if (!done[k]) { // the same for the lanes of a group
+#pragma unroll
+                        for (int j = 0; j < 3; ++j) {
+                            if constexpr (STAGE) {
+                                s2[k][j] = ld_stage(slot(0, k, j));
+                                last[k][j] = ld_stage(slot(1, k, j));
+                                S[k][j] = ld_stage(slot(4, k, j));
+                            }
+                        }
+                        if constexpr (STAGE)
+                            __syncwarp(mask); // the loads precede the lead's stores
+                        done[k] = correct_position(ts.corr, h, it, a.ncorr, s2[k], S[k], a8[k], last[k],
+                            fast[k]);
+#pragma unroll
+                        for (int j = 0; j < 3; ++j) {
+                            if constexpr (STAGE) {
+                                if (lead) {
+                                    st_stage(slot(1, k, j), last[k][j]);
+                                    if (done[k])
+                                        st_stage(slot(0, k, j), a8[k][j]);
+                                }
+                            } else if (done[k]) {
+                                s2[k][j] = a8[k][j];
+                            }
+                        }
+                    }
+                    all = all && done[k];
+                }
+                if constexpr (STAGE)
+                    __syncwarp(mask); // the lead's stores precede the group's loads
 #pragma unroll
                 for (int k = 0; k < K; ++k)
 #pragma unroll
-                    for (int j = 0; j < 3; ++j) {
-                        if constexpr (STAGE) {
-                            s1[k][j] = ld_stage(slot(0, k, j));
-                            s2[k][j] = ld_stage(slot(1, k, j));
-                            prev[k][j] = ld_stage(slot(2, k, j));
-                            a7[k][j] = ld_stage(slot(3, k, j));
-                            S[k][j] = ld_stage(slot(4, k, j));
-                        }
-                        s[k][j] = prev[k][j] + (a8[k][j] + a7[k][j]) / 2;
-                        v[k][j] = h * (s1[k][j] + a8[k][j] * c_SA[8][8] + s[k][j]);
-                        r[k][j] = h * h * (s2[k][j] + a8[k][j] * c_GJ[8][8] + S[k][j]);
-                    }
+                    for (int j = 0; j < 3; ++j)
+                        r[k][j] = STAGE ? ld_stage(slot(1, k, j)) : last[k][j];
+                if (all)
+                    break;
             }
+            __syncwarp(warp); // groups that were done earlier wait: the warp's walks stay converged
+#pragma unroll
+            for (int k = 0; k < K; ++k)
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    a8[k][j] = STAGE ? ld_stage(slot(0, k, j)) : s2[k][j];
+                    if constexpr (STAGE) {
+                        prev[k][j] = ld_stage(slot(2, k, j));
+                        s1[k][j] = ld_stage(slot(3, k, j));
+                        S[k][j] = ld_stage(slot(4, k, j));
+                        a7[k][j] = __ldcg(st + (kHist + (ring0 + 8 - (ring0 > 0 ? 9 : 0)) * 3 + j) * n + obj[k]);
+                    }
+                    s[k][j] = prev[k][j] + (a8[k][j] + a7[k][j]) / 2;
+                    v[k][j] = h * (s1[k][j] + a8[k][j] * c_SA[8][8] + s[k][j]);
+                }
+            if constexpr (STAGE)
+                __syncwarp(mask); // the loads precede the lead's stores of the next step
 #pragma unroll
             for (int k = 0; k < K; ++k)
 #pragma unroll

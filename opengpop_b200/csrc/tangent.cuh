@@ -3,6 +3,8 @@
 // sums, differences and scaling by constants; products of two tangents do not occur (the force
 // models supply a + J dr themselves).
 #pragma once
+#include "common.cuh"
+
 #include <cuda_runtime.h>
 
 namespace gpop {
@@ -31,6 +33,8 @@ __device__ __forceinline__ Tan& operator+=(Tan& a, Tan b)
 __device__ __forceinline__ double fma(double a, double b, double c) { return ::fma(a, b, c); }
 __device__ __forceinline__ Tan fma(double c, Tan a, Tan b) { return Tan(::fma(c, a.v, b.v), ::fma(c, a.d, b.d)); }
 __device__ __forceinline__ Tan fma(Tan a, double c, Tan b) { return Tan(::fma(a.v, c, b.v), ::fma(a.d, c, b.d)); }
+
+__device__ __forceinline__ bool same_bits(Tan a, Tan b) { return same_bits(a.v, b.v) && same_bits(a.d, b.d); }
 
 __device__ __forceinline__ double value(double x) { return x; }
 __device__ __forceinline__ double value(Tan x) { return x.v; }

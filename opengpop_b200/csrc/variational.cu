@@ -18,6 +18,7 @@
 // The reverse pass below applies the transposes of these maps in the opposite order, with J^T at
 // the last evaluation point r(K-1), recomputed from the checkpoint of the step's 64-step segment.
 #include "common.cuh"
+#include "corrector.cuh"
 #include "gj8_tables.cuh"
 #include "gravity.cuh"
 #include "hermite.cuh"
@@ -32,11 +33,14 @@ namespace {
 
 // Tangent force: a(r) and J(r) dr, epoch tables as in ForceGravity (force_model.cu:59-109).
 struct LaneForceTan {
+    static constexpr bool kPositionOnly = true;
     GravSmem g;
     int l, P;
     unsigned mask;
     const double* gen_m;
     const double* prop_m;
+    // the lanes carry different tangents and evaluate together
+    __device__ __forceinline__ unsigned agree(unsigned bits) const { return __reduce_or_sync(mask, bits); }
     __device__ __forceinline__ void eval(const double* M, const Tan* r, Tan* a) const
     {
         const double rv[3] = { r[0].v, r[1].v, r[2].v };
@@ -58,7 +62,7 @@ struct LaneForceTan {
 };
 
 // One GJ8 step (predict, then ncorr evaluate-correct passes) on a history held in logical order
-// (hist[8] newest). eval(r, a, pass) evaluates the force at r for corrector pass `pass`.
+// (hist[8] newest). eval(r, a) evaluates the force, a function of the position alone, at r.
 template <class T, class Eval>
 __device__ __forceinline__ void gj8_step(const Eval& eval, double h, int ncorr, T (&hist)[9][3],
     T (&s)[3], T (&S)[3], T (&r)[3], T (&v)[3])
@@ -88,13 +92,18 @@ __device__ __forceinline__ void gj8_step(const Eval& eval, double h, int ncorr, 
         a8[j] = 0.0;
     }
     for (int it = 0; it < ncorr; ++it) { // GpuPropagator::Correct (gpu_propagator.cu:61-119)
-        eval(r, a8, it);
+        eval(r, a8);
+        bool same = true;
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
             s[j] = prev[j] + (a8[j] + a7[j]) / 2;
             v[j] = h * (s1[j] + a8[j] * c_SA[8][8] + s[j]);
-            r[j] = h * h * (s2[j] + a8[j] * c_GJ[8][8] + S[j]);
+            const T rn = h * h * (s2[j] + a8[j] * c_GJ[8][8] + S[j]);
+            same = same && same_bits(rn, r[j]);
+            r[j] = rn;
         }
+        if (same) // the passes left would return the same bits (as gj8_kernel)
+            break;
     }
 #pragma unroll
     for (int c = 0; c < 8; ++c)
@@ -162,16 +171,15 @@ __global__ void __launch_bounds__(256, 1) stm_kernel(TableSrc ts, VarArgs a)
         // primal passes; the Jacobian at the last evaluation point serves every pass of the
         // tangent step (as in the reverse sweep)
         double rl[3];
-        auto evalp = [&](const double* rr, double* aa, int it) {
-            if (it == a.ncorr - 1)
-                for (int j = 0; j < 3; ++j)
-                    rl[j] = rr[j];
+        auto evalp = [&](const double* rr, double* aa) {
+            for (int j = 0; j < 3; ++j)
+                rl[j] = rr[j];
             gravity_gcrs_lanes<false>(g, l, P, M, rr, aa, mask);
         };
         gj8_step<double>(evalp, a.h, a.ncorr, hist, s, S, r, v);
         double av[3], J[3][3];
         gravity_jac_gcrs_lanes(g, l, P, M, rl, av, J, mask);
-        auto evalt = [&](const double* rr, double* aa, int) {
+        auto evalt = [&](const double* rr, double* aa) {
 #pragma unroll
             for (int i = 0; i < 3; ++i)
                 aa[i] = J[i][0] * rr[0] + J[i][1] * rr[1] + J[i][2] * rr[2];
@@ -316,8 +324,8 @@ __global__ void __launch_bounds__(256, 1) adjoint_kernel(TableSrc ts, AdjArgs a)
             for (int step = lo; step <= hi; ++step) {
                 const double* M = a.prop_m + (size_t)(step + 4) * 9;
                 double* it_base = a.scratch + (size_t)(step - lo) * 3 * U + u;
-                auto eval = [&](const double* rr, double* aa, int it) {
-                    if (l == 0 && it == K - 1)
+                auto eval = [&](const double* rr, double* aa) {
+                    if (l == 0)
 #pragma unroll
                         for (int j = 0; j < 3; ++j)
                             it_base[(int64_t)j * U] = rr[j];
