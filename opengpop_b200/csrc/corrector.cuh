@@ -17,7 +17,7 @@ namespace gpop {
 //   pass r = F(r);
 // - else the fixed point under a(r) + J y, J the Jacobian of the central term and J2 and y the
 //   distance to that point: the next evaluation is three digits nearer than that of a plain pass.
-//   When |F(r) - r| is at most `near` of r (corrector_model: 3e-15, about 1e-8 m in LEO), what J
+//   When |F(r) - r| is at most `near` of r (corrector_model: 9.6e-15 for JGM3, 7e-8 m in LEO), what J
 //   leaves out of the acceleration is below a tenth of its last bit: a + J y is the acceleration at
 //   the fixed point to rounding, and no evaluation follows.
 // Positions, sums and the acceleration stay FP64; J y, a correction of their last digits, is FP32.

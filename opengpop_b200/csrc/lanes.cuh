@@ -11,14 +11,6 @@
 
 namespace gpop {
 
-// Lane setup by prefix products over the object's lanes (log2 P shuffle steps) instead of each
-// lane's own powers of (C1 + i S1) and q (tuned batch rates on B200, object-steps/s per SM:
-// degree 8 with 32 lanes 3.5e5 -> 4.7e5, degree 70 with 32 lanes 1.49e5 -> 1.65e5).
-#ifndef GPOP_LANE_SCAN
-#define GPOP_LANE_SCAN 1
-#endif
-constexpr bool kLaneScan = GPOP_LANE_SCAN != 0;
-
 // Stages a lane-layout blob into shared memory (after a 128-byte mbarrier slot) and binds it.
 __device__ __forceinline__ bool bind_lane_table(uint8_t* smem, const TableSrc& ts, unsigned* err, GravSmem& g)
 {
@@ -90,80 +82,155 @@ __device__ __forceinline__ void cpow(double c1, double s1, int p, double& rc, do
     rs = xs;
 }
 
-// Gravity in the Earth-fixed frame of K objects with the columns split over the P lanes of each
-// object's group (lane l takes columns l, l + P, ...); the per-object totals are added across the
-// P lanes. As gravity_itrs in mixed mode: the head columns m <= 8 are combined in FP64 (their
-// terms of degree > 8 summed in FP32 per column), the columns m > 8 are walked, combined and
-// summed in FP32 and added to the FP64 totals once. PAIRS: FP64 lanes walk two of their columns
-// side by side (the one-object GJ8 lane kernel; kernels with fewer registers to spare keep one at a
-// time).
-template <bool MIXED, int K, bool PAIRS = false>
-__device__ __forceinline__ void gravity_itrs_lk(const GravSmem& gs, int l, int P, const double (&x)[K],
-    const double (&y)[K], const double (&z)[K], double (&ax)[K], double (&ay)[K], double (&az)[K],
+// What a lane's columns l, l + T, ... start from and step by: z = C1 + i S1 and q to the powers l,
+// l - 1 (the m - 1 values; none for column 0), T and T - 1 (the m - 1 values of column T). T is a
+// power of two, or beyond the last column (then nothing steps and only the first three are made). The
+// powers come from the squares z^2, z^4, ... that every lane forms: two dependent operations per bit,
+// where a scan over the lanes adds a shuffle to each.
+struct LanePowers {
+    double Cm, Sm, Cp, Sp, qm, CP, SP, CPm1, SPm1, qP;
+};
+__device__ __forceinline__ LanePowers lane_powers(double C1, double S1, double q, int l, int T, bool steps)
+{
+    LanePowers w;
+    const int e = l > 0 ? l - 1 : 0;
+    double bc = C1, bs = S1, bq = q, xc = 1.0, xs = 0.0, xq = 1.0;
+    w.CPm1 = 1.0;
+    w.SPm1 = 0.0;
+    for (int o = 1; o < T; o <<= 1) {
+        double tc, ts;
+        cmul(xc, xs, bc, bs, tc, ts);
+        const bool on = (e & o) != 0;
+        xc = on ? tc : xc;
+        xs = on ? ts : xs;
+        xq = on ? xq * bq : xq;
+        if (steps)
+            cmul(w.CPm1, w.SPm1, bc, bs, w.CPm1, w.SPm1);
+        cmul(bc, bs, bc, bs, bc, bs);
+        bq *= bq;
+    }
+    w.CP = bc;
+    w.SP = bs;
+    w.qP = bq;
+    cmul(xc, xs, C1, S1, w.Cm, w.Sm);
+    w.qm = xq * q;
+    w.Cp = l > 0 ? xc : 0.0;
+    w.Sp = l > 0 ? xs : 0.0;
+    w.Cm = l > 0 ? w.Cm : 1.0;
+    w.Sm = l > 0 ? w.Sm : 0.0;
+    w.qm = l > 0 ? w.qm : 1.0;
+    return w;
+}
+
+// Totals of four values over the P lanes (a power of two) of each aligned group, in every lane. From
+// four lanes the first two levels halve what a lane still carries: 2 + 1 + log2 P - 2 exchanges and
+// four broadcasts of a value instead of 4 log2 P exchanges.
+__device__ __forceinline__ void lane_sum4(double& a, double& b, double& c, double& d, int l, int P,
     unsigned mask)
 {
+    if (P >= 4) {
+        const int h = P >> 1, f = P >> 2;
+        const bool hi = (l & h) != 0, hf = (l & f) != 0;
+        double x = hi ? c : a, y = hi ? d : b;
+        x += __shfl_xor_sync(mask, hi ? a : c, h);
+        y += __shfl_xor_sync(mask, hi ? b : d, h);
+        double t = hf ? y : x;
+        t += __shfl_xor_sync(mask, hf ? x : y, f);
+        for (int o = P >> 3; o > 0; o >>= 1)
+            t += __shfl_xor_sync(mask, t, o);
+        a = __shfl_sync(mask, t, 0, P);
+        b = __shfl_sync(mask, t, f, P);
+        c = __shfl_sync(mask, t, h, P);
+        d = __shfl_sync(mask, t, h + f, P);
+    } else if (P == 2) {
+        a += __shfl_xor_sync(mask, a, 1);
+        b += __shfl_xor_sync(mask, b, 1);
+        c += __shfl_xor_sync(mask, c, 1);
+        d += __shfl_xor_sync(mask, d, 1);
+    }
+}
+
+// The lanes of a group inside one warp: lane l of P, the group's lanes of the warp.
+struct WarpTeam {
+    int l, P;
+    unsigned mask;
+    __device__ __forceinline__ void sum4(double& a, double& b, double& c, double& d) const
+    {
+        lane_sum4(a, b, c, d, l, P, mask);
+    }
+};
+
+// A group of whole warps (T = 32 warps threads, at least one per column): lane sums in each warp, then
+// over the warps through shared memory. buf holds 2 x 4 x warps doubles of this group; the two halves
+// take turns, so that one barrier per sum is enough (a warp that is a sum ahead writes the other half,
+// and cannot be two ahead). bar: the group's named barrier.
+struct BlockTeam {
+    int l, P, warps, bar;
+    double* buf;
+    mutable int half;
+    __device__ __forceinline__ void sum4(double& a, double& b, double& c, double& d) const
+    {
+        const int lane = l & 31;
+        lane_sum4(a, b, c, d, lane, 32, 0xffffffffu);
+        double* h = buf + half * 4 * warps;
+        if (lane < 4)
+            h[(l >> 5) * 4 + lane] = lane == 0 ? a : lane == 1 ? b : lane == 2 ? c : d;
+        asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(P) : "memory");
+        a = b = c = d = 0.0;
+        for (int w = 0; w < warps; ++w) {
+            a += h[w * 4];
+            b += h[w * 4 + 1];
+            c += h[w * 4 + 2];
+            d += h[w * 4 + 3];
+        }
+        half ^= 1;
+    }
+};
+
+// Gravity in the Earth-fixed frame of K objects with the columns split over the P lanes of each
+// object's group (lane l takes columns l, l + P, ...; P a power of two, or more than the columns); the
+// per-object totals are added across the group. As gravity_itrs in mixed mode: the head columns
+// m <= 8 are combined in FP64 (their terms of degree > 8 summed in FP32 per column), the columns m > 8
+// are walked, combined and summed in FP32 and added to the FP64 totals once. PAIRS: FP64 lanes walk two
+// of their columns side by side (the one-object GJ8 lane kernel; kernels with fewer registers to spare
+// keep one at a time).
+template <bool MIXED, int K, bool PAIRS = false, class Team = WarpTeam>
+__device__ __forceinline__ void gravity_itrs_team(const GravSmem& gs, const Team& team, const double (&x)[K],
+    const double (&y)[K], const double (&z)[K], double (&ax)[K], double (&ay)[K], double (&az)[K])
+{
+    const int l = team.l, P = team.P;
     const int L = gs.L;
-    double r[K], q[K], u[K], w[K], C1[K], S1[K], CP[K], SP[K], Cm[K], Sm[K], Cp[K], Sp[K], CPm1[K], SPm1[K];
+    double ri[K], q[K], u[K], w[K], C1[K], S1[K], CP[K], SP[K], Cm[K], Sm[K], Cp[K], Sp[K], CPm1[K], SPm1[K];
     double qm[K], qP[K], G[K], H[K], J[K], KK[K];
     float uf[K], wf[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-        r[k] = sqrt(x[k] * x[k] + y[k] * y[k] + z[k] * z[k]);
-        const double eps = z[k] / r[k];
-        q[k] = gs.radius / r[k];
+        ri[k] = inv_norm(x[k], y[k], z[k]);
+        const double eps = z[k] * ri[k];
+        q[k] = gs.radius * ri[k];
         u[k] = q[k] * eps;
         w[k] = q[k] * q[k];
         uf[k] = (float)u[k];
         wf[k] = (float)w[k];
-        C1[k] = x[k] / r[k];
-        S1[k] = y[k] / r[k];
+        C1[k] = x[k] * ri[k];
+        S1[k] = y[k] * ri[k];
         G[k] = H[k] = J[k] = KK[k] = 0.0;
-        if (kLaneScan && P > 1) {
-            // prefix products over the group's lanes (segments of width P): lane l ends with
-            // z^(l+1) and q^(l+1), z = C1 + i S1; the lane's first column, the step between its
-            // columns and the m - 1 values follow by shuffles
-            double zc = C1[k], zs = S1[k], zq = q[k];
-            for (int o = 1; o < P; o <<= 1) {
-                const double pc = __shfl_up_sync(mask, zc, o, P), ps = __shfl_up_sync(mask, zs, o, P);
-                const double pq = __shfl_up_sync(mask, zq, o, P);
-                if (l >= o) {
-                    cmul(pc, ps, zc, zs, zc, zs);
-                    zq = pq * zq;
-                }
-            }
-            const double c1 = __shfl_up_sync(mask, zc, 1, P), s1 = __shfl_up_sync(mask, zs, 1, P);
-            const double q1 = __shfl_up_sync(mask, zq, 1, P);
-            const double c2 = __shfl_up_sync(mask, zc, 2, P), s2 = __shfl_up_sync(mask, zs, 2, P);
-            Cm[k] = l >= 1 ? c1 : 1.0; // z^l
-            Sm[k] = l >= 1 ? s1 : 0.0;
-            qm[k] = l >= 1 ? q1 : 1.0; // q^l
-            Cp[k] = l >= 2 ? c2 : (l == 1 ? 1.0 : 0.0); // z^(l-1); column 0 has no J, K or H part
-            Sp[k] = l >= 2 ? s2 : 0.0;
-            CP[k] = __shfl_sync(mask, zc, P - 1, P); // z^P: step between this lane's columns
-            SP[k] = __shfl_sync(mask, zs, P - 1, P);
-            qP[k] = __shfl_sync(mask, zq, P - 1, P);
-            CPm1[k] = __shfl_sync(mask, zc, P - 2, P); // z^(P-1): the m - 1 values of column P
-            SPm1[k] = __shfl_sync(mask, zs, P - 2, P);
-            continue;
-        }
-        cpow(C1[k], S1[k], P, CP[k], SP[k]); // step between this lane's columns
-        cpow(C1[k], S1[k], l, Cm[k], Sm[k]);
-        if (l > 0)
-            cpow(C1[k], S1[k], l - 1, Cp[k], Sp[k]);
-        else
-            Cp[k] = Sp[k] = 0.0; // column 0 has no J, K or H part
-        cpow(C1[k], S1[k], P - 1, CPm1[k], SPm1[k]); // the m - 1 values of column P
-        qm[k] = 1.0;
-        qP[k] = 1.0;
-        for (int i = 0; i < l; ++i)
-            qm[k] *= q[k];
-        for (int i = 0; i < P; ++i)
-            qP[k] *= q[k];
+        const LanePowers lp = lane_powers(C1[k], S1[k], q[k], l, P, P <= L);
+        Cm[k] = lp.Cm;
+        Sm[k] = lp.Sm;
+        Cp[k] = lp.Cp;
+        Sp[k] = lp.Sp;
+        qm[k] = lp.qm;
+        CP[k] = lp.CP;
+        SP[k] = lp.SP;
+        CPm1[k] = lp.CPm1;
+        SPm1[k] = lp.SPm1;
+        qP[k] = lp.qP;
     }
     const int Lhead = (MIXED && L > kMixedSplit) ? kMixedSplit : L;
     // column bases of the lane's next column are read one column ahead (they are shared-memory
     // loads the walk's first table read depends on)
-    int b64 = gs.cb64[l], b32 = gs.cb32[l];
+    int b64 = gs.cb64[l < 127 ? l : 127], b32 = gs.cb32[l < 127 ? l : 127];
     int m = l;
     if constexpr (!MIXED && PAIRS && kLanePairColumns) {
         // FP64: two of this lane's columns (m and m + P) side by side, so each object carries two
@@ -312,19 +379,17 @@ __device__ __forceinline__ void gravity_itrs_lk(const GravSmem& gs, int l, int P
     }
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-        for (int o = P >> 1; o > 0; o >>= 1) {
-            G[k] += __shfl_xor_sync(mask, G[k], o);
-            H[k] += __shfl_xor_sync(mask, H[k], o);
-            J[k] += __shfl_xor_sync(mask, J[k], o);
-            KK[k] += __shfl_xor_sync(mask, KK[k], o);
-        }
-        const double Gt = G[k] + 1.0; // eq. 4-13
-        const double Lambda = Gt + z[k] * H[k] / r[k];
-        const double c = -gs.gm / (r[k] * r[k]);
-        ax[k] = c * (Lambda * x[k] / r[k] - J[k]);
-        ay[k] = c * (Lambda * y[k] / r[k] - KK[k]);
-        az[k] = c * (Lambda * z[k] / r[k] - H[k]);
+        team.sum4(G[k], H[k], J[k], KK[k]);
+        assemble_itrs(gs.gm, x[k], y[k], z[k], ri[k], G[k], H[k], J[k], KK[k], ax[k], ay[k], az[k]);
     }
+}
+
+template <bool MIXED, int K, bool PAIRS = false>
+__device__ __forceinline__ void gravity_itrs_lk(const GravSmem& gs, int l, int P, const double (&x)[K],
+    const double (&y)[K], const double (&z)[K], double (&ax)[K], double (&ay)[K], double (&az)[K],
+    unsigned mask)
+{
+    gravity_itrs_team<MIXED, K, PAIRS>(gs, WarpTeam { l, P, mask }, x, y, z, ax, ay, az);
 }
 
 template <bool MIXED>
@@ -340,9 +405,9 @@ __device__ __forceinline__ void gravity_itrs_lanes(const GravSmem& gs, int l, in
 }
 
 // K objects: GCRS positions r[k] with the ITRS<-GCRS matrix M of gravity_gcrs.
-template <bool MIXED, int K, bool PAIRS = false>
-__device__ __forceinline__ void gravity_gcrs_lk(const GravSmem& gs, int l, int P, const double* __restrict__ M,
-    const double (&r)[K][3], double (&a)[K][3], unsigned mask)
+template <bool MIXED, int K, bool PAIRS = false, class Team = WarpTeam>
+__device__ __forceinline__ void gravity_gcrs_team(const GravSmem& gs, const Team& team,
+    const double* __restrict__ M, const double (&r)[K][3], double (&a)[K][3])
 {
     double m[9];
 #pragma unroll
@@ -355,13 +420,20 @@ __device__ __forceinline__ void gravity_gcrs_lk(const GravSmem& gs, int l, int P
         py[k] = m[3] * r[k][0] + m[4] * r[k][1] + m[5] * r[k][2];
         pz[k] = m[6] * r[k][0] + m[7] * r[k][1] + m[8] * r[k][2];
     }
-    gravity_itrs_lk<MIXED, K, PAIRS>(gs, l, P, px, py, pz, ax, ay, az, mask);
+    gravity_itrs_team<MIXED, K, PAIRS>(gs, team, px, py, pz, ax, ay, az);
 #pragma unroll
     for (int k = 0; k < K; ++k) {
         a[k][0] = m[0] * ax[k] + m[3] * ay[k] + m[6] * az[k];
         a[k][1] = m[1] * ax[k] + m[4] * ay[k] + m[7] * az[k];
         a[k][2] = m[2] * ax[k] + m[5] * ay[k] + m[8] * az[k];
     }
+}
+
+template <bool MIXED, int K, bool PAIRS = false>
+__device__ __forceinline__ void gravity_gcrs_lk(const GravSmem& gs, int l, int P, const double* __restrict__ M,
+    const double (&r)[K][3], double (&a)[K][3], unsigned mask)
+{
+    gravity_gcrs_team<MIXED, K, PAIRS>(gs, WarpTeam { l, P, mask }, M, r, a);
 }
 
 template <bool MIXED>
