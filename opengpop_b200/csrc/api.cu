@@ -145,7 +145,7 @@ gpop_status propagator_init(gpop_propagator* p, cudaStream_t s)
         if (st != GPOP_OK)
             return st;
     }
-    if ((e = p->state->ensure((size_t)kStateArrays * p->n * sizeof(double))) != cudaSuccess)
+    if ((e = p->state->ensure(state_bytes(p->n))) != cudaSuccess)
         return fail(ctx, GPOP_ERR_NOMEM, std::string("propagation state: ") + cudaGetErrorString(e));
     return GPOP_OK;
 }
@@ -176,9 +176,9 @@ gpop_status propagator_step(gpop_propagator* p, int steps, double* traj_r, doubl
     a.r0 = p->r;
     a.v0 = p->v;
     if (!p->started) {
-        if ((e = launch_startup(ts, a, ctx->num_sms, s)) != cudaSuccess)
+        if ((e = launch_startup(ts, a, ctx->num_sms, s, &lane_ts)) != cudaSuccess)
             return cuda_fail(ctx, e, "startup kernel");
-        ctx->launches++;
+        ctx->launches += p->kind == GPOP_FORCE_GRAVITY ? startup_launches(p->ncorr) : 1;
         p->started = true;
     }
     a.traj_r = traj_r;

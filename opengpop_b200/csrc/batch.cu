@@ -11,30 +11,13 @@
 #include "corrector.cuh"
 #include "frames.cuh"
 #include "gravity.cuh"
-#include "integrator.cuh"
+#include "gj8_tables.cuh"
 #include "lanes.cuh"
+#include "startup.cuh"
 
 #include <type_traits>
 
 namespace gpop {
-
-// Force model of one request (startup kernel, one lane per object).
-template <bool MIXED> struct ForceReq {
-    static constexpr bool kPositionOnly = true;
-    GravSmem g;
-    const double* gen_m;
-    const double* prop_m;
-    __device__ __forceinline__ unsigned agree(unsigned bits) const { return bits; }
-    __device__ __forceinline__ void prop(const double* r, const double*, int idx, double* a) const
-    {
-        gravity_gcrs1<MIXED>(g, prop_m + (size_t)idx * 9, r, a);
-    }
-    __device__ __forceinline__ void gen(const double* r, const double*, int step, int k, double* a) const
-    {
-        const int s = step > 0 ? step - 1 : step;
-        gravity_gcrs1<MIXED>(g, gen_m + (size_t)((s + 4) * 10 + k) * 9, r, a);
-    }
-};
 
 template <bool MIXED>
 __device__ __forceinline__ bool stage_batch_table(uint8_t* smem, const TableSrc& ts, unsigned* err, GravSmem& g)
@@ -49,47 +32,6 @@ __device__ __forceinline__ bool stage_batch_table(uint8_t* smem, const TableSrc&
     g.t64 = reinterpret_cast<const GravEntry64*>(tab);
     g.t32 = reinterpret_cast<const GravEntry32*>(tab + ts.off32);
     return ok;
-}
-
-template <bool MIXED>
-__global__ void __launch_bounds__(256) batch_startup_kernel(TableSrc ts, BatchArgs a)
-{
-    extern __shared__ __align__(128) uint8_t smem[];
-    GravSmem g0;
-    if (!stage_batch_table<MIXED>(smem, ts, a.err, g0))
-        return;
-    const int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= a.n_obj)
-        return;
-    const BatchReq rq = a.reqs[a.obj_req[o]];
-    ForceReq<MIXED> f;
-    f.g = g0;
-    f.g.L = rq.L;
-    f.gen_m = rq.gen_m;
-    f.prop_m = rq.prop_m;
-    double r0[3], v0[3];
-    for (int j = 0; j < 3; ++j) {
-        r0[j] = a.r0[o * 3 + j];
-        v0[j] = a.v0[o * 3 + j];
-    }
-    StartupMats m;
-    run_startup(f, rq.h, a.ncorr, r0, v0, m);
-    const int64_t n = a.n_obj;
-    double* st = a.state;
-    const bool fix_q3 = (a.flags & 2u) != 0;
-    for (int j = 0; j < 3; ++j) {
-        st[(kR + j) * n + o] = m.r[8][j];
-        st[(kV + j) * n + o] = m.v[8][j];
-        st[(kSs + j) * n + o] = m.s[8][j];
-        st[(kSb + j) * n + o] = m.S[8][j];
-        for (int c = 0; c < 9; ++c)
-            st[(kHist + c * 3 + j) * n + o] = m.a[c][j];
-        for (int k = 0; k < 4; ++k) {
-            st[(kRep + k * 6 + j) * n + o] = m.r[5 + k][j];
-            st[(kRep + k * 6 + 3 + j) * n + o] = m.v[5 + k][j];
-            st[(kRepA + k * 3 + j) * n + o] = fix_q3 ? m.a[5 + k][j] : m.a[8][j];
-        }
-    }
 }
 
 // Two objects per lane may walk the gravity columns two at a time (as gj8_kernel does), in
@@ -322,23 +264,21 @@ template <class K> static cudaError_t set_smem(K kernel, size_t bytes)
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
-cudaError_t launch_batch_startup(const TableSrc& ts, const BatchArgs& a, int num_sms, cudaStream_t s)
+cudaError_t launch_batch_startup(const TableSrc& lane_ts, const TableSrc& plain_ts, const BatchArgs& a,
+    int num_sms, cudaStream_t s)
 {
-    if (a.n_obj <= 0)
-        return cudaSuccess;
-    LaunchShape ls = pick_shape(a.n_obj, 256, num_sms);
-    const size_t smem = table_smem_bytes(ts);
-    cudaError_t e;
-    if (ts.mixed) {
-        if ((e = set_smem(batch_startup_kernel<true>, smem)) != cudaSuccess)
-            return e;
-        batch_startup_kernel<true><<<ls.grid, ls.block, smem, s>>>(ts, a);
-    } else {
-        if ((e = set_smem(batch_startup_kernel<false>, smem)) != cudaSuccess)
-            return e;
-        batch_startup_kernel<false><<<ls.grid, ls.block, smem, s>>>(ts, a);
-    }
-    return cudaGetLastError();
+    StartupArgs b;
+    b.n = a.n_obj;
+    b.reqs = a.reqs;
+    b.obj_req = a.obj_req;
+    b.ncorr = a.ncorr;
+    b.flags = a.flags;
+    b.r0 = a.r0;
+    b.v0 = a.v0;
+    b.state = a.state;
+    b.counters = reinterpret_cast<int*>(a.state + (size_t)kStateArrays * a.n_obj);
+    b.err = a.err;
+    return launch_startup_gravity(plain_ts, lane_ts, b, num_sms, s);
 }
 
 template <bool MIXED, bool STAGE, bool PAIRS>

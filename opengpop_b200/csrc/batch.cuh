@@ -36,7 +36,7 @@ struct BatchArgs {
     const BatchItem* items = nullptr;
     int n_items = 0;
     int* next_item = nullptr; // work-queue head (zeroed before the launch)
-    const int* obj_req = nullptr; // request of each flattened object (startup kernel)
+    const int* obj_req = nullptr; // request of each flattened object (startup)
     int64_t n_obj = 0;
     int ncorr = 7;
     uint32_t flags = 0;
@@ -50,9 +50,11 @@ struct BatchArgs {
     bool pair_walk = false; // two-object items walk two gravity columns at a time
 };
 
-cudaError_t launch_batch_startup(const TableSrc& ts, const BatchArgs& a, int num_sms, cudaStream_t s);
-// lane_ts: the lane-layout table; plain_ts: the same model in the plain layout (batches of
-// single-lane items). blocks: persistent grid size; block: threads per block.
+// lane_ts: the lane-layout table; plain_ts: the same model in the plain layout.
+cudaError_t launch_batch_startup(const TableSrc& lane_ts, const TableSrc& plain_ts, const BatchArgs& a,
+    int num_sms, cudaStream_t s);
+// The plain table serves batches of single-lane items. blocks: persistent grid size; block: threads per
+// block.
 cudaError_t launch_batch_gj8(const TableSrc& lane_ts, const TableSrc& plain_ts, const BatchArgs& a,
     int blocks, int block, cudaStream_t s);
 cudaError_t launch_frames_batch(const FrameData& fd, const int* cal, const int* epoch_req,

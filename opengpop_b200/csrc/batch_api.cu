@@ -435,7 +435,7 @@ static gpop_status run_batch(gpop_ctx* ctx, const gpop_request* reqs, int32_t n_
             || (e = bc->reqs.ensure(n_req * sizeof(BatchReq))) != cudaSuccess
             || (e = bc->items.ensure(std::max<size_t>(1, plan.items.size()) * sizeof(BatchItem))) != cudaSuccess
             || (e = bc->obj_req.ensure((size_t)N * sizeof(int))) != cudaSuccess
-            || (e = bc->state.ensure((size_t)kStateArrays * N * sizeof(double))) != cudaSuccess
+            || (e = bc->state.ensure(state_bytes(N))) != cudaSuccess
             || (e = bc->queue.ensure(sizeof(int))) != cudaSuccess)
             return fail(ctx, GPOP_ERR_NOMEM, std::string("batch buffers: ") + cudaGetErrorString(e));
         for (size_t t = 0; t < tables.size(); ++t) {
@@ -490,7 +490,6 @@ static gpop_status run_batch(gpop_ctx* ctx, const gpop_request* reqs, int32_t n_
             return cuda_fail(ctx, e, "batch plan upload");
         // ---- capture: frames, startup, queue reset, persistent GJ8 ----
         const bool mixed = ctx->cfg.precision == GPOP_MIXED;
-        TableSrc ts = ctx->table(mixed);
         BatchArgs a;
         a.reqs = bc->reqs.as<BatchReq>();
         a.n_req = n_req;
@@ -515,7 +514,7 @@ static gpop_status run_batch(gpop_ctx* ctx, const gpop_request* reqs, int32_t n_
         cudaError_t le = launch_frames_batch(ctx->frames, bc->cal.as<int>(), bc->epoch_req.as<int>(),
             bc->sec.as<double>(), (int)E, dtab, s);
         if (le == cudaSuccess)
-            le = launch_batch_startup(ts, a, ctx->num_sms, s);
+            le = launch_batch_startup(ctx->lane_table(mixed), ctx->table(mixed), a, ctx->num_sms, s);
         if (le == cudaSuccess)
             le = cudaMemsetAsync(bc->queue.p, 0, sizeof(int), s);
         if (le == cudaSuccess)
@@ -539,7 +538,7 @@ static gpop_status run_batch(gpop_ctx* ctx, const gpop_request* reqs, int32_t n_
     timer.mark(s);
     if ((e = cudaGraphLaunch(bc->exec, s)) != cudaSuccess)
         return cuda_fail(ctx, e, "batch graph launch");
-    ctx->launches += 3;
+    ctx->launches += 2 + startup_launches(ctx->cfg.n_corrections);
     timer.mark(s);
     if ((e = cudaMemcpyAsync(host + 6 * N, dio + 6 * N, (size_t)N * 6 * sizeof(double), cudaMemcpyDeviceToHost, s))
         != cudaSuccess)
@@ -664,7 +663,7 @@ gpop_status gpop_tune(gpop_ctx* ctx, const char* cache_path)
                 && (e = cudaEventSynchronize(e1)) == cudaSuccess
                 && (e = cudaEventElapsedTime(&t, e0, e1)) == cudaSuccess)
                 ms = std::min(ms, t);
-            ctx->launches += 3;
+            ctx->launches += 2 + startup_launches(ctx->cfg.n_corrections);
         }
         if (e0)
             cudaEventDestroy(e0);

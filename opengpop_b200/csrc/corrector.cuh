@@ -6,6 +6,40 @@
 
 namespace gpop {
 
+// J of a position: the Jacobian of
+//   a = -GM/r^2 u - GM b/r^2 [(1 - 5 s^2) u + 2 s e],  b = 1.5 J2 R^2/r^2, s = u . e,
+// e the polar axis (the frame's z: off the Earth's axis by some 1e-3, which J2 turns into 1e-6 of J).
+struct CorrJacobian {
+    float u[3], len, g, b; // unit vector, r, GM / r^3
+    __device__ __forceinline__ CorrJacobian() {}
+    __device__ __forceinline__ CorrJacobian(const CorrModel& cm, const double (&r)[3])
+    {
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+            u[j] = (float)r[j];
+        const float r2 = u[0] * u[0] + u[1] * u[1] + u[2] * u[2];
+        const float ri = rsqrtf(r2);
+        len = r2 * ri;
+        g = (cm.gm * ri) * ri * ri;
+        b = cm.j2 * ri * ri;
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+            u[j] *= ri;
+    }
+    __device__ __forceinline__ void apply(const float (&y)[3], float (&o)[3]) const
+    {
+        const float s = u[2], c5 = 1.f - 5.f * s * s;
+        const float dr = u[0] * y[0] + u[1] * y[1] + u[2] * y[2];
+        const float t = s * (y[2] - s * dr); // r/2 times the change of s^2
+        const float pu = 3.f * dr + b * (5.f * dr * c5 + 10.f * t);
+        const float py = 1.f + b * c5;
+        const float pz = b * (10.f * dr * s - 2.f * y[2]);
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+            o[j] = g * (pu * u[j] - py * y[j] + (j == 2 ? pz : 0.f));
+    }
+};
+
 // The corrector iterates the position to the fixed point of
 //   F(r) = h^2 (s2 + GJ[8][8] a(r) + S)   (gpu_propagator.cu:86-119),
 // one gravity evaluation per pass; s and v of the step follow from the last acceleration. Each pass
@@ -43,61 +77,38 @@ __device__ __forceinline__ bool correct_position(const CorrModel& cm, double h, 
     }
     if (same)
         return true;
-    float d[3], u[3];
+    float d[3];
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
+    for (int j = 0; j < 3; ++j)
         d[j] = (float)(rn[j] - r[j]);
-        u[j] = (float)r[j];
-    }
-    const float r2 = u[0] * u[0] + u[1] * u[1] + u[2] * u[2];
-    const float ri = rsqrtf(r2);
-    const float len = r2 * ri;
-    const float g = (cm.gm * ri) * ri * ri; // GM / r^3
-    const float k = (float)(h * h * c_GJ[8][8]) * g;
+    const CorrJacobian jac(cm, r);
+    const float hg = (float)(h * h * c_GJ[8][8]);
     const float dmax = fmaxf(fmaxf(fabsf(d[0]), fabsf(d[1])), fabsf(d[2]));
     if (it == 0) {
         // change of the plain iteration after its last pass, with one power of rho to spare
-        const float rho = 2.2f * fabsf(k);
+        const float rho = 2.2f * fabsf(hg * jac.g);
         float left = dmax;
         for (int i = 2; i < ncorr && i < 10; ++i)
             left *= rho;
-        fast = ncorr > 2 && rho < 0.1f && left <= 0x1p-54f * len && len >= cm.low;
+        fast = ncorr > 2 && rho < 0.1f && left <= 0x1p-54f * jac.len && jac.len >= cm.low;
     }
-    const bool near = dmax <= cm.near * len;
+    const bool near = dmax <= cm.near * jac.len;
     if (!fast || (it == ncorr - 1 && !near)) {
 #pragma unroll
         for (int j = 0; j < 3; ++j)
             r[j] = rn[j];
         return it == ncorr - 1;
     }
-#pragma unroll
-    for (int j = 0; j < 3; ++j)
-        u[j] *= ri;
-    // a = -GM/r^2 u - GM b/r^2 [(1 - 5 s^2) u + 2 s e], b = 1.5 J2 R^2/r^2, s = u . e, e the polar
-    // axis (the frame's z: off the Earth's axis by some 1e-3, which J2 turns into 1e-6 of J);
-    // jac(y) = J y of it
-    const float b = cm.j2 * ri * ri, s = u[2], c5 = 1.f - 5.f * s * s;
-    auto jac = [&](const float (&y)[3], float (&o)[3]) {
-        const float dr = u[0] * y[0] + u[1] * y[1] + u[2] * y[2];
-        const float t = s * (y[2] - s * dr); // r/2 times the change of s^2
-        const float pu = 3.f * dr + b * (5.f * dr * c5 + 10.f * t);
-        const float py = 1.f + b * c5;
-        const float pz = b * (10.f * dr * s - 2.f * y[2]);
-#pragma unroll
-        for (int j = 0; j < 3; ++j)
-            o[j] = g * (pu * u[j] - py * y[j] + (j == 2 ? pz : 0.f));
-    };
     // y = (I - h^2 GJ[8][8] J)^-1 d to second order
-    const float hg = (float)(h * h * c_GJ[8][8]);
     float y[3] = { d[0], d[1], d[2] }, o[3];
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-        jac(y, o);
+        jac.apply(y, o);
 #pragma unroll
         for (int j = 0; j < 3; ++j)
             y[j] = d[j] + hg * o[j];
     }
-    jac(y, o);
+    jac.apply(y, o);
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
         const double aj = a[j] + (double)o[j];

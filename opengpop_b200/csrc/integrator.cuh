@@ -150,140 +150,4 @@ __device__ void run_startup(const F& f, double h, int ncorr, const T* r0, const 
             break;
 }
 
-// ---- the same startup for two objects in lockstep (the split block's startup kernel) ----
-// F2 provides gen2(r, v, step, k, a) and prop2(r, v, idx, a) over both objects at once
-// ([2][3] arrays), and any2(x), whether x holds for any thread; those may hold block-wide barriers,
-// so every thread of a block makes the same calls in the same order (the control flow below depends
-// on any2's answers and on no other data). Per object the arithmetic
-// is that of rk8_step, corrector_correct and run_startup. A thread that carries no objects
-// (active false) makes the same force calls and skips the arithmetic around them.
-template <class F2>
-__device__ void rk8_step2(const F2& f, double h, int step, StartupMats (&m)[2], bool active)
-{
-    const double hh = step > 0 ? h : -h;
-    const int base = 4 + step + (step > 0 ? -1 : 1);
-    double Kx[2][10][3], Kv[2][10][3];
-    double tx[2][3] = {}, tv[2][3] = {};
-    for (int o = 0; o < 2 && active; ++o)
-        for (int j = 0; j < 3; ++j) {
-            tx[o][j] = m[o].r[base][j];
-            tv[o][j] = m[o].v[base][j];
-            Kx[o][0][j] = tv[o][j];
-        }
-    {
-        double acc[2][3];
-        f.gen2(tx, tv, step, 0, acc);
-        for (int o = 0; o < 2 && active; ++o)
-            for (int j = 0; j < 3; ++j)
-                Kv[o][0][j] = acc[o][j];
-    }
-    for (int k = 1; k <= 9; ++k) {
-        for (int o = 0; o < 2 && active; ++o)
-            for (int j = 0; j < 3; ++j) {
-                double sx = 0.0, sv = 0.0;
-                for (int i = 0; i < k; ++i) {
-                    sx = fma(c_RKA[k - 1][i], Kx[o][i][j], sx);
-                    sv = fma(c_RKA[k - 1][i], Kv[o][i][j], sv);
-                }
-                tx[o][j] = fma(hh, sx, m[o].r[base][j]);
-                tv[o][j] = fma(hh, sv, m[o].v[base][j]);
-            }
-        double acc[2][3];
-        f.gen2(tx, tv, step, k, acc);
-        for (int o = 0; o < 2 && active; ++o)
-            for (int j = 0; j < 3; ++j) {
-                Kv[o][k][j] = acc[o][j];
-                Kx[o][k][j] = tv[o][j];
-            }
-    }
-    const int col = 4 + step;
-    for (int o = 0; o < 2 && active; ++o)
-        for (int j = 0; j < 3; ++j) {
-            double sx = 0.0, sv = 0.0;
-            for (int k = 0; k < 10; ++k) {
-                sx = fma(Kx[o][k][j], c_RKB[k], sx);
-                sv = fma(Kv[o][k][j], c_RKB[k], sv);
-            }
-            m[o].v[col][j] = fma(hh, sv, m[o].v[base][j]);
-            m[o].r[col][j] = fma(hh, sx, m[o].r[base][j]);
-        }
-}
-
-template <class F2>
-__device__ void corrector_accel2(const F2& f, StartupMats (&m)[2], int i, bool active)
-{
-    double r[2][3] = {}, v[2][3] = {}, acc[2][3];
-    for (int o = 0; o < 2 && active; ++o)
-        for (int j = 0; j < 3; ++j) {
-            r[o][j] = m[o].r[i][j];
-            v[o][j] = m[o].v[i][j];
-        }
-    f.prop2(r, v, i, acc);
-    for (int o = 0; o < 2 && active; ++o)
-        for (int j = 0; j < 3; ++j)
-            m[o].a[i][j] = acc[o][j];
-}
-
-// As corrector_correct: a column is evaluated where it moved for any object of the block (any2).
-template <class F2>
-__device__ bool corrector_correct2(const F2& f, double h, StartupMats (&m)[2], bool active)
-{
-    const double h2 = h * h;
-    unsigned moved = 0;
-    for (int o = 0; o < 2 && active; ++o) {
-        corrector_s0(h, m[o]);
-        corrector_all_s(m[o]);
-        for (int c = 0; c < 9; ++c) {
-            if (c == 4)
-                continue; // the epoch column is restored
-            for (int j = 0; j < 3; ++j) {
-                double sv = 0.0, sr = 0.0;
-                for (int k = 0; k < 9; ++k) {
-                    sv = fma(m[o].a[k][j], c_SA[c][k], sv);
-                    sr = fma(m[o].a[k][j], c_GJ[c][k], sr);
-                }
-                m[o].v[c][j] = h * (sv + m[o].s[c][j]);
-                const double rn = h2 * (sr + m[o].S[c][j]);
-                if (!same_bits(rn, m[o].r[c][j]))
-                    moved |= 1u << c;
-                m[o].r[c][j] = rn;
-            }
-        }
-    }
-    bool any = false;
-    for (int c = 0; c < 9; ++c) {
-        if (c == 4 || !f.any2(moved >> c & 1)) // the same for every thread of the block
-            continue;
-        any = true;
-        corrector_accel2(f, m, c, active);
-    }
-    return any;
-}
-
-template <class F2>
-__device__ void run_startup2(const F2& f, double h, int ncorr, const double (&r0)[2][3],
-    const double (&v0)[2][3], StartupMats (&m)[2], bool active)
-{
-    for (int o = 0; o < 2 && active; ++o) {
-        for (int c = 0; c < 9; ++c)
-            for (int j = 0; j < 3; ++j)
-                m[o].r[c][j] = m[o].v[c][j] = m[o].a[c][j] = m[o].s[c][j] = m[o].S[c][j] = 0.0;
-        for (int j = 0; j < 3; ++j) {
-            m[o].r[4][j] = r0[o][j];
-            m[o].v[4][j] = v0[o][j];
-        }
-    }
-    for (int i = 1; i <= 4; ++i) {
-        rk8_step2(f, h, i, m, active);
-        rk8_step2(f, h, -i, m, active);
-    }
-    if (ncorr <= 0)
-        return;
-    for (int i = 0; i < 9; ++i)
-        corrector_accel2(f, m, i, active);
-    for (int i = 0; i < ncorr; ++i)
-        if (!corrector_correct2(f, h, m, active)) // the same for every thread of the block
-            break;
-}
-
 } // namespace gpop

@@ -34,6 +34,9 @@ enum StateSlot : int {
     kX0 = 75, // split block exchange (12 values per object) when it does not fit in shared memory
     kStateArrays = 87
 };
+constexpr int kStartupCounters = 64; // ints after the state arrays, one per startup corrector pass
+// Bytes of the state of n objects with the startup's counters.
+inline size_t state_bytes(int64_t n) { return (size_t)kStateArrays * n * sizeof(double) + kStartupCounters * sizeof(int); }
 
 struct PropArgs {
     int64_t n = 0;
@@ -71,7 +74,12 @@ LaunchShape pick_shape(int64_t n, int max_block, int num_sms);
 // Dynamic shared memory one block of the current device may opt in to (0 if it cannot be read).
 size_t max_smem_optin();
 
-cudaError_t launch_startup(const TableSrc& ts, const PropArgs& a, int num_sms, cudaStream_t s);
+// Kernels of the startup pipeline: the RK8 chains, their columns, two per corrector pass, the end.
+inline int startup_launches(int ncorr) { return 3 + 2 * ncorr; }
+// Startup of a.n objects. Gravity with the state and the lane-layout table at hand runs the pipeline of
+// startup.cu; analytic forces, compensated sums and the unit entry point one thread per object.
+cudaError_t launch_startup(const TableSrc& ts, const PropArgs& a, int num_sms, cudaStream_t s,
+    const TableSrc* lane_ts = nullptr);
 // How many objects a GJ8 thread carries through the gravity triangle walk (0 = by problem size).
 // kWalkLanes: P lanes per object split the gravity columns (few objects; P from lanes_per_object).
 // kWalkLanesTwo: P lanes per group of two objects (P from lane_pair_lanes, else 2), the default

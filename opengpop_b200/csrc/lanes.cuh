@@ -158,6 +158,7 @@ struct WarpTeam {
     {
         lane_sum4(a, b, c, d, l, P, mask);
     }
+    __device__ __forceinline__ void sync() const { __syncwarp(mask); }
 };
 
 // A group of whole warps (T = 32 warps threads, at least one per column): lane sums in each warp, then
@@ -168,6 +169,10 @@ struct BlockTeam {
     int l, P, warps, bar;
     double* buf;
     mutable int half;
+    __device__ __forceinline__ void sync() const
+    {
+        asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(P) : "memory");
+    }
     __device__ __forceinline__ void sum4(double& a, double& b, double& c, double& d) const
     {
         const int lane = l & 31;
@@ -175,7 +180,7 @@ struct BlockTeam {
         double* h = buf + half * 4 * warps;
         if (lane < 4)
             h[(l >> 5) * 4 + lane] = lane == 0 ? a : lane == 1 ? b : lane == 2 ? c : d;
-        asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(P) : "memory");
+        sync();
         a = b = c = d = 0.0;
         for (int w = 0; w < warps; ++w) {
             a += h[w * 4];

@@ -37,7 +37,7 @@ constexpr int kMaxEpochs = 4 + kMaxSteps + 1; // propagation table entries
 // Scratch layout in doubles: state | generation matrices | propagation matrices | generation
 // seconds | propagation seconds | error word
 constexpr size_t kOffState = 0;
-constexpr size_t kOffGen = kOffState + (size_t)kStateArrays * kMaxObjects;
+constexpr size_t kOffGen = kOffState + (size_t)kStateArrays * kMaxObjects + kStartupCounters / 2;
 constexpr size_t kOffProp = kOffGen + 80 * 9;
 constexpr size_t kOffGenSec = kOffProp + (size_t)kMaxEpochs * 9;
 constexpr size_t kOffPropSec = kOffGenSec + 80;
@@ -137,7 +137,7 @@ extern "C" gpop_status gpop_propagate_device_noalloc(gpop_ctx* ctx, const gpop_t
     a.err = err;
     a.r0 = r_dev;
     a.v0 = v_dev;
-    if ((e = launch_startup(ts, a, ctx->num_sms, s)) != cudaSuccess)
+    if ((e = launch_startup(ts, a, ctx->num_sms, s, &lane_ts)) != cudaSuccess)
         return cuda_fail(ctx, e, "startup kernel");
     const int chunk = ctx->steps_per_launch;
     for (int b = 1; b <= steps; b += chunk) {
@@ -150,7 +150,7 @@ extern "C" gpop_status gpop_propagate_device_noalloc(gpop_ctx* ctx, const gpop_t
             != cudaSuccess)
             return cuda_fail(ctx, e, "GJ8 kernel");
     }
-    ctx->launches += 4 + (steps + chunk - 1) / chunk;
+    ctx->launches += 3 + startup_launches(ctx->cfg.n_corrections) + (steps + chunk - 1) / chunk;
     unsigned word = 0;
     if ((e = cudaMemcpyAsync(&word, err, sizeof(unsigned), cudaMemcpyDeviceToHost, s)) != cudaSuccess
         || (e = cudaStreamSynchronize(s)) != cudaSuccess)
