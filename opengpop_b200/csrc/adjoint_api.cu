@@ -55,11 +55,17 @@ gpop_status upload(gpop_ctx* ctx, DevBuf& d, const double* host, size_t count, c
     return GPOP_OK;
 }
 
-// FP64 propagation of n objects (device AoS r, v in place) that saves the GJ8 state after the
-// startup and after every 64th step, and optionally the trajectory ([steps][3][n] r, v, a).
-gpop_status forward_checkpointed(gpop_ctx* ctx, gpop_propagator& p, const gpop_time* start, double h,
-    int32_t steps, int64_t n, double* r, double* v, DevBuf& ckpt, double* traj_r, double* traj_v,
-    double* traj_a, cudaStream_t s)
+constexpr int64_t kVarObjects = 65536; // objects whose startup tangents are held at once
+constexpr size_t kWindowBytes = (size_t)512 << 20; // Jacobians held at once
+
+gpop_status nomem(gpop_ctx* ctx, const char* what, cudaError_t e)
+{
+    return fail(ctx, GPOP_ERR_NOMEM, std::string(what) + ": " + cudaGetErrorString(e));
+}
+
+// A fresh FP64 propagation of n objects (device AoS r, v in place).
+gpop_status begin(gpop_ctx* ctx, gpop_propagator& p, const gpop_time* start, double h, int32_t steps, int64_t n,
+    double* r, double* v, cudaStream_t s)
 {
     p.ctx = ctx;
     p.kind = GPOP_FORCE_GRAVITY;
@@ -71,67 +77,260 @@ gpop_status forward_checkpointed(gpop_ctx* ctx, gpop_propagator& p, const gpop_t
     p.r = r;
     p.v = v;
     p.mixed = false;
-    gpop_status st = propagator_init(&p, s);
-    if (st != GPOP_OK)
-        return st;
+    return propagator_init(&p, s);
+}
+
+// Positions of the startup's stages and columns, their Jacobians and the startup tangents.
+struct StartupTangents {
+    DevBuf stage_pos, col_pos, stage_jac, col_jac, out;
+    ~StartupTangents()
+    {
+        for (DevBuf* b : { &stage_pos, &col_pos, &stage_jac, &col_jac, &out })
+            b->release();
+    }
+    gpop_status reserve(gpop_ctx* ctx, gpop_propagator& p)
+    {
+        const size_t n = (size_t)p.n;
+        cudaError_t e;
+        if ((e = stage_pos.ensure(240 * n * 8)) != cudaSuccess || (e = col_pos.ensure(27 * n * 8)) != cudaSuccess
+            || (e = stage_jac.ensure(720 * n * 8)) != cudaSuccess || (e = col_jac.ensure(81 * n * 8)) != cudaSuccess
+            || (e = out.ensure((size_t)kStartupTangents * 6 * n * 8)) != cudaSuccess)
+            return nomem(ctx, "startup tangents", e);
+        p.stage_pos = stage_pos.as<double>();
+        p.col_pos = col_pos.as<double>();
+        return GPOP_OK;
+    }
+    // after the startup of p has run
+    gpop_status make(gpop_ctx* ctx, const gpop_propagator& p, cudaStream_t s)
+    {
+        JacPoints j;
+        j.n = j.width = p.n;
+        j.err = ctx->err_word.as<unsigned>();
+        j.pos = stage_pos.as<double>();
+        j.M = p.gen_m->as<double>();
+        j.items = 80;
+        j.total = 80 * p.n;
+        j.jac = stage_jac.as<double>();
+        cudaError_t e = launch_jac_points(ctx->table(false), j, ctx->num_sms, s);
+        j.pos = col_pos.as<double>();
+        j.M = p.prop_m->as<double>();
+        j.items = 9;
+        j.total = 9 * p.n;
+        j.jac = col_jac.as<double>();
+        if (e == cudaSuccess)
+            e = launch_jac_points(ctx->table(false), j, ctx->num_sms, s);
+        StartupTangentArgs t;
+        t.n = p.n;
+        t.h = p.h;
+        t.ncorr = p.ncorr;
+        t.stage_jac = stage_jac.as<double>();
+        t.col_jac = col_jac.as<double>();
+        t.out = out.as<double>();
+        if (e == cudaSuccess)
+            e = launch_startup_tangents(t, s);
+        if (e != cudaSuccess)
+            return cuda_fail(ctx, e, "startup tangents");
+        ctx->launches += 4;
+        return GPOP_OK;
+    }
+};
+
+// Forward run of the adjoint: the whole trajectory's positions in traj_r (and v, a when asked for), or,
+// with traj_r NULL, the GJ8 state after the startup and after every 64th step in ckpt.
+gpop_status forward_run(gpop_ctx* ctx, gpop_propagator& p, int32_t steps, double* traj_r, double* traj_v,
+    double* traj_a, DevBuf& ckpt, cudaStream_t s)
+{
+    if (traj_r)
+        return propagator_step(&p, steps, traj_r, traj_v, traj_a, s);
+    const int64_t n = p.n;
     const int nseg = (steps - 1) / kCheckpointSteps + 1;
     const size_t ck_elems = (size_t)kCheckpointArrays * n;
     cudaError_t e = ckpt.ensure(std::max(1, nseg) * ck_elems * sizeof(double));
     if (e != cudaSuccess)
-        return fail(ctx, GPOP_ERR_NOMEM, std::string("checkpoints: ") + cudaGetErrorString(e));
+        return nomem(ctx, "checkpoints", e);
     const double* state_ck = p.state->as<double>() + (size_t)kSs * n;
-    auto tr = [&](double* base, int done) { return base ? base + (size_t)done * 3 * n : nullptr; };
+    gpop_status st;
     int done = std::min(steps, 4); // startup + the replayed steps: the GJ8 state is final here
-    if ((st = propagator_step(&p, done, tr(traj_r, 0), tr(traj_v, 0), tr(traj_a, 0), s)) != GPOP_OK)
+    if ((st = propagator_step(&p, done, nullptr, nullptr, nullptr, s)) != GPOP_OK)
         return st;
-    if ((e = cudaMemcpyAsync(ckpt.p, state_ck, ck_elems * sizeof(double), cudaMemcpyDeviceToDevice, s))
-        != cudaSuccess)
-        return cuda_fail(ctx, e, "checkpoint copy");
-    for (int seg = 0; done < steps; ++seg) {
-        const int target = std::min(steps, (seg + 1) * kCheckpointSteps);
-        if ((st = propagator_step(&p, target - done, tr(traj_r, done), tr(traj_v, done), tr(traj_a, done), s))
-            != GPOP_OK)
+    for (int seg = 0;; ++seg) {
+        if ((e = cudaMemcpyAsync(ckpt.as<double>() + (size_t)seg * ck_elems, state_ck, ck_elems * sizeof(double),
+                 cudaMemcpyDeviceToDevice, s))
+            != cudaSuccess)
+            return cuda_fail(ctx, e, "checkpoint copy");
+        if (seg + 1 >= nseg)
+            return GPOP_OK; // the last segment is run by the reverse sweep alone
+        const int target = (seg + 1) * kCheckpointSteps;
+        if ((st = propagator_step(&p, target - done, nullptr, nullptr, nullptr, s)) != GPOP_OK)
             return st;
         done = target;
-        if (done < steps
-            && (e = cudaMemcpyAsync(ckpt.as<double>() + (size_t)(seg + 1) * ck_elems, state_ck,
-                    ck_elems * sizeof(double), cudaMemcpyDeviceToDevice, s))
-                != cudaSuccess)
-            return cuda_fail(ctx, e, "checkpoint copy");
     }
-    return GPOP_OK;
 }
 
-// Reverse sweep for n_units seeded units over a checkpointed forward run.
-gpop_status run_adjoint(gpop_ctx* ctx, gpop_propagator& p, int32_t steps, int64_t n_obj,
-    const double* r0, const double* v0, const DevBuf& ckpt, int64_t n_units, const int* unit_obj,
-    const int* seed_step0, const double* seeds, double* grad, DevBuf& scratch, cudaStream_t s)
+// Reverse sweep over a forward run. step0: host copy of the units' first seeded step, obj_host of their
+// objects. Device: unit_obj, seed_step0, seeds, grad.
+gpop_status run_adjoint(gpop_ctx* ctx, gpop_propagator& p, int32_t steps, const double* r0, const double* v0,
+    const double* traj_r, const DevBuf& ckpt, StartupTangents& tan, const std::vector<int>& step0,
+    const std::vector<int>& obj_host, const int* unit_obj, const int* seed_step0, const double* seeds, double* grad,
+    cudaStream_t s)
 {
-    const size_t scr = (size_t)kCheckpointSteps * 3 * n_units;
-    cudaError_t e = scratch.ensure(scr * sizeof(double));
-    if (e != cudaSuccess)
-        return fail(ctx, GPOP_ERR_NOMEM, std::string("adjoint scratch: ") + cudaGetErrorString(e));
-    AdjArgs a;
-    a.n_obj = n_obj;
-    a.n_units = n_units;
-    a.unit_obj = unit_obj;
+    const int64_t U = (int64_t)step0.size(), n = p.n;
+    struct Bufs {
+        DevBuf rank, sweep, jac, offset, pos;
+        ~Bufs()
+        {
+            for (DevBuf* b : { &rank, &sweep, &jac, &offset, &pos })
+                b->release();
+        }
+    } B;
+    // ranks: units by their last seeded step, latest first
+    std::vector<int> rank(2 * U); // unit, then object of each rank
+    for (int64_t u = 0; u < U; ++u)
+        rank[u] = (int)u;
+    auto last = [&](int u) { return std::min(step0[u] + 2, steps); };
+    std::stable_sort(rank.begin(), rank.begin() + U, [&](int a, int b) { return last(a) > last(b); });
+    for (int64_t u = 0; u < U; ++u)
+        rank[U + u] = obj_host[rank[u]];
+    cudaError_t e;
+    if ((e = B.rank.ensure(2 * U * sizeof(int))) != cudaSuccess
+        || (e = B.sweep.ensure((size_t)kAdjSweep * U * sizeof(double))) != cudaSuccess)
+        return nomem(ctx, "adjoint buffers", e);
+    if ((e = cudaMemcpyAsync(B.rank.p, rank.data(), 2 * U * sizeof(int), cudaMemcpyHostToDevice, s)) != cudaSuccess)
+        return cuda_fail(ctx, e, "unit ranks");
+    AdjSweepArgs a;
+    a.n_units = U;
+    a.unit = B.rank.as<int>();
     a.seed_step0 = seed_step0;
     a.seeds = seeds;
     a.steps = steps;
     a.h = p.h;
     a.ncorr = ctx->cfg.n_corrections;
-    a.flags = ctx->cfg.flags;
-    a.gen_m = p.gen_m->as<double>();
-    a.prop_m = p.prop_m->as<double>();
-    a.r0 = r0;
-    a.v0 = v0;
-    a.ckpt = ckpt.as<double>();
-    a.scratch = scratch.as<double>();
-    a.grad = grad;
-    a.err = ctx->err_word.as<unsigned>();
-    if ((e = launch_adjoint(ctx->lane_table(false), a, s)) != cudaSuccess)
+    a.sweep = B.sweep.as<double>();
+    a.first = true;
+    int hi = U > 0 ? last(rank[0]) : 0;
+    int64_t cnt = 0; // ranks that take part at the present step
+    if (hi < 5 && (e = launch_adjoint_sweep(a, s)) != cudaSuccess) // nothing to sweep: zero adjoints
         return cuda_fail(ctx, e, "adjoint kernel");
-    ctx->launches++;
+    const size_t limit = std::max<size_t>(kWindowBytes / 72, (size_t)U);
+    while (hi >= 5) {
+        const int floor_step = traj_r ? 5 : std::max(5, (hi - 1) / kCheckpointSteps * kCheckpointSteps + 1);
+        // ranks per step from hi down, as many steps as the Jacobians' budget takes
+        std::vector<int64_t> width;
+        size_t total = 0;
+        int lo = hi + 1;
+        int64_t c = cnt;
+        while (lo > floor_step) {
+            while (c < U && last(rank[c]) >= lo - 1)
+                ++c;
+            if (total > 0 && total + (size_t)c > limit)
+                break;
+            total += (size_t)c;
+            width.push_back(c);
+            --lo;
+        }
+        cnt = width.back();
+        std::vector<int64_t> offset(width.size()); // ascending steps
+        int64_t at = 0;
+        for (size_t i = 0; i < width.size(); ++i) {
+            offset[i] = at;
+            at += width[width.size() - 1 - i];
+        }
+        if ((e = B.jac.ensure(9 * total * sizeof(double))) != cudaSuccess
+            || (e = B.offset.ensure(offset.size() * sizeof(int64_t))) != cudaSuccess)
+            return nomem(ctx, "adjoint Jacobians", e);
+        if ((e = cudaMemcpyAsync(B.offset.p, offset.data(), offset.size() * sizeof(int64_t), cudaMemcpyHostToDevice, s))
+            != cudaSuccess)
+            return cuda_fail(ctx, e, "adjoint window");
+        const double* pos = traj_r ? traj_r + (size_t)(lo - 1) * 3 * n : nullptr;
+        if (!traj_r) { // run the window's segment again from its checkpoint
+            const int seg = (lo - 1) / kCheckpointSteps, from = std::max(5, seg * kCheckpointSteps + 1);
+            if ((e = B.pos.ensure((size_t)(hi - from + 1) * 3 * n * sizeof(double))) != cudaSuccess)
+                return nomem(ctx, "adjoint segment", e);
+            const size_t ck = (size_t)kCheckpointArrays * n;
+            if ((e = cudaMemcpyAsync(p.state->as<double>() + (size_t)kSs * n, ckpt.as<double>() + (size_t)seg * ck,
+                     ck * sizeof(double), cudaMemcpyDeviceToDevice, s))
+                != cudaSuccess)
+                return cuda_fail(ctx, e, "checkpoint restore");
+            p.done = from - 1;
+            const gpop_status st = propagator_step(&p, hi - from + 1, B.pos.as<double>(), nullptr, nullptr, s);
+            if (st != GPOP_OK)
+                return st;
+            pos = B.pos.as<double>() + (size_t)(lo - from) * 3 * n;
+        }
+        JacPoints j;
+        j.n = n;
+        j.pos = pos;
+        j.M = p.prop_m->as<double>() + (size_t)(lo + 4) * 9;
+        j.items = (int)offset.size();
+        j.offset = B.offset.as<int64_t>();
+        j.obj = B.rank.as<int>() + U;
+        j.total = (int64_t)total;
+        j.jac = B.jac.as<double>();
+        j.err = ctx->err_word.as<unsigned>();
+        a.step_lo = lo;
+        a.step_hi = hi;
+        a.jac = j.jac;
+        a.offset = j.offset;
+        a.total = j.total;
+        if ((e = launch_jac_points(ctx->table(false), j, ctx->num_sms, s)) != cudaSuccess
+            || (e = launch_adjoint_sweep(a, s)) != cudaSuccess)
+            return cuda_fail(ctx, e, "adjoint kernel");
+        ctx->launches += 2;
+        a.first = false;
+        hi = lo - 1;
+    }
+    // the startup's part, for the objects whose tangents are at hand, or piece by piece
+    AdjFinishArgs f;
+    f.n_units = U;
+    f.unit = a.unit;
+    f.unit_obj = unit_obj;
+    f.seed_step0 = seed_step0;
+    f.seeds = seeds;
+    f.steps = steps;
+    f.flags = ctx->cfg.flags;
+    f.sweep = a.sweep;
+    f.grad = grad;
+    for (int64_t lo = 0; lo < n; lo += kVarObjects) {
+        f.obj_lo = lo;
+        f.n = std::min(kVarObjects, n - lo);
+        gpop_status st;
+        if (n <= kVarObjects) {
+            if ((st = tan.make(ctx, p, s)) != GPOP_OK)
+                return st;
+        } else {
+            gpop_propagator q;
+            DevBuf rv;
+            struct Free {
+                DevBuf& b;
+                ~Free() { b.release(); }
+            } free_rv { rv };
+            const size_t bytes = (size_t)f.n * 3 * sizeof(double);
+            if ((e = rv.ensure(2 * bytes)) != cudaSuccess || (e = q.own_state.ensure(state_bytes(f.n))) != cudaSuccess)
+                return nomem(ctx, "startup tangents", e);
+            q.ctx = ctx;
+            q.start = p.start;
+            q.h = p.h;
+            q.ncorr = p.ncorr;
+            q.max_steps = 1;
+            q.n = f.n;
+            q.r = rv.as<double>();
+            q.v = q.r + 3 * f.n;
+            q.gen_m = p.gen_m;
+            q.prop_m = p.prop_m;
+            if ((e = cudaMemcpyAsync(q.r, r0 + 3 * lo, bytes, cudaMemcpyDeviceToDevice, s)) != cudaSuccess
+                || (e = cudaMemcpyAsync(q.v, v0 + 3 * lo, bytes, cudaMemcpyDeviceToDevice, s)) != cudaSuccess)
+                return cuda_fail(ctx, e, "startup tangents");
+            if ((st = tan.reserve(ctx, q)) != GPOP_OK || (st = propagator_step(&q, 1, nullptr, nullptr, nullptr, s)) != GPOP_OK
+                || (st = tan.make(ctx, q, s)) != GPOP_OK)
+                return st;
+        }
+        f.startup = tan.out.as<double>();
+        if ((e = launch_adjoint_finish(f, s)) != cudaSuccess)
+            return cuda_fail(ctx, e, "adjoint kernel");
+        ctx->launches++;
+        if (n > kVarObjects && (e = cudaStreamSynchronize(s)) != cudaSuccess) // the piece's buffers are used again
+            return cuda_fail(ctx, e, "adjoint kernel");
+    }
     return check_device_errors(ctx, s);
 }
 
@@ -150,8 +349,8 @@ gpop_status gpop_gravity_jacobian(gpop_ctx* ctx, int64_t n, const double* r_dev,
     if (e != cudaSuccess)
         return cuda_fail(ctx, e, "cudaSetDevice");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if ((e = launch_jacobian(ctx->lane_table(false), n, r_dev, frame9_dev, a_dev, jac_dev,
-             ctx->err_word.as<unsigned>(), s))
+    if ((e = launch_jacobian(ctx->table(false), ctx->lane_table(false), n, r_dev, frame9_dev, a_dev, jac_dev,
+             ctx->err_word.as<unsigned>(), ctx->num_sms, s))
         != cudaSuccess)
         return cuda_fail(ctx, e, "Jacobian kernel");
     ctx->launches++;
@@ -180,38 +379,70 @@ gpop_status gpop_stm(gpop_ctx* ctx, const gpop_time* start, double h, int32_t st
         return GPOP_OK;
     }
     cudaStream_t s = nullptr;
-    ScopedBufs B;
-    DevBuf &gen = B.b[0], &prop = B.b[1], &dr = B.b[2], &dv = B.b[3], &dro = B.b[4], &dvo = B.b[5],
-           &dphi = B.b[6];
-    if ((st = build_epoch_tables(ctx, start, h, steps, gen, prop, s)) != GPOP_OK
-        || (st = upload(ctx, dr, r_in, 3 * n, s)) != GPOP_OK || (st = upload(ctx, dv, v_in, 3 * n, s)) != GPOP_OK)
-        return st;
-    cudaError_t e;
-    if ((e = dro.ensure(3 * n * sizeof(double))) != cudaSuccess || (e = dvo.ensure(3 * n * sizeof(double))) != cudaSuccess
-        || (e = dphi.ensure(36 * n * sizeof(double))) != cudaSuccess)
-        return fail(ctx, GPOP_ERR_NOMEM, std::string("STM buffers: ") + cudaGetErrorString(e));
-    VarArgs a;
-    a.n = n;
-    a.steps = steps;
-    a.h = h;
-    a.ncorr = ctx->cfg.n_corrections;
-    a.flags = ctx->cfg.flags;
-    a.gen_m = gen.as<double>();
-    a.prop_m = prop.as<double>();
-    a.r0 = dr.as<double>();
-    a.v0 = dv.as<double>();
-    a.r_out = dro.as<double>();
-    a.v_out = dvo.as<double>();
-    a.phi = dphi.as<double>();
-    a.err = ctx->err_word.as<unsigned>();
-    if ((e = launch_stm(ctx->lane_table(false), a, s)) != cudaSuccess)
-        return cuda_fail(ctx, e, "STM kernel");
-    ctx->launches++;
-    if ((e = cudaMemcpyAsync(stm_out, dphi.p, 36 * n * sizeof(double), cudaMemcpyDeviceToHost, s)) != cudaSuccess
-        || (r_out && (e = cudaMemcpyAsync(r_out, dro.p, 3 * n * sizeof(double), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
-        || (v_out && (e = cudaMemcpyAsync(v_out, dvo.p, 3 * n * sizeof(double), cudaMemcpyDeviceToHost, s)) != cudaSuccess))
-        return cuda_fail(ctx, e, "STM download");
-    return check_device_errors(ctx, s);
+    for (int64_t lo = 0; lo < n; lo += kVarObjects) {
+        const int64_t m = std::min(kVarObjects, n - lo);
+        ScopedBufs B;
+        DevBuf &dr = B.b[0], &dv = B.b[1], &dphi = B.b[2], &pos = B.b[3], &jac = B.b[4], &sweep = B.b[5];
+        StartupTangents tan;
+        gpop_propagator p;
+        if ((st = upload(ctx, dr, r_in + 3 * lo, 3 * m, s)) != GPOP_OK || (st = upload(ctx, dv, v_in + 3 * lo, 3 * m, s)) != GPOP_OK
+            || (st = begin(ctx, p, start, h, steps, m, dr.as<double>(), dv.as<double>(), s)) != GPOP_OK
+            || (st = tan.reserve(ctx, p)) != GPOP_OK)
+            return st;
+        const int window = (int)std::min<int64_t>(steps, std::max<int64_t>(1, (int64_t)(kWindowBytes / 96) / m));
+        cudaError_t e;
+        if ((e = dphi.ensure(36 * m * sizeof(double))) != cudaSuccess
+            || (e = pos.ensure((size_t)window * 3 * m * sizeof(double))) != cudaSuccess
+            || (e = jac.ensure((size_t)window * 9 * m * sizeof(double))) != cudaSuccess
+            || (e = sweep.ensure((size_t)kStmSweep * 6 * m * sizeof(double))) != cudaSuccess)
+            return nomem(ctx, "STM buffers", e);
+        int done = std::min(steps, 4);
+        if ((st = propagator_step(&p, done, nullptr, nullptr, nullptr, s)) != GPOP_OK || (st = tan.make(ctx, p, s)) != GPOP_OK)
+            return st;
+        StmArgs a;
+        a.n = m;
+        a.steps = steps;
+        a.h = h;
+        a.ncorr = ctx->cfg.n_corrections;
+        a.first = true;
+        a.startup = tan.out.as<double>();
+        a.sweep = sweep.as<double>();
+        a.phi = dphi.as<double>();
+        do {
+            const int w = std::min(window, steps - done);
+            a.step_lo = done + 1;
+            a.step_hi = done + w;
+            a.last = a.step_hi >= steps;
+            if (w > 0) {
+                if ((st = propagator_step(&p, w, pos.as<double>(), nullptr, nullptr, s)) != GPOP_OK)
+                    return st;
+                JacPoints j;
+                j.n = j.width = m;
+                j.pos = pos.as<double>();
+                j.M = p.prop_m->as<double>() + (size_t)(a.step_lo + 4) * 9;
+                j.items = w;
+                j.total = (int64_t)w * m;
+                j.jac = jac.as<double>();
+                j.err = ctx->err_word.as<unsigned>();
+                if ((e = launch_jac_points(ctx->table(false), j, ctx->num_sms, s)) != cudaSuccess)
+                    return cuda_fail(ctx, e, "STM Jacobians");
+                a.jac = j.jac;
+                ctx->launches++;
+            }
+            if ((e = launch_stm_sweep(a, s)) != cudaSuccess)
+                return cuda_fail(ctx, e, "STM kernel");
+            ctx->launches++;
+            a.first = false;
+            done += w;
+        } while (done < steps);
+        if ((e = cudaMemcpyAsync(stm_out + 36 * lo, dphi.p, 36 * m * sizeof(double), cudaMemcpyDeviceToHost, s)) != cudaSuccess
+            || (r_out && (e = cudaMemcpyAsync(r_out + 3 * lo, dr.p, 3 * m * sizeof(double), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
+            || (v_out && (e = cudaMemcpyAsync(v_out + 3 * lo, dv.p, 3 * m * sizeof(double), cudaMemcpyDeviceToHost, s)) != cudaSuccess))
+            return cuda_fail(ctx, e, "STM download");
+        if ((st = check_device_errors(ctx, s)) != GPOP_OK)
+            return st;
+    }
+    return GPOP_OK;
 }
 
 gpop_status gpop_propagate_vjp(gpop_ctx* ctx, const gpop_time* start, double h, int32_t steps, int64_t n,
@@ -234,15 +465,21 @@ gpop_status gpop_propagate_vjp(gpop_ctx* ctx, const gpop_time* start, double h, 
     }
     cudaStream_t s = nullptr;
     ScopedBufs B;
-    DevBuf &dr = B.b[0], &dv = B.b[1], &dr0 = B.b[2], &dv0 = B.b[3], &ck = B.b[4], &scr = B.b[5],
+    DevBuf &dr = B.b[0], &dv = B.b[1], &dr0 = B.b[2], &dv0 = B.b[3], &ck = B.b[4], &traj = B.b[5],
            &dobj = B.b[6], &dstep = B.b[7], &dseed = B.b[8], &dgrad = B.b[9];
+    StartupTangents tan;
     if ((st = upload(ctx, dr, r_in, 3 * n, s)) != GPOP_OK || (st = upload(ctx, dv, v_in, 3 * n, s)) != GPOP_OK
         || (st = upload(ctx, dr0, r_in, 3 * n, s)) != GPOP_OK || (st = upload(ctx, dv0, v_in, 3 * n, s)) != GPOP_OK)
         return st;
+    // the positions of every step when they fit, else checkpoints
+    const size_t traj_bytes = (size_t)steps * 3 * n * sizeof(double);
+    const bool store = traj_bytes <= ctx->adjoint_store && traj.ensure(traj_bytes) == cudaSuccess;
+    if (!store)
+        cudaGetLastError(); // a failed allocation
     gpop_propagator p;
-    if ((st = forward_checkpointed(ctx, p, start, h, steps, n, dr.as<double>(), dv.as<double>(), ck, nullptr,
-             nullptr, nullptr, s))
-        != GPOP_OK)
+    if ((st = begin(ctx, p, start, h, steps, n, dr.as<double>(), dv.as<double>(), s)) != GPOP_OK
+        || (n <= kVarObjects && (st = tan.reserve(ctx, p)) != GPOP_OK)
+        || (st = forward_run(ctx, p, steps, store ? traj.as<double>() : nullptr, nullptr, nullptr, ck, s)) != GPOP_OK)
         return st;
     // seeds on the final state: node 0 at the last step
     std::vector<int> obj(n), step0(n, steps);
@@ -263,8 +500,8 @@ gpop_status gpop_propagate_vjp(gpop_ctx* ctx, const gpop_time* start, double h, 
     if ((e = cudaMemcpyAsync(dobj.p, obj.data(), n * sizeof(int), cudaMemcpyHostToDevice, s)) != cudaSuccess
         || (e = cudaMemcpyAsync(dstep.p, step0.data(), n * sizeof(int), cudaMemcpyHostToDevice, s)) != cudaSuccess)
         return cuda_fail(ctx, e, "seed upload");
-    if ((st = run_adjoint(ctx, p, steps, n, dr0.as<double>(), dv0.as<double>(), ck, n, dobj.as<int>(),
-             dstep.as<int>(), dseed.as<double>(), dgrad.as<double>(), scr, s))
+    if ((st = run_adjoint(ctx, p, steps, dr0.as<double>(), dv0.as<double>(), store ? traj.as<double>() : nullptr, ck,
+             tan, step0, obj, dobj.as<int>(), dstep.as<int>(), dseed.as<double>(), dgrad.as<double>(), s))
         != GPOP_OK)
         return st;
     std::vector<double> g(6 * n);
@@ -299,7 +536,8 @@ gpop_status gpop_miss_gradient(gpop_ctx* ctx, const gpop_time* start, double h, 
     const size_t traj_bytes = (size_t)steps * 3 * n * sizeof(double);
     cudaStream_t s = nullptr;
     ScopedBufs B;
-    DevBuf &dr = B.b[0], &dv = B.b[1], &dr0 = B.b[2], &dv0 = B.b[3], &ck = B.b[4], &scr = B.b[5],
+    StartupTangents tan;
+    DevBuf &dr = B.b[0], &dv = B.b[1], &dr0 = B.b[2], &dv0 = B.b[3], &ck = B.b[4],
            &traj = B.b[6], &dpairs = B.b[7], &units = B.b[8], &dseed = B.b[9], &out = B.b[10],
            &dgrad = B.b[11];
     if ((st = upload(ctx, dr, r_in, 3 * n, s)) != GPOP_OK || (st = upload(ctx, dv, v_in, 3 * n, s)) != GPOP_OK
@@ -317,9 +555,9 @@ gpop_status gpop_miss_gradient(gpop_ctx* ctx, const gpop_time* start, double h, 
     double* tr = traj.as<double>();
     const size_t tn = (size_t)steps * 3 * n;
     gpop_propagator p;
-    if ((st = forward_checkpointed(ctx, p, start, h, steps, n, dr.as<double>(), dv.as<double>(), ck, tr, tr + tn,
-             tr + 2 * tn, s))
-        != GPOP_OK)
+    if ((st = begin(ctx, p, start, h, steps, n, dr.as<double>(), dv.as<double>(), s)) != GPOP_OK
+        || (n <= kVarObjects && (st = tan.reserve(ctx, p)) != GPOP_OK)
+        || (st = forward_run(ctx, p, steps, tr, tr + tn, tr + 2 * tn, ck, s)) != GPOP_OK)
         return st;
     if ((e = cudaMemcpyAsync(dpairs.p, pairs, 2 * n_pairs * sizeof(int32_t), cudaMemcpyHostToDevice, s)) != cudaSuccess)
         return cuda_fail(ctx, e, "pair upload");
@@ -341,9 +579,12 @@ gpop_status gpop_miss_gradient(gpop_ctx* ctx, const gpop_time* start, double h, 
     if ((e = launch_pair_approach(pa, s)) != cudaSuccess)
         return cuda_fail(ctx, e, "pair approach kernel");
     ctx->launches++;
-    traj.release(); // the reverse sweep needs only the checkpoints
-    if ((st = run_adjoint(ctx, p, steps, n, dr0.as<double>(), dv0.as<double>(), ck, U, pa.unit_obj,
-             pa.seed_step0, pa.seeds, dgrad.as<double>(), scr, s))
+    std::vector<int> step0(U), obj(U);
+    if ((e = cudaMemcpy(step0.data(), pa.seed_step0, U * sizeof(int), cudaMemcpyDeviceToHost)) != cudaSuccess)
+        return cuda_fail(ctx, e, "pair approach kernel");
+    std::copy(pairs, pairs + U, obj.begin());
+    if ((st = run_adjoint(ctx, p, steps, dr0.as<double>(), dv0.as<double>(), tr, ck, tan, step0, obj, pa.unit_obj,
+             pa.seed_step0, pa.seeds, dgrad.as<double>(), s))
         != GPOP_OK)
         return st;
     std::vector<double> g(6 * U);

@@ -175,6 +175,8 @@ gpop_status propagator_step(gpop_propagator* p, int steps, double* traj_r, doubl
     a.err = ctx->err_word.as<unsigned>();
     a.r0 = p->r;
     a.v0 = p->v;
+    a.stage_pos = p->stage_pos;
+    a.col_pos = p->col_pos;
     if (!p->started) {
         if ((e = launch_startup(ts, a, ctx->num_sms, s, &lane_ts)) != cudaSuccess)
             return cuda_fail(ctx, e, "startup kernel");
@@ -272,6 +274,8 @@ gpop_status gpop_create(const gpop_config* cfg_in, gpop_ctx** out)
         ctx->steps_per_launch = std::max(1, atoi(spl));
     if (const char* wm = std::getenv("GPOP_WALK_MODE"))
         ctx->walk_mode = std::min((int)kWalkTwoPlain, std::max(0, atoi(wm)));
+    if (const char* mb = std::getenv("GPOP_ADJOINT_STORE_MB"))
+        ctx->adjoint_store = (size_t)std::max(0L, atol(mb)) << 20;
     if (const char* ws = std::getenv("GPOP_TEST_FIRST_WAIT_SPINS"))
         ctx->first_wait_spins = (uint32_t)std::min(1L << 22, std::max(0L, atol(ws)));
     cudaError_t e = cudaSetDevice(cfg.device);

@@ -79,6 +79,9 @@ struct gpop_ctx {
     int num_sms = 148;
     int steps_per_launch = 64;
     int block_override = 0; // GJ8 block size chosen by the tuner (0 = default policy)
+    // largest trajectory (bytes) the adjoint keeps whole; above, segments are run again from checkpoints
+    // (GPOP_ADJOINT_STORE_MB, read when a context is made)
+    size_t adjoint_store = (size_t)32 << 30;
     int walk_mode = 0; // GJ8 triangle walk (WalkMode; 0 = default)
     // first staging wait of every kernel (TableSrc::wait_spins); GPOP_TEST_FIRST_WAIT_SPINS, a
     // test setting, lowers it so that a test can watch the wait give up
@@ -160,6 +163,8 @@ struct gpop_propagator {
     int done = 0;
     bool started = false;
     bool mixed = false;
+    double* stage_pos = nullptr; // StartupArgs::stage_pos, col_pos (variational equations)
+    double* col_pos = nullptr;
     gpop::DevBuf own_state, own_gen, own_prop;
     gpop::DevBuf *state = &own_state, *gen_m = &own_gen, *prop_m = &own_prop;
     ~gpop_propagator()

@@ -1,12 +1,8 @@
 // integrator.cuh -- RK8 startup and mid-corrector device code (lib/gpu_startup/src/gpu_startup.cu),
-// shared by the single-request, batched and variational kernels. A force model F provides
+// for one thread per object. A force model F provides
 //   gen(r, v, step, k, a)  -- acceleration at RK8 stage k of startup step `step` (+-1..4)
 //   prop(r, v, idx, a)     -- acceleration at propagation epoch index idx (t = (idx - 4) h)
 //   kPositionOnly          -- whether a depends on r (and the epoch) alone
-//   agree(bits)            -- bits set for any of the threads that evaluate together
-// The state type T is double, or a value with a tangent (variational equations): the startup is
-// linear in the state apart from the force evaluations, so only + - and scaling by constants are
-// applied to T.
 #pragma once
 #include "common.cuh"
 #include "gj8_tables.cuh"
@@ -121,7 +117,6 @@ template <class F, class T> __device__ bool corrector_correct(const F& f, double
             m.r[c][j] = rn;
         }
     }
-    moved = f.agree(moved);
     for (int c = 0; c < 9; ++c)
         if (moved >> c & 1)
             f.prop(m.r[c], m.v[c], c, m.a[c]);
@@ -148,6 +143,48 @@ __device__ void run_startup(const F& f, double h, int ncorr, const T* r0, const 
     for (int i = 0; i < ncorr; ++i)
         if (!corrector_correct(f, h, m))
             break;
+}
+
+// ---- the pass over all columns at once (the startup pipeline and its tangents) ----
+// One pass of StartupCorrector::Correct (gpu_startup.cu:247-294) from accelerations acc: positions of
+// the eight columns, velocities of columns 5..8, s and S of column 8.
+struct PassResult {
+    double r[9][3], v[4][3], s8[3], S8[3];
+};
+__device__ inline void corrector_pass(double h, const double (&acc)[9][3], const double (&r4)[3], const double (&v4)[3],
+    PassResult& o)
+{
+    const double hinv = 1 / h, h2inv = 1 / (h * h), h2 = h * h;
+    for (int j = 0; j < 3; ++j) {
+        double sb = 0.0, sa = 0.0;
+        for (int k = 0; k < 9; ++k) {
+            sb = fma(c_SA[4][k], acc[k][j], sb);
+            sa = fma(c_GJ[4][k], acc[k][j], sa);
+        }
+        double s[9], S[9];
+        s[4] = fma(hinv, v4[j], -sb);
+        S[4] = fma(h2inv, r4[j], -sa);
+        for (int i = 1; i <= 4; ++i) {
+            s[4 + i] = s[3 + i] + (acc[3 + i][j] + acc[4 + i][j]) / 2;
+            s[4 - i] = s[5 - i] - (acc[5 - i][j] + acc[4 - i][j]) / 2;
+            S[4 + i] = s[3 + i] + S[3 + i] + acc[3 + i][j] / 2;
+            S[4 - i] = -s[5 - i] + S[5 - i] + acc[5 - i][j] / 2;
+        }
+        for (int c = 0; c < 9; ++c) {
+            if (c == 4)
+                continue;
+            double sv = 0.0, sr = 0.0;
+            for (int k = 0; k < 9; ++k) {
+                sv = fma(acc[k][j], c_SA[c][k], sv);
+                sr = fma(acc[k][j], c_GJ[c][k], sr);
+            }
+            if (c > 4)
+                o.v[c - 5][j] = h * (sv + s[c]);
+            o.r[c][j] = h2 * (sr + S[c]);
+        }
+        o.s8[j] = s[8];
+        o.S8[j] = S[8];
+    }
 }
 
 } // namespace gpop

@@ -26,7 +26,6 @@ template <bool MIXED, bool COMP = false> struct ForceGravity {
     GravSmem g;
     const double* gen_m;
     const double* prop_m;
-    __device__ __forceinline__ unsigned agree(unsigned bits) const { return bits; }
     // ForceModel::ComputePropagationAcceleration (force_model.cu:91-109): epoch index idx
     __device__ __forceinline__ void prop(const double* r, const double*, int idx, double* a) const
     {
@@ -54,7 +53,6 @@ struct ForceAnalytic {
     static constexpr bool kMixed = false;
     int kind;
     double h;
-    __device__ __forceinline__ unsigned agree(unsigned bits) const { return bits; }
     __device__ void eval(const double* p, const double* v, double t, double* a) const
     {
         double val = 0.0;
@@ -1015,6 +1013,8 @@ cudaError_t launch_startup(const TableSrc& ts, const PropArgs& a, int num_sms, c
         b.counters = reinterpret_cast<int*>(a.state + (size_t)kStateArrays * a.n);
         b.check = true;
         b.err = a.err;
+        b.stage_pos = a.stage_pos;
+        b.col_pos = a.col_pos;
         return launch_startup_gravity(ts, *lane_ts, b, num_sms, s);
     }
     LaunchShape ls = pick_shape(a.n, 256, num_sms);

@@ -18,6 +18,7 @@
 #include "corrector.cuh"
 #include "gj8_tables.cuh"
 #include "gravity.cuh"
+#include "integrator.cuh"
 #include "lanes.cuh"
 #include "startup.cuh"
 
@@ -145,11 +146,11 @@ __device__ __forceinline__ void to_gcrs(const double* __restrict__ M, double x, 
 
 // ---- RK8 ----
 // Chain 0 of an object runs columns 4 -> 8, chain 1 columns 4 -> 0; K objects in lockstep. eval(M, r, acc)
-// evaluates the K objects, keep.put/get hold the stage accelerations, store(...) writes a value of an
-// object once (one lane of its group).
-template <int K, class Eval, class Keep, class Put>
+// evaluates the K objects, keep.put/get hold the stage accelerations, put(...) writes a value of an
+// object to the state and stage(...) a stage's position (one lane of its group each).
+template <int K, class Eval, class Keep, class Put, class Stage>
 __device__ __forceinline__ void rk8_chain(int chain, double h, const double* gen_m, double (&r)[K][3],
-    double (&v)[K][3], const Eval& eval, const Keep& keep, const Put& put)
+    double (&v)[K][3], const Eval& eval, const Keep& keep, const Put& put, const Stage& stage)
 {
     const double hh = chain == 0 ? h : -h;
 #pragma unroll
@@ -172,6 +173,7 @@ __device__ __forceinline__ void rk8_chain(int chain, double h, const double* gen
                     for (int p = 0; p < st - 1; ++p)
                         q = fma(c_rkn.a[st][p], keep.get(p, k, j), q);
                     t[k][j] = fma(hh, fma(c_rkn.c[st], v[k][j], hh * q), r[k][j]);
+                    stage(k, (s + 4) * 10 + st, j, t[k][j]);
                 }
             eval(gen_m + (size_t)((s + 4) * 10 + st) * 9, t, acc);
 #pragma unroll
@@ -276,7 +278,11 @@ __global__ void __launch_bounds__(256, 1) startup_rk8_kernel(TableSrc ts, Startu
         if (live[k])
             a.state[(size_t)slot * a.n + obj[k]] = x;
     };
-    rk8_chain<K>(chain, src.h, src.gen_m, r, v, eval, KeepLocal<K> { kept }, put);
+    auto stage = [&](int k, int i, int j, double x) {
+        if (a.stage_pos && live[k])
+            a.stage_pos[((size_t)i * 3 + j) * a.n + obj[k]] = x;
+    };
+    rk8_chain<K>(chain, src.h, src.gen_m, r, v, eval, KeepLocal<K> { kept }, put, stage);
 }
 
 // Stage accelerations of a lane group in shared memory, written by its first lane.
@@ -343,7 +349,11 @@ __global__ void __launch_bounds__(384, 1) startup_rk8_team_kernel(TableSrc ts, S
             a.state[(size_t)slot * a.n + o] = x;
     };
     using Team = typename TeamOf<WARPS>::type;
-    rk8_chain<1>(chain, src.h, src.gen_m, r, v, eval, KeepShared<Team> { own, team }, put);
+    auto stage = [&](int, int i, int j, double x) {
+        if (a.stage_pos && team.l == 0)
+            a.stage_pos[((size_t)i * 3 + j) * a.n + o] = x;
+    };
+    rk8_chain<1>(chain, src.h, src.gen_m, r, v, eval, KeepShared<Team> { own, team }, put, stage);
 }
 
 // ---- accelerations of columns ----
@@ -451,47 +461,6 @@ __global__ void __launch_bounds__(384, 1) startup_eval_team_kernel(TableSrc ts, 
 }
 
 // ---- corrector ----
-// One pass of StartupCorrector::Correct (gpu_startup.cu:247-294) from accelerations acc: positions of
-// the eight columns, velocities of columns 5..8, s and S of column 8.
-struct PassResult {
-    double r[9][3], v[4][3], s8[3], S8[3];
-};
-__device__ void corrector_pass(double h, const double (&acc)[9][3], const double (&r4)[3], const double (&v4)[3],
-    PassResult& o)
-{
-    const double hinv = 1 / h, h2inv = 1 / (h * h), h2 = h * h;
-    for (int j = 0; j < 3; ++j) {
-        double sb = 0.0, sa = 0.0;
-        for (int k = 0; k < 9; ++k) {
-            sb = fma(c_SA[4][k], acc[k][j], sb);
-            sa = fma(c_GJ[4][k], acc[k][j], sa);
-        }
-        double s[9], S[9];
-        s[4] = fma(hinv, v4[j], -sb);
-        S[4] = fma(h2inv, r4[j], -sa);
-        for (int i = 1; i <= 4; ++i) {
-            s[4 + i] = s[3 + i] + (acc[3 + i][j] + acc[4 + i][j]) / 2;
-            s[4 - i] = s[5 - i] - (acc[5 - i][j] + acc[4 - i][j]) / 2;
-            S[4 + i] = s[3 + i] + S[3 + i] + acc[3 + i][j] / 2;
-            S[4 - i] = -s[5 - i] + S[5 - i] + acc[5 - i][j] / 2;
-        }
-        for (int c = 0; c < 9; ++c) {
-            if (c == 4)
-                continue;
-            double sv = 0.0, sr = 0.0;
-            for (int k = 0; k < 9; ++k) {
-                sv = fma(acc[k][j], c_SA[c][k], sv);
-                sr = fma(acc[k][j], c_GJ[c][k], sr);
-            }
-            if (c > 4)
-                o.v[c - 5][j] = h * (sv + s[c]);
-            o.r[c][j] = h2 * (sr + S[c]);
-        }
-        o.s8[j] = s[8];
-        o.S8[j] = S[8];
-    }
-}
-
 // Corrector pass `it` of every object that is not done: lists the columns whose accelerations the next
 // evaluation must renew. The rule is correct_position's, over the eight columns at once:
 // - no column's position moves by a bit: every further pass would repeat this one, done;
@@ -623,6 +592,9 @@ __global__ void __launch_bounds__(128) startup_finish_kernel(StartupArgs a)
     double* st = a.state + o;
     const bool fix_q3 = (a.flags & 2u) != 0;
     double r[4][3], v[4][3], e[4][3];
+    if (a.col_pos)
+        for (int i = 0; i < 27; ++i)
+            a.col_pos[(size_t)i * n + o] = st[(kSr + i) * n];
     for (int k = 0; k < 4; ++k)
         for (int j = 0; j < 3; ++j) {
             r[k][j] = st[(kSr + (5 + k) * 3 + j) * n];

@@ -22,6 +22,10 @@ struct StartupArgs {
     int* counters = nullptr; // kStartupCounters: evaluations listed by each corrector pass
     bool check = false; // raise kErrBadInput for states gravity cannot take
     unsigned* err = nullptr;
+    // for the variational equations (may be NULL): positions of the 80 RK8 stages, in the order of gen_m,
+    // and of the nine columns at the end, [.][3][n]
+    double* stage_pos = nullptr;
+    double* col_pos = nullptr;
 };
 
 // plain: the plain table, lanes: the lane-layout table of the same precision.

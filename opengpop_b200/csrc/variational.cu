@@ -1,380 +1,451 @@
 // variational.cu -- forward variational equations (6x6 STM), the adjoint (reverse sweep) of the
 // GJ8 propagation, and the closest approach of listed pairs with miss-distance seeds.
 //
-// Every object (STM) or adjoint unit runs on kVarLanes = 8 lanes of a warp. The lanes split the
-// gravity columns (lanes.cuh) and share the acceleration and its Jacobian; lane d < 6 carries the
-// tangent of initial-state direction d. The integrator is the same discrete map as the forward
-// propagation (startup: integrator.cuh; GJ8 step: gpu_propagator.cu:28-119 as in gj8_kernel),
-// so the tangents and adjoints are the derivatives of that map with one simplification: the
-// Jacobian of a GJ8 step's corrector passes is taken once, at the step's last evaluation point
-// (the corrector converges, so the passes' iterates differ by far less than the truncation error);
-// the startup is differentiated exactly. Forward tangents and the reverse sweep make the same
-// choice, so they are exact transposes of each other.
+// Tangents and adjoints are the derivatives of the discrete map of the forward propagation (startup, GJ8
+// steps: gpu_propagator.cu:28-119) with one simplification: the Jacobian of a step's corrector passes is
+// taken once, at the step's position (the corrector converges, so the passes' iterates differ by far less
+// than the truncation error); the startup's columns likewise. Forward tangents and the reverse sweep make
+// the same choice, so they are exact transposes of each other.
+//
+// The Jacobians depend on the positions alone, not on the tangents. So the forward propagation runs with
+// the propagation's own kernels and keeps its positions (per step, and of the startup's 80 stages and nine
+// columns); one kernel makes all the Jacobians, a (point, object) per thread with the table read by
+// broadcast; and the tangents or the adjoint follow as short linear recurrences, a thread per direction or
+// unit. One kernel of 8 lanes per object that walked primal, Jacobian and tangents in turn (and ran the
+// segments of the reverse sweep twice) measured, with the corrector's early end: 1,000 STMs over 360 steps
+// 43.8 ms, 1,200 miss gradients over 720 steps 75 ms for the sweep alone; FIGURES
 //
 // Adjoint of one GJ8 step n (K = number of corrector passes, iterates r(0..K-1), a(i) = f(r(i))):
 //   S' = S + s + h8/2,  r(0) = h^2 (sum_c GJ[9][c] h_c + S'),  s1 = sum_c SA[8][c] h_(c+1),
 //   s2 = sum_c GJ[8][c] h_(c+1),  r(i+1) = h^2 (s2 + GJ[8][8] a(i) + S'),
 //   s_n = s + (a(K-1) + h8)/2,  v_n = h (s1 + SA[8][8] a(K-1) + s_n),  history <- (h_1..h_8, a(K-1)).
-// The reverse pass below applies the transposes of these maps in the opposite order, with J^T at
-// the last evaluation point r(K-1), recomputed from the checkpoint of the step's 64-step segment.
+// The reverse pass below applies the transposes of these maps in the opposite order.
 #include "common.cuh"
-#include "corrector.cuh"
 #include "gj8_tables.cuh"
-#include "gravity.cuh"
 #include "hermite.cuh"
 #include "integrator.cuh"
-#include "lanes.cuh"
-#include "tangent.cuh"
+#include "jacobian.cuh"
 #include "variational.cuh"
+
+#include <algorithm>
 
 namespace gpop {
 
 namespace {
 
-// Tangent force: a(r) and J(r) dr, epoch tables as in ForceGravity (force_model.cu:59-109).
-struct LaneForceTan {
-    static constexpr bool kPositionOnly = true;
-    GravSmem g;
-    int l, P;
-    unsigned mask;
-    const double* gen_m;
-    const double* prop_m;
-    // the lanes carry different tangents and evaluate together
-    __device__ __forceinline__ unsigned agree(unsigned bits) const { return __reduce_or_sync(mask, bits); }
-    __device__ __forceinline__ void eval(const double* M, const Tan* r, Tan* a) const
-    {
-        const double rv[3] = { r[0].v, r[1].v, r[2].v };
-        double av[3], J[3][3];
-        gravity_jac_gcrs_lanes(g, l, P, M, rv, av, J, mask);
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-            a[i] = Tan(av[i], J[i][0] * r[0].d + J[i][1] * r[1].d + J[i][2] * r[2].d);
-    }
-    __device__ __forceinline__ void prop(const Tan* r, const Tan*, int idx, Tan* a) const
-    {
-        eval(prop_m + (size_t)idx * 9, r, a);
-    }
-    __device__ __forceinline__ void gen(const Tan* r, const Tan*, int step, int k, Tan* a) const
-    {
-        const int s = step > 0 ? step - 1 : step;
-        eval(gen_m + (size_t)((s + 4) * 10 + k) * 9, r, a);
-    }
-};
-
-// One GJ8 step (predict, then ncorr evaluate-correct passes) on a history held in logical order
-// (hist[8] newest). eval(r, a) evaluates the force, a function of the position alone, at r.
-template <class T, class Eval>
-__device__ __forceinline__ void gj8_step(const Eval& eval, double h, int ncorr, T (&hist)[9][3],
-    T (&s)[3], T (&S)[3], T (&r)[3], T (&v)[3])
+__device__ __forceinline__ bool bind_plain64(uint8_t* smem, const TableSrc& ts, unsigned* err, GravSmem& g)
 {
-    T s1[3], s2[3], prev[3], a7[3], a8[3];
-#pragma unroll
-    for (int j = 0; j < 3; ++j) { // Predictor::Predict (dev_functions.cu:20-50)
-        T vt = 0.0, rt = 0.0;
-#pragma unroll
-        for (int c = 0; c < 9; ++c) {
-            vt = fma(hist[c][j], c_SA[9][c], vt);
-            rt = fma(hist[c][j], c_GJ[9][c], rt);
+    const bool ok = stage_to_smem(smem + 128, ts.src, ts.bytes, reinterpret_cast<uint64_t*>(smem), err, ts.wait_spins);
+    g.L = ts.L;
+    g.Lt = ts.L;
+    g.radius = ts.radius;
+    g.gm = ts.gm;
+    g.t64 = reinterpret_cast<const GravEntry64*>(smem + 128);
+    g.t32 = nullptr;
+    return ok;
+}
+
+} // namespace
+
+// ---- Jacobians of many points ----
+__global__ void __launch_bounds__(256, 1) jac_points_kernel(TableSrc ts, JacPoints a)
+{
+    extern __shared__ __align__(128) uint8_t smem[];
+    GravSmem g;
+    if (!bind_plain64(smem, ts, a.err, g))
+        return;
+    const int64_t T = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < a.total; t += T) {
+        int64_t i, u;
+        if (a.offset) { // the item whose range holds t
+            int lo = 0, hi = a.items - 1;
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) / 2;
+                if (a.offset[mid] <= t)
+                    lo = mid;
+                else
+                    hi = mid - 1;
+            }
+            i = lo;
+            u = t - a.offset[lo];
+        } else {
+            i = t / a.width;
+            u = t - i * a.width;
         }
-        S[j] += s[j] + hist[8][j] / 2;
-        v[j] = (vt + s[j] + hist[8][j] / 2) * h;
-        r[j] = (rt + S[j]) * h * h;
-        T c1 = 0.0, c2 = 0.0;
+        const int64_t o = a.obj ? a.obj[u] : u;
+        double r[3], acc[3], J[3][3];
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-            c1 = fma(hist[c + 1][j], c_SA[8][c], c1);
-            c2 = fma(hist[c + 1][j], c_GJ[8][c], c2);
-        }
-        s1[j] = c1;
-        s2[j] = c2;
-        prev[j] = s[j];
-        a7[j] = hist[8][j];
-        a8[j] = 0.0;
+        for (int j = 0; j < 3; ++j)
+            r[j] = a.pos[(i * 3 + j) * a.n + o];
+        gravity_jac_gcrs<false>(g, 0, 1, a.M + (size_t)i * 9, r, acc, J, 0u);
+#pragma unroll
+        for (int k = 0; k < 9; ++k)
+            a.jac[(int64_t)k * a.total + t] = J[k / 3][k % 3];
     }
-    for (int it = 0; it < ncorr; ++it) { // GpuPropagator::Correct (gpu_propagator.cu:61-119)
-        eval(r, a8);
+}
+
+namespace {
+
+__device__ __forceinline__ void load_jac(const double* __restrict__ jac, int64_t total, int64_t t, double (&J)[3][3])
+{
+#pragma unroll
+    for (int k = 0; k < 9; ++k)
+        J[k / 3][k % 3] = __ldg(jac + (int64_t)k * total + t);
+}
+
+__device__ __forceinline__ void mul(const double (&J)[3][3], const double (&x)[3], double (&y)[3])
+{
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        y[i] = J[i][0] * x[0] + J[i][1] * x[1] + J[i][2] * x[2];
+}
+
+} // namespace
+
+// ---- startup tangents ----
+// RK8 (gpu_startup.cu:108-144) of direction dir and chain: thread t = ((chain 6 + dir) n + o). The stage
+// states as in rk8_step; the columns' position tangents go to out slot (col 3 + j).
+__global__ void __launch_bounds__(128) rk8_tangent_kernel(StartupTangentArgs a)
+{
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= 12 * a.n)
+        return;
+    const int64_t n = a.n, o = t % n;
+    const int cd = (int)(t / n), chain = cd / 6, dir = cd % 6;
+    const double hh = chain == 0 ? a.h : -a.h;
+    double r[3], v[3], Kx[10][3], Kv[10][3];
+    for (int j = 0; j < 3; ++j) {
+        r[j] = dir == j ? 1.0 : 0.0;
+        v[j] = dir == 3 + j ? 1.0 : 0.0;
+        if (chain == 0)
+            a.out[((int64_t)(4 * 3 + j) * 6 + dir) * n + o] = r[j];
+    }
+    for (int i = 1; i <= 4; ++i) {
+        const int s = chain == 0 ? i - 1 : -i;
+        for (int k = 0; k < 10; ++k) {
+            double x[3];
+            for (int j = 0; j < 3; ++j) {
+                double sx = 0.0, sv = 0.0;
+                for (int p = 0; p < k; ++p) {
+                    sx = fma(c_RKA[k - 1][p], Kx[p][j], sx);
+                    sv = fma(c_RKA[k - 1][p], Kv[p][j], sv);
+                }
+                x[j] = fma(hh, sx, r[j]);
+                Kx[k][j] = fma(hh, sv, v[j]);
+            }
+            double J[3][3];
+            load_jac(a.stage_jac, 80 * n, (int64_t)((s + 4) * 10 + k) * n + o, J);
+            mul(J, x, Kv[k]);
+        }
+        const int col = chain == 0 ? 4 + i : 4 - i;
+        for (int j = 0; j < 3; ++j) {
+            double sx = 0.0, sv = 0.0;
+            for (int k = 0; k < 10; ++k) {
+                sx = fma(Kx[k][j], c_RKB[k], sx);
+                sv = fma(Kv[k][j], c_RKB[k], sv);
+            }
+            v[j] = fma(hh, sv, v[j]);
+            r[j] = fma(hh, sx, r[j]);
+            a.out[((int64_t)(col * 3 + j) * 6 + dir) * n + o] = r[j];
+        }
+    }
+}
+
+// The mid-corrector's passes of direction dir, with one Jacobian per column: out slots 0..26 the
+// accelerations, 27..32 s and S of column 8, 33..44 and 45..56 positions and velocities of columns 5..8.
+__global__ void __launch_bounds__(128) corrector_tangent_kernel(StartupTangentArgs a)
+{
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= 6 * a.n)
+        return;
+    const int64_t n = a.n, o = t % n;
+    const int dir = (int)(t / n);
+    double* out = a.out + (int64_t)dir * n + o;
+    auto slot = [&](int k) -> double& { return out[(int64_t)k * 6 * n]; };
+    double dr[9][3], da[9][3], r4[3], v4[3];
+    for (int c = 0; c < 9; ++c)
+        for (int j = 0; j < 3; ++j)
+            dr[c][j] = slot(c * 3 + j);
+    for (int j = 0; j < 3; ++j) {
+        r4[j] = dir == j ? 1.0 : 0.0;
+        v4[j] = dir == 3 + j ? 1.0 : 0.0;
+    }
+    auto accel = [&](int c) {
+        double J[3][3];
+        load_jac(a.col_jac, 9 * n, (int64_t)c * n + o, J);
+        mul(J, dr[c], da[c]);
+    };
+    for (int c = 0; c < 9; ++c)
+        accel(c);
+    PassResult p;
+    for (int it = 0; it < a.ncorr; ++it) {
+        corrector_pass(a.h, da, r4, v4, p);
         bool same = true;
+        for (int c = 0; c < 9; ++c) {
+            if (c == 4)
+                continue;
+            for (int j = 0; j < 3; ++j) {
+                same = same && same_bits(dr[c][j], p.r[c][j]);
+                dr[c][j] = p.r[c][j];
+            }
+            accel(c);
+        }
+        if (same) // every further pass repeats this one
+            break;
+    }
+    for (int j = 0; j < 3; ++j) {
+        for (int c = 0; c < 9; ++c)
+            slot(c * 3 + j) = da[c][j];
+        slot(27 + j) = p.s8[j];
+        slot(30 + j) = p.S8[j];
+        for (int k = 0; k < 4; ++k) {
+            slot(33 + k * 3 + j) = dr[5 + k][j];
+            slot(45 + k * 3 + j) = p.v[k][j];
+        }
+    }
+}
+
+// ---- forward variational equations: steps [step_lo, step_hi] of every (direction, object) ----
+__global__ void __launch_bounds__(128) stm_sweep_kernel(StmArgs a)
+{
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t n = a.n, W = 6 * n;
+    if (t >= W)
+        return;
+    const int64_t o = t % n;
+    const int dir = (int)(t / n);
+    const double h = a.h;
+    double hist[9][3], s[3], S[3], r[3], v[3];
+    double* st = a.sweep + t; // 39 arrays of 6 n: history, s, S, r, v
+    if (a.first) {
+        const double* T = a.startup + t;
+        const int rep = a.steps < 4 ? a.steps : 4; // steps 1..4 replay the startup columns
+        for (int j = 0; j < 3; ++j) {
+            for (int c = 0; c < 9; ++c)
+                hist[c][j] = T[(int64_t)(c * 3 + j) * W];
+            s[j] = T[(int64_t)(27 + j) * W];
+            S[j] = T[(int64_t)(30 + j) * W];
+            r[j] = T[(int64_t)(33 + (rep - 1) * 3 + j) * W];
+            v[j] = T[(int64_t)(45 + (rep - 1) * 3 + j) * W];
+        }
+    } else {
+        for (int j = 0; j < 3; ++j) {
+            for (int c = 0; c < 9; ++c)
+                hist[c][j] = st[(int64_t)(c * 3 + j) * W];
+            s[j] = st[(int64_t)(27 + j) * W];
+            S[j] = st[(int64_t)(30 + j) * W];
+            r[j] = st[(int64_t)(33 + j) * W];
+            v[j] = st[(int64_t)(36 + j) * W];
+        }
+    }
+    const int64_t total = (int64_t)(a.step_hi - a.step_lo + 1) * n;
+    double Jn[3][3];
+    if (a.step_lo <= a.step_hi)
+        load_jac(a.jac, total, o, Jn);
+    for (int step = a.step_lo; step <= a.step_hi; ++step) {
+        double J[3][3];
+#pragma unroll
+        for (int k = 0; k < 9; ++k)
+            J[k / 3][k % 3] = Jn[k / 3][k % 3];
+        if (step < a.step_hi) // the next step's Jacobian loads during this step
+            load_jac(a.jac, total, (int64_t)(step + 1 - a.step_lo) * n + o, Jn);
+        double s1[3], s2[3], prev[3], a7[3], a8[3];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) { // as gj8_kernel
+            double rt = 0.0;
+#pragma unroll
+            for (int c = 0; c < 9; ++c)
+                rt = fma(hist[c][j], c_GJ[9][c], rt);
+            S[j] += s[j] + hist[8][j] / 2;
+            r[j] = (rt + S[j]) * h * h;
+            double c1 = 0.0, c2 = 0.0;
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                c1 = fma(hist[c + 1][j], c_SA[8][c], c1);
+                c2 = fma(hist[c + 1][j], c_GJ[8][c], c2);
+            }
+            s1[j] = c1;
+            s2[j] = c2;
+            prev[j] = s[j];
+            a7[j] = hist[8][j];
+            a8[j] = 0.0;
+        }
+        for (int it = 0; it < a.ncorr; ++it) {
+            mul(J, r, a8);
+            bool same = true;
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                const double rn = h * h * (s2[j] + a8[j] * c_GJ[8][8] + S[j]);
+                same = same && same_bits(rn, r[j]);
+                r[j] = rn;
+            }
+            if (same) // every further pass repeats this one
+                break;
+        }
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
             s[j] = prev[j] + (a8[j] + a7[j]) / 2;
             v[j] = h * (s1[j] + a8[j] * c_SA[8][8] + s[j]);
-            const T rn = h * h * (s2[j] + a8[j] * c_GJ[8][8] + S[j]);
-            same = same && same_bits(rn, r[j]);
-            r[j] = rn;
-        }
-        if (same) // the passes left would return the same bits (as gj8_kernel)
-            break;
-    }
 #pragma unroll
-    for (int c = 0; c < 8; ++c)
-#pragma unroll
-        for (int j = 0; j < 3; ++j)
-            hist[c][j] = hist[c + 1][j];
-#pragma unroll
-    for (int j = 0; j < 3; ++j)
-        hist[8][j] = a8[j];
-}
-
-__device__ __forceinline__ bool stage_table64(uint8_t* smem, const TableSrc& ts, unsigned* err, GravSmem& g)
-{
-    return bind_lane_table(smem, ts, err, g); // FP64 lane-layout table
-}
-
-} // namespace
-
-// ---- forward variational equations ----
-__global__ void __launch_bounds__(256, 1) stm_kernel(TableSrc ts, VarArgs a)
-{
-    extern __shared__ __align__(128) uint8_t smem[];
-    GravSmem g;
-    if (!stage_table64(smem, ts, a.err, g))
-        return;
-    const int P = kVarLanes;
-    const int64_t gid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / P;
-    const int l = (int)(threadIdx.x % P);
-    if (gid >= a.n)
-        return; // the lanes of a group share gid; shuffles stay inside the group
-    const int64_t o = gid;
-    const unsigned mask = 0xffu << (threadIdx.x & 24);
-    const int dir = l < 6 ? l : -1;
-    LaneForceTan f { g, l, P, mask, a.gen_m, a.prop_m };
-    Tan r0[3], v0[3];
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-        r0[j] = Tan(a.r0[o * 3 + j], dir == j ? 1.0 : 0.0);
-        v0[j] = Tan(a.v0[o * 3 + j], dir == 3 + j ? 1.0 : 0.0);
-    }
-    // primal state (every lane) and the tangent of this lane's direction
-    double hist[9][3], s[3], S[3], r[3], v[3], dh[9][3], ds[3], dS[3], dr[3], dv[3];
-    {
-        StartupMatsT<Tan> m; // the startup: exact tangents, Jacobian at every evaluation
-        run_startup(f, a.h, a.ncorr, r0, v0, m);
-        const int rep = a.steps < 4 ? a.steps : 4; // steps 1..4 replay the startup columns
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            for (int c = 0; c < 9; ++c) {
-                hist[c][j] = m.a[c][j].v;
-                dh[c][j] = m.a[c][j].d;
-            }
-            s[j] = m.s[8][j].v;
-            ds[j] = m.s[8][j].d;
-            S[j] = m.S[8][j].v;
-            dS[j] = m.S[8][j].d;
-            r[j] = m.r[4 + rep][j].v;
-            dr[j] = m.r[4 + rep][j].d;
-            v[j] = m.v[4 + rep][j].v;
-            dv[j] = m.v[4 + rep][j].d;
+            for (int c = 0; c < 8; ++c)
+                hist[c][j] = hist[c + 1][j];
+            hist[8][j] = a8[j];
         }
     }
-    for (int step = 5; step <= a.steps; ++step) {
-        const double* M = a.prop_m + (size_t)(step + 4) * 9;
-        // primal passes; the Jacobian at the last evaluation point serves every pass of the
-        // tangent step (as in the reverse sweep)
-        double rl[3];
-        auto evalp = [&](const double* rr, double* aa) {
-            for (int j = 0; j < 3; ++j)
-                rl[j] = rr[j];
-            gravity_gcrs_lanes<false>(g, l, P, M, rr, aa, mask);
-        };
-        gj8_step<double>(evalp, a.h, a.ncorr, hist, s, S, r, v);
-        double av[3], J[3][3];
-        gravity_jac_gcrs_lanes(g, l, P, M, rl, av, J, mask);
-        auto evalt = [&](const double* rr, double* aa) {
-#pragma unroll
-            for (int i = 0; i < 3; ++i)
-                aa[i] = J[i][0] * rr[0] + J[i][1] * rr[1] + J[i][2] * rr[2];
-        };
-        gj8_step<double>(evalt, a.h, a.ncorr, dh, ds, dS, dr, dv);
-    }
-    if (l == 0 && a.r_out)
-        for (int j = 0; j < 3; ++j) {
-            a.r_out[o * 3 + j] = r[j];
-            a.v_out[o * 3 + j] = v[j];
-        }
-    if (dir >= 0)
-        for (int i = 0; i < 3; ++i) {
-            a.phi[(o * 6 + i) * 6 + dir] = dr[i];
-            a.phi[(o * 6 + 3 + i) * 6 + dir] = dv[i];
-        }
-}
-
-// ---- adjoint ----
-namespace {
-
-// Reverse of one GJ8 step (see the header comment). hb: history adjoints in logical order after
-// the step on entry, before it on exit; sb, Sb: adjoints of s and S likewise.
-// iter: the step's last evaluation point r(K-1) (3 values, stride apart); its Jacobian stands for
-// every corrector pass (the corrector converges: the iterates differ by far less than the step's
-// truncation error, and the forward tangents make the same choice).
-__device__ __forceinline__ void gj8_reverse_step(const GravSmem& g, int l, int P, unsigned mask,
-    const double* M, double h, int ncorr, const double* iter, int64_t stride, const double* seed,
-    double (&hb)[9][3], double (&sb)[3], double (&Sb)[3])
-{
-    const double h2 = h * h;
-    double abar[3], s1b[3], s2b[3], Spb[3], prevb[3], a7b[3];
-#pragma unroll
-    for (int j = 0; j < 3; ++j)
-        abar[j] = hb[8][j] + (seed ? seed[6 + j] : 0.0);
-#pragma unroll
-    for (int c = 8; c >= 1; --c)
-#pragma unroll
-        for (int j = 0; j < 3; ++j)
-            hb[c][j] = hb[c - 1][j];
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-        hb[0][j] = 0.0;
-        const double rb = seed ? seed[j] : 0.0, vb = seed ? seed[3 + j] : 0.0;
-        const double sK = sb[j] + h * vb; // s_n feeds v_n = h (s1 + SA88 a + s_n)
-        s1b[j] = h * vb;
-        abar[j] += h * c_SA[8][8] * vb + sK / 2;
-        prevb[j] = sK;
-        a7b[j] = sK / 2;
-        s2b[j] = h2 * rb;
-        abar[j] += h2 * c_GJ[8][8] * rb;
-        Spb[j] = Sb[j] + h2 * rb;
-    }
-    double J[3][3];
-    {
-        double ri[3], av[3];
-#pragma unroll
-        for (int j = 0; j < 3; ++j)
-            ri[j] = iter[(int64_t)j * stride];
-        gravity_jac_gcrs_lanes(g, l, P, M, ri, av, J, mask);
-    }
-    for (int it = ncorr - 1; it >= 0; --it) {
-        double rb[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-            rb[k] = J[0][k] * abar[0] + J[1][k] * abar[1] + J[2][k] * abar[2];
-        if (it >= 1) {
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                s2b[j] += h2 * rb[j];
-                Spb[j] += h2 * rb[j];
-                abar[j] = h2 * c_GJ[8][8] * rb[j];
-            }
-        } else {
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-#pragma unroll
-                for (int c = 0; c < 9; ++c)
-                    hb[c][j] += h2 * c_GJ[9][c] * rb[j];
-                Spb[j] += h2 * rb[j];
-            }
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-#pragma unroll
-        for (int c = 0; c < 8; ++c)
-            hb[c + 1][j] += c_SA[8][c] * s1b[j] + c_GJ[8][c] * s2b[j];
-        hb[8][j] += a7b[j] + Spb[j] / 2; // a7 = h8, and S' = S + s + h8/2
-        Sb[j] = Spb[j];
-        sb[j] = prevb[j] + Spb[j];
-    }
-}
-
-} // namespace
-
-__global__ void __launch_bounds__(256, 1) adjoint_kernel(TableSrc ts, AdjArgs a)
-{
-    extern __shared__ __align__(128) uint8_t smem[];
-    GravSmem g;
-    if (!stage_table64(smem, ts, a.err, g))
-        return;
-    const int P = kVarLanes;
-    const int64_t gid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / P;
-    const int l = (int)(threadIdx.x % P);
-    if (gid >= a.n_units)
-        return; // groups run independently: every shuffle and warp sync names the group only
-    const int64_t u = gid;
-    const unsigned mask = 0xffu << (threadIdx.x & 24);
-    const int64_t o = a.unit_obj[u];
-    const int64_t n = a.n_obj, U = a.n_units;
-    const int N = a.steps, K = a.ncorr;
-    const int k0 = a.seed_step0[u];
-    const int kend = k0 + 2 < N ? k0 + 2 : N;
-    const double* seeds = a.seeds + u * 27;
-    double hb[9][3], sb[3], Sb[3];
-#pragma unroll
     for (int j = 0; j < 3; ++j) {
         for (int c = 0; c < 9; ++c)
-            hb[c][j] = 0.0;
-        sb[j] = Sb[j] = 0.0;
+            st[(int64_t)(c * 3 + j) * W] = hist[c][j];
+        st[(int64_t)(27 + j) * W] = s[j];
+        st[(int64_t)(30 + j) * W] = S[j];
+        st[(int64_t)(33 + j) * W] = r[j];
+        st[(int64_t)(36 + j) * W] = v[j];
+        if (a.last) {
+            a.phi[(o * 6 + j) * 6 + dir] = r[j];
+            a.phi[(o * 6 + 3 + j) * 6 + dir] = v[j];
+        }
     }
-    if (kend >= 5) {
-        for (int seg = (kend - 1) / kCheckpointSteps; seg >= 0; --seg) {
-            const int lo = seg == 0 ? 5 : seg * kCheckpointSteps + 1;
-            const int hi = (seg + 1) * kCheckpointSteps < kend ? (seg + 1) * kCheckpointSteps : kend;
-            if (lo > hi)
-                continue;
-            // recompute the segment from its checkpoint, keeping every corrector iterate
-            const double* ck = a.ckpt + (size_t)seg * kCheckpointArrays * n;
-            double hist[9][3], s[3], S[3], r[3], v[3];
-            const int ring0 = (lo - 5) % 9;
+}
+
+// ---- adjoint: steps [step_lo, step_hi] of every unit, in reverse ----
+// hb: history adjoints in logical order after the step on entry, before it on exit; sb, Sb: adjoints of
+// s and S likewise. Units are in rank order (the latest last step first): at a step the ranks whose last
+// step is not before it take part, and its Jacobians lie at offset[step - step_lo] + rank.
+__global__ void __launch_bounds__(64) adjoint_sweep_kernel(AdjSweepArgs a)
+{
+    const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; // rank
+    if (u >= a.n_units)
+        return;
+    const int64_t U = a.n_units, unit = a.unit ? a.unit[u] : u;
+    const double h = a.h, h2 = h * h;
+    const int k0 = a.seed_step0[unit];
+    const int kend = min(k0 + 2, a.steps);
+    const double* seeds = a.seeds + unit * 27;
+    double hb[9][3], sb[3], Sb[3];
+    double* st = a.sweep + u;
 #pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                s[j] = ck[(0 + j) * n + o]; // arrays kSs, kSb, kHist relative to kSs
-                S[j] = ck[(3 + j) * n + o];
-                for (int c = 0; c < 9; ++c) {
-                    const int slot = (ring0 + c) % 9;
-                    hist[c][j] = ck[(6 + slot * 3 + j) * n + o];
+    for (int j = 0; j < 3; ++j) {
+#pragma unroll
+        for (int c = 0; c < 9; ++c)
+            hb[c][j] = a.first ? 0.0 : st[(c * 3 + j) * U];
+        sb[j] = a.first ? 0.0 : st[(27 + j) * U];
+        Sb[j] = a.first ? 0.0 : st[(30 + j) * U];
+    }
+    auto at = [&](int step) {
+        const int i = step - a.step_lo;
+        return a.offset ? a.offset[i] + u : (int64_t)i * U + u;
+    };
+    const int top = min(kend, a.step_hi);
+    double Jn[3][3];
+    if (top >= a.step_lo)
+        load_jac(a.jac, a.total, at(top), Jn);
+    for (int step = top; step >= a.step_lo; --step) {
+        double J[3][3];
+#pragma unroll
+        for (int k = 0; k < 9; ++k)
+            J[k / 3][k % 3] = Jn[k / 3][k % 3];
+        if (step > a.step_lo) // the next Jacobian loads during this step
+            load_jac(a.jac, a.total, at(step - 1), Jn);
+        const int node = step - k0;
+        const double* seed = (node >= 0 && node < 3) ? seeds + node * 9 : nullptr;
+        double abar[3], s1b[3], s2b[3], Spb[3], prevb[3], a7b[3];
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+            abar[j] = hb[8][j] + (seed ? seed[6 + j] : 0.0);
+#pragma unroll
+        for (int c = 8; c >= 1; --c)
+#pragma unroll
+            for (int j = 0; j < 3; ++j)
+                hb[c][j] = hb[c - 1][j];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            hb[0][j] = 0.0;
+            const double rb = seed ? seed[j] : 0.0, vb = seed ? seed[3 + j] : 0.0;
+            const double sK = sb[j] + h * vb; // s_n feeds v_n = h (s1 + SA88 a + s_n)
+            s1b[j] = h * vb;
+            abar[j] += h * c_SA[8][8] * vb + sK / 2;
+            prevb[j] = sK;
+            a7b[j] = sK / 2;
+            s2b[j] = h2 * rb;
+            abar[j] += h2 * c_GJ[8][8] * rb;
+            Spb[j] = Sb[j] + h2 * rb;
+        }
+        for (int it = a.ncorr - 1; it >= 0; --it) {
+            double rb[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                rb[k] = J[0][k] * abar[0] + J[1][k] * abar[1] + J[2][k] * abar[2];
+            if (it >= 1) {
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    s2b[j] += h2 * rb[j];
+                    Spb[j] += h2 * rb[j];
+                    abar[j] = h2 * c_GJ[8][8] * rb[j];
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+#pragma unroll
+                    for (int c = 0; c < 9; ++c)
+                        hb[c][j] += h2 * c_GJ[9][c] * rb[j];
+                    Spb[j] += h2 * rb[j];
                 }
             }
-            for (int step = lo; step <= hi; ++step) {
-                const double* M = a.prop_m + (size_t)(step + 4) * 9;
-                double* it_base = a.scratch + (size_t)(step - lo) * 3 * U + u;
-                auto eval = [&](const double* rr, double* aa) {
-                    if (l == 0)
+        }
 #pragma unroll
-                        for (int j = 0; j < 3; ++j)
-                            it_base[(int64_t)j * U] = rr[j];
-                    gravity_gcrs_lanes<false>(g, l, P, M, rr, aa, mask);
-                };
-                gj8_step<double>(eval, a.h, K, hist, s, S, r, v);
-            }
-            __syncwarp(mask);
-            for (int step = hi; step >= lo; --step) {
-                const double* M = a.prop_m + (size_t)(step + 4) * 9;
-                const double* it_base = a.scratch + (size_t)(step - lo) * 3 * U + u;
-                const int node = step - k0;
-                const double* seed = (node >= 0 && node < 3) ? seeds + node * 9 : nullptr;
-                gj8_reverse_step(g, l, P, mask, M, a.h, K, it_base, U, seed, hb, sb, Sb);
-            }
-            __syncwarp(mask); // the next segment overwrites the iterates
+        for (int j = 0; j < 3; ++j) {
+#pragma unroll
+            for (int c = 0; c < 8; ++c)
+                hb[c + 1][j] += c_SA[8][c] * s1b[j] + c_GJ[8][c] * s2b[j];
+            hb[8][j] += a7b[j] + Spb[j] / 2; // a7 = h8, and S' = S + s + h8/2
+            Sb[j] = Spb[j];
+            sb[j] = prevb[j] + Spb[j];
         }
     }
-    // startup: forward tangents of its outputs along direction l, dotted with their adjoints
-    const int dir = l < 6 ? l : -1;
-    LaneForceTan ft { g, l, P, mask, a.gen_m, a.prop_m };
-    Tan r0[3], v0[3];
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
-        r0[j] = Tan(a.r0[o * 3 + j], dir == j ? 1.0 : 0.0);
-        v0[j] = Tan(a.v0[o * 3 + j], dir == 3 + j ? 1.0 : 0.0);
-    }
-    StartupMatsT<Tan> m;
-    run_startup(ft, a.h, K, r0, v0, m);
-    double gsum = 0.0; // history, s and S adjoints are those of the step-5 inputs (zero if none)
 #pragma unroll
+        for (int c = 0; c < 9; ++c)
+            st[(c * 3 + j) * U] = hb[c][j];
+        st[(27 + j) * U] = sb[j];
+        st[(30 + j) * U] = Sb[j];
+    }
+}
+
+// Gradient of the units whose object lies in [obj_lo, obj_lo + n): the startup's outputs along each
+// initial-state direction, contracted with their adjoints. Thread t = rank 6 + dir.
+__global__ void __launch_bounds__(128) adjoint_finish_kernel(AdjFinishArgs a)
+{
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= 6 * a.n_units)
+        return;
+    const int64_t u = t / 6, U = a.n_units, unit = a.unit ? a.unit[u] : u;
+    const int dir = (int)(t % 6);
+    const int64_t o = a.unit_obj[unit] - a.obj_lo;
+    if (o < 0 || o >= a.n)
+        return;
+    const double* T = a.startup + (int64_t)dir * a.n + o;
+    const int64_t W = 6 * a.n;
+    const double* st = a.sweep + u;
+    double g = 0.0; // history, s and S adjoints are those of the step-5 inputs (zero if none)
     for (int j = 0; j < 3; ++j) {
         for (int c = 0; c < 9; ++c)
-            gsum += hb[c][j] * m.a[c][j].d;
-        gsum += sb[j] * m.s[8][j].d + Sb[j] * m.S[8][j].d;
+            g += st[(c * 3 + j) * U] * T[(int64_t)(c * 3 + j) * W];
+        g += st[(27 + j) * U] * T[(int64_t)(27 + j) * W] + st[(30 + j) * U] * T[(int64_t)(30 + j) * W];
     }
     const bool fix_q3 = (a.flags & 2u) != 0;
+    const int k0 = a.seed_step0[unit];
     for (int node = 0; node < 3; ++node) { // seeds on the replayed steps 1..4
         const int step = k0 + node;
-        if (step < 1 || step > 4 || step > N)
+        if (step < 1 || step > 4 || step > a.steps)
             continue;
-        const double* sd = seeds + node * 9;
+        const double* sd = a.seeds + unit * 27 + node * 9;
         for (int j = 0; j < 3; ++j) {
-            gsum += sd[j] * m.r[4 + step][j].d + sd[3 + j] * m.v[4 + step][j].d;
-            gsum += sd[6 + j] * (fix_q3 ? m.a[4 + step][j].d : m.a[8][j].d);
+            g += sd[j] * T[(int64_t)(33 + (step - 1) * 3 + j) * W]
+                + sd[3 + j] * T[(int64_t)(45 + (step - 1) * 3 + j) * W];
+            g += sd[6 + j] * T[(int64_t)((fix_q3 ? 4 + step : 8) * 3 + j) * W];
         }
     }
-    if (dir >= 0)
-        a.grad[u * 6 + dir] = gsum;
+    a.grad[unit * 6 + dir] = g;
 }
 
 // ---- closest approach of listed pairs, with the seeds of d(miss) ----
@@ -487,34 +558,53 @@ __global__ void __launch_bounds__(128) pair_approach_kernel(PairArgs a)
 }
 
 // ---- launchers ----
-static size_t var_smem(const TableSrc& ts) { return 128 + (size_t)ts.bytes; }
-
-cudaError_t launch_stm(const TableSrc& ts, const VarArgs& a, cudaStream_t s)
+cudaError_t launch_jac_points(const TableSrc& plain64, const JacPoints& a, int num_sms, cudaStream_t s)
 {
-    if (a.n <= 0)
+    if (a.total <= 0)
         return cudaSuccess;
-    const size_t smem = var_smem(ts);
-    cudaError_t e = cudaFuncSetAttribute(stm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const size_t smem = 128 + (size_t)plain64.bytes;
+    const cudaError_t e
+        = cudaFuncSetAttribute(jac_points_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess)
         return e;
-    const int block = 256;
-    const int64_t blocks = (a.n * kVarLanes + block - 1) / block;
-    stm_kernel<<<(unsigned)blocks, block, smem, s>>>(ts, a);
+    // few points spread over the SMs in blocks of a warp or more, many take a block of 8 warps per SM
+    const int64_t per_sm = (a.total + num_sms - 1) / num_sms;
+    const int block = (int)std::min<int64_t>(256, std::max<int64_t>(32, (per_sm + 31) / 32 * 32));
+    const unsigned grid = (unsigned)std::min<int64_t>(num_sms, (a.total + block - 1) / block);
+    jac_points_kernel<<<grid, block, smem, s>>>(plain64, a);
     return cudaGetLastError();
 }
 
-cudaError_t launch_adjoint(const TableSrc& ts, const AdjArgs& a, cudaStream_t s)
+cudaError_t launch_startup_tangents(const StartupTangentArgs& a, cudaStream_t s)
+{
+    if (a.n <= 0)
+        return cudaSuccess;
+    rk8_tangent_kernel<<<(unsigned)((12 * a.n + 127) / 128), 128, 0, s>>>(a);
+    corrector_tangent_kernel<<<(unsigned)((6 * a.n + 127) / 128), 128, 0, s>>>(a);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_stm_sweep(const StmArgs& a, cudaStream_t s)
+{
+    if (a.n <= 0)
+        return cudaSuccess;
+    stm_sweep_kernel<<<(unsigned)((6 * a.n + 127) / 128), 128, 0, s>>>(a);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_adjoint_sweep(const AdjSweepArgs& a, cudaStream_t s)
 {
     if (a.n_units <= 0)
         return cudaSuccess;
-    const size_t smem = var_smem(ts);
-    cudaError_t e
-        = cudaFuncSetAttribute(adjoint_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess)
-        return e;
-    const int block = 256;
-    const int64_t blocks = (a.n_units * kVarLanes + block - 1) / block;
-    adjoint_kernel<<<(unsigned)blocks, block, smem, s>>>(ts, a);
+    adjoint_sweep_kernel<<<(unsigned)((a.n_units + 63) / 64), 64, 0, s>>>(a);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_adjoint_finish(const AdjFinishArgs& a, cudaStream_t s)
+{
+    if (a.n_units <= 0)
+        return cudaSuccess;
+    adjoint_finish_kernel<<<(unsigned)((6 * a.n_units + 127) / 128), 128, 0, s>>>(a);
     return cudaGetLastError();
 }
 
@@ -526,48 +616,67 @@ cudaError_t launch_pair_approach(const PairArgs& a, cudaStream_t s)
     return cudaGetLastError();
 }
 
-// ---- acceleration Jacobian of many positions (one group of kVarLanes lanes each) ----
-__global__ void __launch_bounds__(256, 1) jacobian_kernel(TableSrc ts, int64_t n, const double* r,
+// ---- acceleration Jacobian of many positions (gpop_gravity_jacobian) ----
+// LANE: P lanes per point on the lane-layout table (few points), else a point per thread on the plain one.
+template <bool LANE>
+__global__ void __launch_bounds__(256, 1) jacobian_kernel(TableSrc ts, int64_t n, int P, const double* r,
     const double* M, double* acc, double* jac, unsigned* err)
 {
     extern __shared__ __align__(128) uint8_t smem[];
     GravSmem g;
-    if (!stage_table64(smem, ts, err, g))
-        return;
-    const int P = kVarLanes;
-    const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / P;
-    const int l = (int)(threadIdx.x % P);
-    if (i >= n)
-        return;
-    const unsigned mask = 0xffu << (threadIdx.x & 24);
-    const double ri[3] = { r[i * 3], r[i * 3 + 1], r[i * 3 + 2] };
-    double a[3], J[3][3];
-    if (M)
-        gravity_jac_gcrs_lanes(g, l, P, M, ri, a, J, mask);
-    else
-        gravity_jac_itrs_lanes(g, l, P, ri[0], ri[1], ri[2], a, J, mask);
-    if (l == 0)
-        for (int k = 0; k < 3; ++k) {
-            if (acc)
-                acc[i * 3 + k] = a[k];
-            for (int m = 0; m < 3; ++m)
-                jac[(i * 3 + k) * 3 + m] = J[k][m];
-        }
+    if constexpr (LANE) {
+        if (!bind_lane_table(smem, ts, err, g))
+            return;
+    } else {
+        if (!bind_plain64(smem, ts, err, g))
+            return;
+    }
+    const int lane = (int)threadIdx.x & 31, l = LANE ? (int)threadIdx.x % P : 0;
+    const unsigned mask = !LANE ? 0u : P == 32 ? 0xffffffffu : ((1u << P) - 1u) << (lane & ~(P - 1));
+    const int64_t T = ((int64_t)gridDim.x * blockDim.x) / P;
+    for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / P; i < n; i += T) {
+        const double ri[3] = { r[i * 3], r[i * 3 + 1], r[i * 3 + 2] };
+        double a[3], J[3][3];
+        if (M)
+            gravity_jac_gcrs<LANE>(g, l, P, M, ri, a, J, mask);
+        else
+            gravity_jac_itrs<LANE>(g, l, P, ri[0], ri[1], ri[2], a, J, mask);
+        if (l == 0)
+            for (int k = 0; k < 3; ++k) {
+                if (acc)
+                    acc[i * 3 + k] = a[k];
+                for (int m = 0; m < 3; ++m)
+                    jac[(i * 3 + k) * 3 + m] = J[k][m];
+            }
+    }
 }
 
-cudaError_t launch_jacobian(const TableSrc& ts, int64_t n, const double* r, const double* M,
-    double* acc, double* jac, unsigned* err, cudaStream_t s)
+// Lanes per point: the most (<= 32) that keep all points in one block of 8 warps per SM; one thread per
+// point once every scheduler has a warp of them (n >= 128 per SM).
+cudaError_t launch_jacobian(const TableSrc& plain64, const TableSrc& lane64, int64_t n, const double* r,
+    const double* M, double* acc, double* jac, unsigned* err, int num_sms, cudaStream_t s)
 {
     if (n <= 0)
         return cudaSuccess;
-    const size_t smem = var_smem(ts);
-    cudaError_t e
-        = cudaFuncSetAttribute(jacobian_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess)
-        return e;
-    const int block = 256;
-    jacobian_kernel<<<(unsigned)((n * kVarLanes + block - 1) / block), block, smem, s>>>(ts, n, r, M, acc,
-        jac, err);
+    int P = 1;
+    if (n < (int64_t)num_sms * 128)
+        for (P = 2; P < 32 && n * 2 * P <= (int64_t)num_sms * 256;)
+            P *= 2;
+    const TableSrc& ts = P > 1 ? lane64 : plain64;
+    const size_t smem = 128 + (size_t)ts.bytes;
+    const int64_t threads = n * P, per_sm = (threads + num_sms - 1) / num_sms;
+    const int block = (int)std::min<int64_t>(256, std::max<int64_t>(32, (per_sm + 31) / 32 * 32));
+    const unsigned grid = (unsigned)std::min<int64_t>(num_sms, (threads + block - 1) / block);
+    cudaError_t e;
+    if (P > 1) {
+        if ((e = cudaFuncSetAttribute(jacobian_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
+            return e;
+        jacobian_kernel<true><<<grid, block, smem, s>>>(ts, n, P, r, M, acc, jac, err);
+    } else {
+        if ((e = cudaFuncSetAttribute(jacobian_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
+            return e;
+        jacobian_kernel<false><<<grid, block, smem, s>>>(ts, n, P, r, M, acc, jac, err);
+    }
     return cudaGetLastError();
 }
 
