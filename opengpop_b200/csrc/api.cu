@@ -163,6 +163,7 @@ gpop_status propagator_step(gpop_propagator* p, int steps, double* traj_r, doubl
         return cuda_fail(ctx, e, "cudaSetDevice");
     const TableSrc ts = ctx->table(p->mixed);
     const TableSrc lane_ts = ctx->lane_table(p->mixed);
+    const TableSrc lane64 = ctx->lane_table(false);
     PropArgs a;
     a.n = p->n;
     a.h = p->h;
@@ -178,7 +179,7 @@ gpop_status propagator_step(gpop_propagator* p, int steps, double* traj_r, doubl
     a.stage_pos = p->stage_pos;
     a.col_pos = p->col_pos;
     if (!p->started) {
-        if ((e = launch_startup(ts, a, ctx->num_sms, s, &lane_ts)) != cudaSuccess)
+        if ((e = launch_startup(ts, a, ctx->num_sms, s, &lane_ts, &lane64)) != cudaSuccess)
             return cuda_fail(ctx, e, "startup kernel");
         ctx->launches += p->kind == GPOP_FORCE_GRAVITY ? startup_launches(p->ncorr) : 1;
         p->started = true;
@@ -195,7 +196,8 @@ gpop_status propagator_step(gpop_propagator* p, int steps, double* traj_r, doubl
         const bool last = a.step_end == end;
         a.out_r = last ? p->r : nullptr;
         a.out_v = last ? p->v : nullptr;
-        if ((e = launch_gj8(ts, a, ctx->num_sms, s, ctx->block_override, ctx->walk_mode, &lane_ts))
+        if ((e = launch_gj8(ts, a, ctx->num_sms, s, ctx->block_override, ctx->walk_mode, &lane_ts,
+                 &lane64))
             != cudaSuccess)
             return cuda_fail(ctx, e, "GJ8 kernel");
         ctx->launches++;
@@ -270,6 +272,8 @@ gpop_status gpop_create(const gpop_config* cfg_in, gpop_ctx** out)
     if (!load_model(ctx->data_dir, cfg.gravity_degree, ctx->md, err))
         return fail(ctx, GPOP_ERR_DATA, err);
     ctx->corr = corrector_model(ctx->md);
+    ctx->plan64 = column_plan(ctx->md.degree, false);
+    ctx->plan_mixed = column_plan(ctx->md.degree, true);
     if (const char* spl = std::getenv("GPOP_STEPS_PER_LAUNCH"))
         ctx->steps_per_launch = std::max(1, atoi(spl));
     if (const char* wm = std::getenv("GPOP_WALK_MODE"))

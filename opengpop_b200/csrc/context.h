@@ -76,6 +76,7 @@ struct gpop_ctx {
     std::string err;
     gpop::ModelData md;
     gpop::CorrModel corr;
+    gpop::ColumnPlan plan64, plan_mixed;
     int num_sms = 148;
     int steps_per_launch = 64;
     int block_override = 0; // GJ8 block size chosen by the tuner (0 = default policy)
@@ -118,6 +119,7 @@ struct gpop_ctx {
         ts.gm = md.gm;
         ts.mixed = mixed_mode;
         ts.lanes = true;
+        ts.plan = mixed_mode ? plan_mixed : plan64;
         ts.src = mixed_mode ? lane_mixed.p : lane64.p;
         ts.bytes = mixed_mode ? lane_mixed_bytes : lane64_bytes;
         ts.off32 = mixed_mode ? lane_mixed_off32 : lane64_off32;

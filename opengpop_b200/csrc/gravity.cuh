@@ -49,7 +49,7 @@ constexpr int kMixedSplit = 8; // highest degree kept in FP64 in the mixed mode
 #define GPOP_PAIR_COLUMNS64 1
 #endif
 #ifndef GPOP_COL64PAIR_UNROLL
-#define GPOP_COL64PAIR_UNROLL 2
+#define GPOP_COL64PAIR_UNROLL 4
 #endif
 constexpr int kCol32x2Unroll = GPOP_COL32X2_UNROLL;
 constexpr int kCol64Unroll = GPOP_COL64_UNROLL;
@@ -646,25 +646,28 @@ __device__ __forceinline__ void assemble_itrs(double gm, double x, double y, dou
     az = c * (Lambda * eps - H);
 }
 
-// The mixed two-object walk from column m0 (a multiple of kHeadGroup, <= 8; the recursions
-// already stepped to it) to L: head groups, then the FP32 tail, whose totals are added into the
-// FP64 ones.
+// The mixed two-object walk over columns m0 .. L (the recursions already stepped to m0): head groups, then
+// the FP32 tail, whose totals are added into the FP64 ones. m0 and L + 1 each lie past the head (m > 8) or
+// on a head group's first column (a multiple of kHeadGroup).
 template <bool LANE, int PU>
-__device__ __forceinline__ void walk_groups_from(MixedWalk2<LANE, PU>& W, int m0)
+__device__ __forceinline__ void walk_groups(MixedWalk2<LANE, PU>& W, int m0, int L)
 {
     constexpr int K = 2;
-    const int L = W.L;
     int m = m0;
 #pragma unroll 1
-    for (; m + kHeadGroup - 1 <= kMixedSplit; m += kHeadGroup)
+    for (; m + kHeadGroup - 1 <= kMixedSplit && m <= L; m += kHeadGroup)
         W.template head_group<kHeadGroup>(m);
     if constexpr (kHeadGroup > 1) { // 9 head columns: what the groups left
         constexpr int rest = (kMixedSplit + 1) % kHeadGroup;
         if constexpr (rest > 0)
-            W.template head_group<rest>(m);
+            if (m <= kMixedSplit && m <= L) {
+                W.template head_group<rest>(m);
+                m += rest;
+            }
     }
+    if (m > L)
+        return;
     W.to_tail();
-    m = kMixedSplit + 1;
 #pragma unroll 1
     for (; m + kTailGroup - 1 <= L; m += kTailGroup)
         W.template tail_group<kTailGroup>(m);
@@ -697,7 +700,7 @@ __device__ __forceinline__ void gravity_itrs_groups(const GravSmem& gs, const do
     for (int k = 0; k < K; ++k)
         ri[k] = inv_norm(x[k], y[k], z[k]);
     MixedWalk2<LANE> W(gs, ri, x, y, z);
-    walk_groups_from(W, 0);
+    walk_groups(W, 0, W.L);
 #pragma unroll
     for (int k = 0; k < K; ++k)
         assemble_itrs(gs.gm, x[k], y[k], z[k], ri[k], W.G[k], W.H[k], W.J[k], W.KK[k], ax[k], ay[k],
@@ -885,7 +888,7 @@ __device__ __forceinline__ void split_high(const GravSmem& gs, const WalkStart& 
 #pragma unroll
         for (int m = 0; m < kSplitColumn; ++m)
             W.skip64();
-        walk_groups_from(W, kSplitColumn);
+        walk_groups(W, kSplitColumn, W.L);
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
             t.G[k] = W.G[k];

@@ -19,6 +19,7 @@ struct TableSrc {
     // lowers it to make the wait give up on purpose)
     uint32_t wait_spins = 1u << 22;
     CorrModel corr;
+    ColumnPlan plan; // (lane layout)
 };
 
 // Byte offset, in a kernel's dynamic shared memory, of what follows a staged table (the 128-byte
@@ -81,7 +82,7 @@ inline int startup_launches(int ncorr) { return 3 + 2 * ncorr; }
 // Startup of a.n objects. Gravity with the state and the lane-layout table at hand runs the pipeline of
 // startup.cu; analytic forces, compensated sums and the unit entry point one thread per object.
 cudaError_t launch_startup(const TableSrc& ts, const PropArgs& a, int num_sms, cudaStream_t s,
-    const TableSrc* lane_ts = nullptr);
+    const TableSrc* lane_ts = nullptr, const TableSrc* lane64 = nullptr);
 // How many objects a GJ8 thread carries through the gravity triangle walk (0 = by problem size).
 // kWalkLanes: P lanes per object split the gravity columns (few objects; P from lanes_per_object).
 // kWalkLanesTwo: P lanes per group of two objects (P from lane_pair_lanes, else 2), the default
@@ -101,9 +102,12 @@ int lane_pair_lanes(int64_t n, int num_sms, bool fp64_gravity);
 int default_walk(int64_t n, int num_sms, bool lanes, bool fp64_gravity);
 // Owner warps of the split block two objects per thread take for n objects (0: a plain block).
 int split_owner_warps(int64_t n, int num_sms, int L);
-// lane_ts: the lane-layout table of the same precision (NULL: no lane-split walk).
+// lane_ts: the lane-layout table of the same precision (NULL: no lane-split walk), lane64: the FP64 one.
 cudaError_t launch_gj8(const TableSrc& ts, const PropArgs& a, int num_sms, cudaStream_t s,
-    int block_override = 0, int walk = 0, const TableSrc* lane_ts = nullptr);
+    int block_override = 0, int walk = 0, const TableSrc* lane_ts = nullptr, const TableSrc* lane64 = nullptr);
+// The same steps with the columns split over the warps of one block per SM (columns.cu): at most 512
+// objects per SM, degree >= 2.
+cudaError_t launch_gj8_columns(const TableSrc& lane_ts, const PropArgs& a, int num_sms, cudaStream_t s);
 cudaError_t launch_gravity(const TableSrc& ts, int64_t n, const double* r, const double* m9,
     double* a, unsigned* err, int num_sms, cudaStream_t s);
 cudaError_t launch_corrector_unit(int kind, double h, int op, double* r27, double* v27, double* a27,

@@ -82,43 +82,48 @@ __device__ __forceinline__ void cpow(double c1, double s1, int p, double& rc, do
     rs = xs;
 }
 
-// What a lane's columns l, l + T, ... start from and step by: z = C1 + i S1 and q to the powers l,
-// l - 1 (the m - 1 values; none for column 0), T and T - 1 (the m - 1 values of column T). T is a
-// power of two, or beyond the last column (then nothing steps and only the first three are made). The
-// powers come from the squares z^2, z^4, ... that every lane forms: two dependent operations per bit,
-// where a scan over the lanes adds a shuffle to each.
+// What a lane's columns m, m + P, ... start from and step by: z = C1 + i S1 and q to the powers m, m - 1 (none
+// for column 0), P and P - 1 (the m - 1 values of column P, for the lane that starts at column 0). P is a
+// power of two, or beyond the last column (one round: only the first three are made). top: the largest m - 1
+// of the group. The powers come from the squares z^2, z^4, ... that every lane forms (two dependent
+// operations per bit, where a scan over the lanes adds a shuffle to each).
 struct LanePowers {
     double Cm, Sm, Cp, Sp, qm, CP, SP, CPm1, SPm1, qP;
 };
-__device__ __forceinline__ LanePowers lane_powers(double C1, double S1, double q, int l, int T, bool steps)
+__device__ __forceinline__ LanePowers lane_powers(double C1, double S1, double q, int m, int top, int P, bool steps)
 {
     LanePowers w;
-    const int e = l > 0 ? l - 1 : 0;
+    const int e = m > 0 ? m - 1 : 0;
     double bc = C1, bs = S1, bq = q, xc = 1.0, xs = 0.0, xq = 1.0;
     w.CPm1 = 1.0;
     w.SPm1 = 0.0;
-    for (int o = 1; o < T; o <<= 1) {
+    w.CP = C1;
+    w.SP = S1;
+    w.qP = q;
+    for (int o = 1; o <= top || (steps && o < P); o <<= 1) {
         double tc, ts;
         cmul(xc, xs, bc, bs, tc, ts);
         const bool on = (e & o) != 0;
         xc = on ? tc : xc;
         xs = on ? ts : xs;
         xq = on ? xq * bq : xq;
-        if (steps)
+        if (steps && o < P)
             cmul(w.CPm1, w.SPm1, bc, bs, w.CPm1, w.SPm1);
         cmul(bc, bs, bc, bs, bc, bs);
         bq *= bq;
+        if (2 * o == P) {
+            w.CP = bc;
+            w.SP = bs;
+            w.qP = bq;
+        }
     }
-    w.CP = bc;
-    w.SP = bs;
-    w.qP = bq;
     cmul(xc, xs, C1, S1, w.Cm, w.Sm);
     w.qm = xq * q;
-    w.Cp = l > 0 ? xc : 0.0;
-    w.Sp = l > 0 ? xs : 0.0;
-    w.Cm = l > 0 ? w.Cm : 1.0;
-    w.Sm = l > 0 ? w.Sm : 0.0;
-    w.qm = l > 0 ? w.qm : 1.0;
+    w.Cp = m > 0 ? xc : 0.0;
+    w.Sp = m > 0 ? xs : 0.0;
+    w.Cm = m > 0 ? w.Cm : 1.0;
+    w.Sm = m > 0 ? w.Sm : 0.0;
+    w.qm = m > 0 ? w.qm : 1.0;
     return w;
 }
 
@@ -192,51 +197,60 @@ struct BlockTeam {
     }
 };
 
-// Gravity in the Earth-fixed frame of K objects with the columns split over the P lanes of each
-// object's group (lane l takes columns l, l + P, ...; P a power of two, or more than the columns); the
-// per-object totals are added across the group. As gravity_itrs in mixed mode: the head columns
-// m <= 8 are combined in FP64 (their terms of degree > 8 summed in FP32 per column), the columns m > 8
-// are walked, combined and summed in FP32 and added to the FP64 totals once. PAIRS: FP64 lanes walk two
-// of their columns side by side (the one-object GJ8 lane kernel; kernels with fewer registers to spare
-// keep one at a time).
-template <bool MIXED, int K, bool PAIRS = false, class Team = WarpTeam>
-__device__ __forceinline__ void gravity_itrs_team(const GravSmem& gs, const Team& team, const double (&x)[K],
-    const double (&y)[K], const double (&z)[K], double (&ax)[K], double (&ay)[K], double (&az)[K])
+// Lanes per group as gravity_itrs_team takes them: P <= 32 lanes of a warp, or whole warps.
+template <bool WARPS> struct TeamOf;
+template <> struct TeamOf<false> {
+    using type = WarpTeam;
+};
+template <> struct TeamOf<true> {
+    using type = BlockTeam;
+};
+template <bool WARPS>
+__device__ __forceinline__ typename TeamOf<WARPS>::type make_team(int P, double* buf)
 {
-    const int l = team.l, P = team.P;
-    const int L = gs.L;
-    double ri[K], q[K], u[K], w[K], C1[K], S1[K], CP[K], SP[K], Cm[K], Sm[K], Cp[K], Sp[K], CPm1[K], SPm1[K];
-    double qm[K], qP[K], G[K], H[K], J[K], KK[K];
+    const int l = (int)threadIdx.x % P;
+    if constexpr (WARPS) {
+        return BlockTeam { l, P, P / 32, 1 + (int)threadIdx.x / P, buf, 0 };
+    } else {
+        const int lane = (int)threadIdx.x & 31;
+        return WarpTeam { l, P, P == 32 ? 0xffffffffu : ((1u << P) - 1u) << (lane & ~(P - 1)) };
+    }
+}
+
+// Doubles of shared memory per group of gj8_team_kernel: the history, then the sums of a group of warps.
+inline __host__ __device__ int team_doubles(int P, bool warps) { return 28 + (warps ? P / 4 : 0); }
+
+// Columns first, first + P, ... up to `last` of K objects, added into G, H, J, KK. As gravity_itrs in mixed
+// mode: the head columns m <= 8 are combined in FP64 (their terms of degree > 8 summed in FP32 per column),
+// the columns m > 8 are walked, combined and summed in FP32 and added to the FP64 totals once. PAIRS: FP64
+// lanes walk two of their columns side by side (kernels with few registers to spare keep one at a time).
+template <bool MIXED, int K, bool PAIRS>
+__device__ __forceinline__ void lane_walk(const GravSmem& gs, int first, int P, int last, const LanePowers (&lp)[K],
+    const double (&u)[K], const double (&w)[K], double (&G)[K], double (&H)[K], double (&J)[K], double (&KK)[K])
+{
+    const int L = gs.L, top = MIXED && L > kMixedSplit ? kMixedSplit : L; // last degree of the FP64 terms
+    double CP[K], SP[K], Cm[K], Sm[K], Cp[K], Sp[K], CPm1[K], SPm1[K], qm[K], qP[K];
     float uf[K], wf[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-        ri[k] = inv_norm(x[k], y[k], z[k]);
-        const double eps = z[k] * ri[k];
-        q[k] = gs.radius * ri[k];
-        u[k] = q[k] * eps;
-        w[k] = q[k] * q[k];
         uf[k] = (float)u[k];
         wf[k] = (float)w[k];
-        C1[k] = x[k] * ri[k];
-        S1[k] = y[k] * ri[k];
-        G[k] = H[k] = J[k] = KK[k] = 0.0;
-        const LanePowers lp = lane_powers(C1[k], S1[k], q[k], l, P, P <= L);
-        Cm[k] = lp.Cm;
-        Sm[k] = lp.Sm;
-        Cp[k] = lp.Cp;
-        Sp[k] = lp.Sp;
-        qm[k] = lp.qm;
-        CP[k] = lp.CP;
-        SP[k] = lp.SP;
-        CPm1[k] = lp.CPm1;
-        SPm1[k] = lp.SPm1;
-        qP[k] = lp.qP;
+        Cm[k] = lp[k].Cm;
+        Sm[k] = lp[k].Sm;
+        Cp[k] = lp[k].Cp;
+        Sp[k] = lp[k].Sp;
+        qm[k] = lp[k].qm;
+        CP[k] = lp[k].CP;
+        SP[k] = lp[k].SP;
+        CPm1[k] = lp[k].CPm1;
+        SPm1[k] = lp[k].SPm1;
+        qP[k] = lp[k].qP;
     }
-    const int Lhead = (MIXED && L > kMixedSplit) ? kMixedSplit : L;
+    const int Lhead = min(last, MIXED && L > kMixedSplit ? kMixedSplit : L);
     // column bases of the lane's next column are read one column ahead (they are shared-memory
     // loads the walk's first table read depends on)
-    int b64 = gs.cb64[l < 127 ? l : 127], b32 = gs.cb32[l < 127 ? l : 127];
-    int m = l;
+    int b64 = gs.cb64[min(first, 127)], b32 = gs.cb32[min(first, 127)];
+    int m = first;
     if constexpr (!MIXED && PAIRS && kLanePairColumns) {
         // FP64: two of this lane's columns (m and m + P) side by side, so each object carries two
         // independent recursions; each column's sums, and their combination, in the order of the
@@ -260,8 +274,8 @@ __device__ __forceinline__ void gravity_itrs_team(const GravSmem& gs, const Team
             const GravEntry64* eb = reinterpret_cast<const GravEntry64*>(reinterpret_cast<const uint4*>(gs.t64) + bb64);
             sa.add(ea, Qa1);
             sb.add(eb, Qb1);
-            column64_pair<K>(ea + 1, eb + 1, Lhead - mb, u, w, Qa1, Qa2, sa, Qb1, Qb2, sb);
-            column64<K>(ea, Lhead - mb + 1, Lhead - m, u, w, Qa1, Qa2, sa);
+            column64_pair<K>(ea + 1, eb + 1, top - mb, u, w, Qa1, Qa2, sa, Qb1, Qb2, sb);
+            column64<K>(ea, top - mb + 1, top - m, u, w, Qa1, Qa2, sa);
             lane_combine<K>(m, sa, CP, SP, CPm1, SPm1, qP, Cm, Sm, Cp, Sp, qm, G, H, J, KK);
             lane_combine<K>(mb, sb, CP, SP, CPm1, SPm1, qP, Cm, Sm, Cp, Sp, qm, G, H, J, KK);
             b64 = nb64;
@@ -280,7 +294,7 @@ __device__ __forceinline__ void gravity_itrs_team(const GravSmem& gs, const Team
         }
         const GravEntry64* e = reinterpret_cast<const GravEntry64*>(reinterpret_cast<const uint4*>(gs.t64) + b64);
         s.add(e, Q1);
-        column64<K>(e, 1, Lhead - m, u, w, Q1, Q2, s);
+        column64<K>(e, 1, top - m, u, w, Q1, Q2, s);
         if constexpr (MIXED) {
             if (L > kMixedSplit) {
                 ColSums32<K> f;
@@ -324,7 +338,7 @@ __device__ __forceinline__ void gravity_itrs_team(const GravSmem& gs, const Team
         b32 = nb32;
     }
     if constexpr (MIXED) {
-        if (m <= L) { // this lane's columns m > 8, in FP32
+        if (m <= last) { // this lane's columns m > 8, in FP32
             float cf[K], sf[K], cpf[K], spf[K], CPf[K], SPf[K], qmf[K], qPf[K];
             float Gf[K], Hf[K], Jf[K], Kf[K];
 #pragma unroll
@@ -339,7 +353,7 @@ __device__ __forceinline__ void gravity_itrs_team(const GravSmem& gs, const Team
                 qPf[k] = (float)qP[k];
                 Gf[k] = Hf[k] = Jf[k] = Kf[k] = 0.f;
             }
-            for (; m <= L; m += P) {
+            for (; m <= last; m += P) {
                 const int nb = gs.cb32[m + P < 127 ? m + P : 127];
                 ColSums32<K> f;
                 const GravEntry32* e32 = reinterpret_cast<const GravEntry32*>(reinterpret_cast<const uint4*>(gs.t32) + b32);
@@ -382,6 +396,27 @@ __device__ __forceinline__ void gravity_itrs_team(const GravSmem& gs, const Team
             }
         }
     }
+}
+
+// Gravity in the Earth-fixed frame of K objects with the columns split over the P lanes of each object's
+// group (lane l takes columns l, l + P, ...; P a power of two, or more than the columns); the per-object
+// totals are added across the group.
+template <bool MIXED, int K, bool PAIRS = false, class Team = WarpTeam>
+__device__ __forceinline__ void gravity_itrs_team(const GravSmem& gs, const Team& team, const double (&x)[K],
+    const double (&y)[K], const double (&z)[K], double (&ax)[K], double (&ay)[K], double (&az)[K])
+{
+    double ri[K], u[K], w[K], G[K], H[K], J[K], KK[K];
+    LanePowers lp[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        ri[k] = inv_norm(x[k], y[k], z[k]);
+        const double q = gs.radius * ri[k];
+        u[k] = q * (z[k] * ri[k]);
+        w[k] = q * q;
+        G[k] = H[k] = J[k] = KK[k] = 0.0;
+        lp[k] = lane_powers(x[k] * ri[k], y[k] * ri[k], q, team.l, team.P - 2, team.P, team.P <= gs.L);
+    }
+    lane_walk<MIXED, K, PAIRS>(gs, team.l, team.P, gs.L, lp, u, w, G, H, J, KK);
 #pragma unroll
     for (int k = 0; k < K; ++k) {
         team.sum4(G[k], H[k], J[k], KK[k]);

@@ -221,6 +221,50 @@ CorrModel corrector_model(const ModelData& md)
     return c;
 }
 
+// Ranges of about equal work: terms (twice for the FP64 ones in mixed precision, a round of P columns costs
+// its longest) and 6 terms' worth of combination per column.
+ColumnPlan column_plan(int L, bool mixed)
+{
+    const int split = 8; // last degree of the FP64 terms
+    ColumnPlan plan {};
+    for (int k = 0; k < 5; ++k) {
+        const int P = 1 << k;
+        auto column = [&](int m) { // cost of the round that starts with column m
+            return L - m + 1 + 6.0 + (mixed && m <= split ? std::min(L, split) - m + 5.0 : 0.0);
+        };
+        // two objects per lane in mixed precision walk the head columns in pairs from even ones
+        auto allowed = [&](int m) { return !(k == 0 && mixed && m <= split && m % 2 != 0); };
+        double lo = 0.0, hi = 1.0;
+        for (int m = 0; m <= L; m += P)
+            hi += column(m);
+        auto fill = [&](double limit) {
+            int m = 0;
+            for (int w = 0; w < kColumnWarps; ++w) {
+                plan.b[k][w] = (short)m;
+                int end = m;
+                double c = 0.0;
+                for (int e = m + 1; e <= L + 1; ++e) {
+                    if ((e - 1 - m) % P == 0)
+                        c += column(e - 1);
+                    if (c > limit)
+                        break;
+                    if (allowed(e) || e == L + 1)
+                        end = e;
+                }
+                m = end;
+            }
+            plan.b[k][kColumnWarps] = (short)m;
+            return m == L + 1;
+        };
+        for (int it = 0; it < 40; ++it) {
+            const double mid = (lo + hi) / 2;
+            (fill(mid) ? hi : lo) = mid;
+        }
+        fill(hi);
+    }
+    return plan;
+}
+
 void build_gravity_tables(const ModelData& md, std::vector<GravEntry64>& t64, std::vector<GravEntry32>& t32)
 {
     const int L = md.degree;

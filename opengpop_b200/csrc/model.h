@@ -45,6 +45,14 @@ struct CorrModel {
 };
 CorrModel corrector_model(const ModelData& md);
 
+// Column ranges of the eight warps that walk a set of objects together (columns.cu): warp w takes columns
+// b[k][w] .. b[k][w + 1] - 1, for sets whose pairs of objects have 2^k lanes each.
+constexpr int kColumnWarps = 8;
+struct ColumnPlan {
+    short b[5][kColumnWarps + 1] = {};
+};
+ColumnPlan column_plan(int L, bool mixed);
+
 // Gravity table entry, one per (n, m) with n >= m, stored column by column (m outer, n = m..L).
 // With the rescaled derived-Legendre recursion
 //   Q(m,m) = q^m, Q(m+1,m) = u Q(m,m), Q(n,m) = u Q(n-1,m) - c(n,m) w Q(n-2,m)

@@ -125,6 +125,7 @@ extern "C" gpop_status gpop_propagate_device_noalloc(gpop_ctx* ctx, const gpop_t
     // the same walk and tables as gpop_propagate_device (both built when the context was made)
     const TableSrc ts = ctx->table(mixed);
     const TableSrc lane_ts = ctx->lane_table(mixed);
+    const TableSrc lane64 = ctx->lane_table(false);
     PropArgs a;
     a.n = n;
     a.h = h;
@@ -137,7 +138,7 @@ extern "C" gpop_status gpop_propagate_device_noalloc(gpop_ctx* ctx, const gpop_t
     a.err = err;
     a.r0 = r_dev;
     a.v0 = v_dev;
-    if ((e = launch_startup(ts, a, ctx->num_sms, s, &lane_ts)) != cudaSuccess)
+    if ((e = launch_startup(ts, a, ctx->num_sms, s, &lane_ts, &lane64)) != cudaSuccess)
         return cuda_fail(ctx, e, "startup kernel");
     const int chunk = ctx->steps_per_launch;
     for (int b = 1; b <= steps; b += chunk) {
@@ -146,7 +147,8 @@ extern "C" gpop_status gpop_propagate_device_noalloc(gpop_ctx* ctx, const gpop_t
         const bool last = a.step_end == steps + 1;
         a.out_r = last ? r_dev : nullptr;
         a.out_v = last ? v_dev : nullptr;
-        if ((e = launch_gj8(ts, a, ctx->num_sms, s, ctx->block_override, ctx->walk_mode, &lane_ts))
+        if ((e = launch_gj8(ts, a, ctx->num_sms, s, ctx->block_override, ctx->walk_mode, &lane_ts,
+                 &lane64))
             != cudaSuccess)
             return cuda_fail(ctx, e, "GJ8 kernel");
     }

@@ -104,6 +104,9 @@ struct ForceAnalytic {
     }
 };
 
+constexpr int kTeamBlock = 256; // largest block of gj8_team_kernel
+constexpr int kLanesBlock = 384; // threads per SM the lane walks are spread to
+
 // ---- table staging ----
 size_t table_smem_bytes(const TableSrc& ts) { return 128 + (size_t)ts.bytes; }
 
@@ -642,19 +645,149 @@ __global__ void __launch_bounds__(K == 1 ? kOneObjectBlock : 256, 1) gj8_kernel(
     }
 }
 
-// ---- GJ8 step with P lanes per group of K objects (few objects) ----
-// Same step as gj8_kernel; the P lanes of a group split the gravity columns of its K objects
-// (lanes.cuh, lane-layout table) and hold identical state; lane 0 of the group stores. Object k
-// of group g is g + k * (groups in the grid). Used when the objects alone leave most warp slots of
-// the GPU empty. MAXT bounds the block (and so the registers a thread may hold): 512 for the many
-// lanes of few objects, 384 for two lanes per object, which then keeps its table loads in flight.
-// STAGE: the corrector's constants of a step (as in gj8_kernel) wait in shared memory during
-// the gravity walks, one copy per lane group written by its lead lane, as in gj8_kernel (two
-// objects per lane group, FP64, 18,944 objects at four lanes: the walk at 254 registers waited on
-// its table loads, short_scoreboard 1.43 per issued instruction, FP64 pipe 59 % busy).
-template <bool MIXED, int K, int MAXT = (K == 1 ? 512 : 256), bool STAGE = false>
-__global__ void __launch_bounds__(MAXT, 1) gj8_lanes_kernel(TableSrc ts, PropArgs a, int P)
+// ---- GJ8 step with a group of lanes per object (few objects) ----
+// Same step as gj8_kernel; the lanes of an object's group split its gravity columns (lanes.cuh, lane-layout
+// table) and hold identical state, and lane 0 stores. A group is P lanes of a warp, or (WARPS) whole warps
+// with a lane per column. The acceleration history lies in shared memory for the launch.
+// Bounds: the latency of an evaluation (one chain of FMAs per column, then a sum over the lanes), so what a
+// step needs besides is kept short: history and sums in shared memory, the next step's rotation prefetched.
+// Blocks of at most 256 threads: with 255 registers a step of one object on 32 lanes takes 9.2 us at 70x70
+// (FP64), with the 168 of 384 threads 16.9.
+template <bool MIXED, bool WARPS>
+__global__ void __launch_bounds__(kTeamBlock, 1) gj8_team_kernel(TableSrc ts, PropArgs a, int P)
 {
+    extern __shared__ __align__(128) uint8_t smem[];
+    GravSmem g;
+    if (!bind_lane_table(smem, ts, a.err, g))
+        return;
+    const int64_t n = a.n; // the state's stride; this launch runs objects [lo, hi)
+    const int64_t lo = a.obj_lo, hi = a.obj_hi < 0 ? n : a.obj_hi;
+    const int in_block = (int)threadIdx.x / P;
+    const int64_t obj = lo + (int64_t)blockIdx.x * (blockDim.x / P) + in_block;
+    const int in_warp = (int)blockDim.x - (int)(threadIdx.x & ~31u); // the block's last warp may be partial
+    const unsigned warp = __ballot_sync(in_warp >= 32 ? 0xffffffffu : (1u << in_warp) - 1u, obj < hi);
+    if (obj >= hi)
+        return; // whole groups leave: shuffles and barriers name the group only
+    // per group: 27 doubles of history [slot][axis], then 8 per warp for the sums of a group of warps
+    double* hist = reinterpret_cast<double*>(smem + stage_offset(ts)) + (size_t)in_block * team_doubles(P, WARPS);
+    const auto team = make_team<WARPS>(P, hist + 27);
+    const int l = team.l;
+    const bool lead = l == 0;
+    double* st = a.state + obj;
+    for (int i = l; i < 27; i += P)
+        hist[i] = st[(kHist + i) * n];
+    team.sync();
+    const double h = a.h;
+    double r[1][3], v[3], s[3], S[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        r[0][j] = st[(kR + j) * n];
+        v[j] = st[(kV + j) * n];
+        s[j] = st[(kSs + j) * n];
+        S[j] = st[(kSb + j) * n];
+    }
+    int ring0 = a.step_begin >= 5 ? (a.step_begin - 5) % 9 : 0;
+    for (int step = a.step_begin; step < a.step_end; ++step) {
+        double a8[1][3];
+        if (step <= 4) {
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                r[0][j] = st[(kRep + (step - 1) * 6 + j) * n];
+                v[j] = st[(kRep + (step - 1) * 6 + 3 + j) * n];
+                a8[0][j] = st[(kRepA + (step - 1) * 3 + j) * n];
+            }
+        } else {
+            const double* M = a.prop_m + (size_t)(step + 4) * 9;
+            if (l < 2 && step + 1 < a.step_end) // the next step's rotation
+                asm volatile("prefetch.global.L1 [%0];" ::"l"(M + 9 + 8 * l));
+            double s1[3], s2[3], prev[3], a7[3];
+#pragma unroll
+            for (int j = 0; j < 3; ++j) { // as gj8_kernel
+                double q[9];
+#pragma unroll
+                for (int c = 0; c < 9; ++c) {
+                    int slot = ring0 + c;
+                    slot -= slot >= 9 ? 9 : 0;
+                    q[c] = hist[slot * 3 + j];
+                }
+                double rt = 0.0, c1 = 0.0, c2 = 0.0;
+#pragma unroll
+                for (int c = 0; c < 9; ++c)
+                    rt = fma(q[c], c_GJ[9][c], rt);
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    c1 = fma(q[c + 1], c_SA[8][c], c1);
+                    c2 = fma(q[c + 1], c_GJ[8][c], c2);
+                }
+                S[j] += s[j] + q[8] / 2;
+                r[0][j] = (rt + S[j]) * h * h;
+                s1[j] = c1;
+                s2[j] = c2;
+                prev[j] = s[j];
+                a7[j] = q[8];
+            }
+            bool fast = false;
+            for (int it = 0; it < a.ncorr; ++it) {
+                gravity_gcrs_team<MIXED, 1, !WARPS>(g, team, M, r, a8);
+                if (correct_position(ts.corr, h, it, a.ncorr, s2, S, a8[0], r[0], fast))
+                    break; // the same for the lanes of a group
+            }
+            if constexpr (!WARPS)
+                __syncwarp(warp); // groups that were done earlier wait: the warp's walks stay converged
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                s[j] = prev[j] + (a8[0][j] + a7[j]) / 2;
+                v[j] = h * (s1[j] + a8[0][j] * c_SA[8][8] + s[j]);
+            }
+            if (lead)
+#pragma unroll
+                for (int j = 0; j < 3; ++j)
+                    hist[ring0 * 3 + j] = a8[0][j];
+            team.sync(); // the ring write precedes the group's loads of the next step
+            ring0 = ring0 == 8 ? 0 : ring0 + 1;
+        }
+        if (lead) {
+            const int64_t t = step - a.traj_step0;
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                if (a.traj_r)
+                    a.traj_r[(t * 3 + j) * n + obj] = r[0][j];
+                if (a.traj_v)
+                    a.traj_v[(t * 3 + j) * n + obj] = v[j];
+                if (a.traj_a)
+                    a.traj_a[(t * 3 + j) * n + obj] = a8[0][j];
+            }
+        }
+    }
+    for (int i = l; i < 27; i += P)
+        st[(kHist + i) * n] = hist[i];
+    if (!lead)
+        return;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        st[(kR + j) * n] = r[0][j];
+        st[(kV + j) * n] = v[j];
+        st[(kSs + j) * n] = s[j];
+        st[(kSb + j) * n] = S[j];
+        if (a.out_r)
+            a.out_r[obj * 3 + j] = r[0][j];
+        if (a.out_v)
+            a.out_v[obj * 3 + j] = v[j];
+    }
+}
+
+// ---- GJ8 step with P lanes per group of two objects ----
+// Same step as gj8_kernel; the P lanes of a group split the gravity columns of its two objects (lanes.cuh,
+// lane-layout table) and hold identical state; lane 0 of the group stores. Object k of group g is
+// g + k * (groups in the grid).
+// STAGE: the corrector's constants of a step (as in gj8_kernel) wait in shared memory during
+// the gravity walks, one copy per lane group written by its lead lane (FP64, 18,944 objects at four lanes:
+// the walk at 254 registers waited on its table loads, short_scoreboard 1.43 per issued instruction, FP64
+// pipe 59 % busy).
+template <bool MIXED, bool STAGE>
+__global__ void __launch_bounds__(256, 1) gj8_lanes_kernel(TableSrc ts, PropArgs a, int P)
+{
+    constexpr int K = 2;
     extern __shared__ __align__(128) uint8_t smem[];
     GravSmem g;
     if (!bind_lane_table(smem, ts, a.err, g))
@@ -760,10 +893,7 @@ __global__ void __launch_bounds__(MAXT, 1) gj8_lanes_kernel(TableSrc ts, PropArg
             const double* M = a.prop_m + (size_t)(step + 4) * 9;
             bool done[K] = {}, fast[K] = {};
             for (int it = 0; it < a.ncorr; ++it) { // as gj8_kernel
-                // two columns at a time for one object per group at up to 384 threads a block (FP64
-                // 1,024 objects: 18.8 against 17.4 M object-steps/s); with two objects per group,
-                // or the 128 registers of 512-thread blocks, that spills (-9 %)
-                gravity_gcrs_lk<MIXED, K, K == 1 && MAXT <= 384>(g, l, P, M, r, a8, mask);
+                gravity_gcrs_lk<MIXED, K>(g, l, P, M, r, a8, mask); // (two columns at a time spill)
                 bool all = true;
 #pragma unroll
                 for (int k = 0; k < K; ++k) {
@@ -994,7 +1124,7 @@ template <class K> static cudaError_t set_smem(K kernel, size_t bytes)
 }
 
 cudaError_t launch_startup(const TableSrc& ts, const PropArgs& a, int num_sms, cudaStream_t s,
-    const TableSrc* lane_ts)
+    const TableSrc* lane_ts, const TableSrc* lane64)
 {
     if (a.n <= 0)
         return cudaSuccess;
@@ -1015,7 +1145,8 @@ cudaError_t launch_startup(const TableSrc& ts, const PropArgs& a, int num_sms, c
         b.err = a.err;
         b.stage_pos = a.stage_pos;
         b.col_pos = a.col_pos;
-        return launch_startup_gravity(ts, *lane_ts, b, num_sms, s);
+        // few objects: the FP64 table, as their steps (step_walk)
+        return launch_startup_gravity(ts, lane64 && 2 * a.n <= 4 * (int64_t)num_sms ? *lane64 : *lane_ts, b, num_sms, s);
     }
     LaunchShape ls = pick_shape(a.n, 256, num_sms);
     if (a.kind == 0) {
@@ -1139,12 +1270,7 @@ static cudaError_t launch_gj8_f(F f, const TableSrc& ts, const PropArgs& a, int 
     return launch_gj8_k<F, 1>(f, ts, a, num_sms, s, block_override);
 }
 
-#ifndef GPOP_LANES_BLOCK_MID
-#define GPOP_LANES_BLOCK_MID 384
-#endif
-constexpr int kLanesBlockMid = GPOP_LANES_BLOCK_MID; // blocks up to this size take the MAXT = 384 kernel
-
-// The most lanes that keep every object in one wave of blocks of at most kLanesBlockMid threads,
+// The most lanes that keep every object in one wave of blocks of at most kLanesBlock threads,
 // so that the lane kernel runs with the registers of its 384-thread variant: fewer lanes with
 // more registers beat more lanes with 128 (B200, 70x70, FP64 / mixed M object-steps/s: 2,048
 // objects 19.0 / 26.1 against 16.2 / 21.2 with 512-thread blocks; 4,096: 25.6 / 36.1 against
@@ -1152,7 +1278,7 @@ constexpr int kLanesBlockMid = GPOP_LANES_BLOCK_MID; // blocks up to this size t
 int lanes_per_object(int64_t n, int num_sms)
 {
     int P = 1;
-    while (P < 32 && n * 2 * P <= (int64_t)num_sms * kLanesBlockMid)
+    while (P < 32 && n * 2 * P <= (int64_t)num_sms * kLanesBlock)
         P *= 2;
     return P;
 }
@@ -1202,7 +1328,7 @@ int default_walk(int64_t n, int num_sms, bool lanes, bool fp64_gravity)
 {
     if (lanes && lane_pair_lanes(n, num_sms, fp64_gravity) > 0)
         return kWalkLanesTwo;
-    if (lanes && (n <= (int64_t)num_sms * 128 || (fp64_gravity && 2 * n <= (int64_t)num_sms * kLanesBlockMid)))
+    if (lanes && (n <= (int64_t)num_sms * 128 || (fp64_gravity && 2 * n <= (int64_t)num_sms * kLanesBlock)))
         return kWalkLanes;
     if (n >= (int64_t)num_sms * 128)
         return fp64_gravity && n <= (int64_t)num_sms * 256 ? kWalkOneObject : kWalkTwoObjects;
@@ -1222,70 +1348,125 @@ static cudaError_t launch_lanes_range(const TableSrc& lt, const PropArgs& a0, in
     const int64_t groups = (hi - lo + K - 1) / K;
     const int64_t threads = groups * P;
     const int64_t per_sm = (threads + num_sms - 1) / num_sms; // spread over every SM
-    const int cap = K == 1 ? 512 : 256;
-    const int block = (int)std::min<int64_t>(cap, std::max<int64_t>(32, ((per_sm + P - 1) / P) * P));
+    const int cap = K == 1 ? kTeamBlock : 256;
+    const int block = (int)std::min<int64_t>(cap / P * P, std::max<int64_t>(std::max(32, P), ((per_sm + P - 1) / P) * P));
     const unsigned grid = (unsigned)((threads + block - 1) / block);
-    const size_t smem = table_smem_bytes(lt);
+    cudaError_t e;
+    if (K == 1) {
+        const bool warps = P > 32;
+        const size_t bytes = stage_offset(lt) + (size_t)(block / P) * team_doubles(P, warps) * 8;
+        auto launch = [&](auto kernel) {
+            if ((e = set_smem(kernel, bytes)) != cudaSuccess)
+                return e;
+            kernel<<<grid, block, bytes, s>>>(lt, a, P);
+            return cudaGetLastError();
+        };
+        if (lt.mixed)
+            return warps ? launch(gj8_team_kernel<true, true>) : launch(gj8_team_kernel<true, false>);
+        return warps ? launch(gj8_team_kernel<false, true>) : launch(gj8_team_kernel<false, false>);
+    }
     // two objects per lane group: the corrector's constants parked in shared memory, one copy per
     // group (gj8_lanes_kernel STAGE), when they fit beside the table
-#ifndef GPOP_STAGE_LANES
-#define GPOP_STAGE_LANES 1
-#endif
-    const size_t staged = GPOP_STAGE_LANES ? stage_offset(lt) + (size_t)kStageDoubles * K * 8 * (block / P)
-                                           : (size_t)1 << 40;
-    cudaError_t e;
-    if (lt.mixed) {
-        if (K == 1 && block <= kLanesBlockMid) {
-            if ((e = set_smem(gj8_lanes_kernel<true, 1, kLanesBlockMid>, smem)) != cudaSuccess)
-                return e;
-            gj8_lanes_kernel<true, 1, kLanesBlockMid><<<grid, block, smem, s>>>(lt, a, P);
-        } else if (K == 1) {
-            if ((e = set_smem(gj8_lanes_kernel<true, 1>, smem)) != cudaSuccess)
-                return e;
-            gj8_lanes_kernel<true, 1><<<grid, block, smem, s>>>(lt, a, P);
-        } else {
-            if (staged <= max_smem_optin()) {
-                if ((e = set_smem(gj8_lanes_kernel<true, 2, 256, true>, staged)) != cudaSuccess)
-                    return e;
-                gj8_lanes_kernel<true, 2, 256, true><<<grid, block, staged, s>>>(lt, a, P);
-            } else {
-                if ((e = set_smem(gj8_lanes_kernel<true, 2>, smem)) != cudaSuccess)
-                    return e;
-                gj8_lanes_kernel<true, 2><<<grid, block, smem, s>>>(lt, a, P);
-            }
+    const size_t smem = table_smem_bytes(lt);
+    const size_t staged = stage_offset(lt) + (size_t)kStageDoubles * K * 8 * (block / P);
+    auto launch = [&](auto kernel, size_t bytes) {
+        if ((e = set_smem(kernel, bytes)) != cudaSuccess)
+            return e;
+        kernel<<<grid, block, bytes, s>>>(lt, a, P);
+        return cudaGetLastError();
+    };
+    if (staged <= max_smem_optin())
+        return lt.mixed ? launch(gj8_lanes_kernel<true, true>, staged) : launch(gj8_lanes_kernel<false, true>, staged);
+    return lt.mixed ? launch(gj8_lanes_kernel<true, false>, smem) : launch(gj8_lanes_kernel<false, false>, smem);
+}
+
+// The walk of cnt objects' steps when none is forced, by objects per SM (o) and degree. Measured on B200, us
+// per step of n = 148 o objects (64-step calls, LEO, 30 s), FP64 / mixed; T<P> a group of P lanes per object, C
+// the columns over a block's warps, 1 and 2 objects per thread, 2p two without the split block:
+//   70x70   o = 1: T96 7.2 / 9.1, T32 9.2 / 10.3       4: T32 11.4 / 11.1, C 11.9 / 13.8
+//           8: C 13.8 / 13.9, T32 16.7 / 14.8         16: C 18.6 / 15.3, T8 24.7 / 21.6
+//          64: C 40.6 / 25.1, 1 91.2 / 89.1          128: C 78.7 / 45.7, 1 94.1 / 90.9
+//         256: C 152 / 87, 2p 156 / 96               320: C 193 / 112, 2 237 / 122
+//         384: C 229 / 133, 2 237 / 122              448: 2 237 / 123, C 266 / 155       512: 2p 260 / 141
+//   50x50   o = 8: T16 11.9 / 10.3, C 12.0 / 11.4    320: C 109 / 72, 2 122 / 67         448: 2 134 / 84, 2p 140 / 82
+//   36x36   o = 24: T8 13.1 / 11.7, C 13.8 / 12.2     32: C 13.7 / 12.2, T8 15.6 / 12.5
+//         192: C 41.2 / 29.1, 1 43.8 / 37.8          256: 1 47.1 / 38.5, 2p 49.9 / 37.6
+//         384: 2 66 / 40                             448: 2p 78 / 51, 2 90 / 64
+//   20x20   o = 4: T32 4.7 / 5.9, T16 6.1 / 5.7       16: T8 6.2 / 6.7, C 8.6 / 9.8
+//          64: C 9.1 / 9.3, T4 11.9 / 10.1           128: 1 13.6 / 15.1, C 14.5 / 14.5
+//         256: 1 18.4 / 17.8, 2p 21.0 / 20.0         448: 2p 31 / 25, 2 49 / 43
+//   8x8     o = 32: T4 3.2 / 3.5                      64: T4 3.6 / 3.8, 1 3.6 / 4.2
+//         128: 1 3.8 / 4.5, 2p 5.8 / 6.1             320: 2p 7.4 / 7.5, 1 8.2 / 9.6
+// With up to four objects per SM the FP64 table is the faster one in mixed precision too (1 object: 7.2 against
+// 9.1 us): a chain of FP64 terms and one of FP32 terms take turns there.
+struct StepWalk {
+    enum Kind { kTeam, kColumns, kOne, kTwo, kTwoPlain } kind = kTwo;
+    int P = 1;
+    bool fp64 = false;
+};
+static StepWalk step_walk(int64_t cnt, int num_sms, int L, bool mixed)
+{
+    StepWalk w;
+    const int64_t o = (cnt + num_sms - 1) / num_sms;
+    const int64_t team = L < 14 ? 64 : L < 28 ? 32 : L < 43 ? 24 : L < 60 ? 8 : 4;
+    const int64_t columns = L < 14 ? 0
+        : L < 28                   ? (mixed ? 128 : 64)
+        : L < 43                   ? 224
+        : L < 60                   ? (mixed ? 256 : 320)
+                                   : (mixed ? 320 : 384);
+    if (o <= team) {
+        const int W = (L + 32) / 32; // warps that hold a column per lane
+        w.kind = StepWalk::kTeam;
+        w.fp64 = o <= 4;
+        if (W > 1 && o <= 2) {
+            w.P = 32 * W;
+            return w;
         }
-    } else {
-        if (K == 1 && block <= kLanesBlockMid) {
-            if ((e = set_smem(gj8_lanes_kernel<false, 1, kLanesBlockMid>, smem)) != cudaSuccess)
-                return e;
-            gj8_lanes_kernel<false, 1, kLanesBlockMid><<<grid, block, smem, s>>>(lt, a, P);
-        } else if (K == 1) {
-            if ((e = set_smem(gj8_lanes_kernel<false, 1>, smem)) != cudaSuccess)
-                return e;
-            gj8_lanes_kernel<false, 1><<<grid, block, smem, s>>>(lt, a, P);
-        } else {
-            if (staged <= max_smem_optin()) {
-                if ((e = set_smem(gj8_lanes_kernel<false, 2, 256, true>, staged)) != cudaSuccess)
-                    return e;
-                gj8_lanes_kernel<false, 2, 256, true><<<grid, block, staged, s>>>(lt, a, P);
-            } else {
-                if ((e = set_smem(gj8_lanes_kernel<false, 2>, smem)) != cudaSuccess)
-                    return e;
-                gj8_lanes_kernel<false, 2><<<grid, block, smem, s>>>(lt, a, P);
-            }
-        }
+        // the most lanes that leave at most `threads` per SM, within what the degree can use
+        const int threads = L < 14 || !mixed ? 128 : 256;
+        w.P = 4;
+        while (w.P < (L < 14 ? 16 : 32) && o * 2 * w.P <= threads)
+            w.P *= 2;
+        if (L >= 14 && L < 28 && !mixed && o > 4)
+            w.P = 8;
+        return w;
     }
-    return cudaGetLastError();
+    if (o <= columns)
+        w.kind = StepWalk::kColumns;
+    else if (o <= 256 && (L < 28 || !mixed))
+        w.kind = StepWalk::kOne;
+    else if (L < 14 || o > 448 || (o > 384 && L < 45))
+        w.kind = StepWalk::kTwoPlain;
+    return w;
 }
 
 cudaError_t launch_gj8(const TableSrc& ts, const PropArgs& a, int num_sms, cudaStream_t s,
-    int block_override, int walk, const TableSrc* lane_ts)
+    int block_override, int walk, const TableSrc* lane_ts, const TableSrc* lane64)
 {
     // objects [lo, hi) of the n the state holds
     const int64_t lo = a.obj_lo, hi = a.obj_hi < 0 ? a.n : a.obj_hi, cnt = hi - lo;
     if (cnt <= 0 || lo < 0 || hi > a.n || a.step_end <= a.step_begin)
         return cudaSuccess;
     const bool forced = walk > 0;
+    if (walk <= 0 && a.kind == 0 && lane_ts && block_override <= 0
+        && !(ts.mixed && (a.flags & kFlagMixedCompensated))) {
+        const StepWalk w = step_walk(cnt, num_sms, ts.L, ts.mixed);
+        switch (w.kind) {
+        case StepWalk::kTeam:
+            return launch_lanes_range(w.fp64 && lane64 ? *lane64 : *lane_ts, a, 1, w.P, lo, hi, num_sms, s);
+        case StepWalk::kColumns:
+            return launch_gj8_columns(*lane_ts, a, num_sms, s);
+        case StepWalk::kOne:
+            walk = kWalkOneObject;
+            break;
+        case StepWalk::kTwoPlain:
+            walk = cnt > (int64_t)num_sms * 512 ? kWalkTwoObjects : kWalkTwoPlain;
+            break;
+        case StepWalk::kTwo:
+            walk = kWalkTwoObjects;
+            break;
+        }
+    }
     const bool comp = a.kind == 0 && ts.mixed && (a.flags & kFlagMixedCompensated);
     if (walk <= 0)
         walk = default_walk(cnt, num_sms, lane_ts && a.kind == 0 && !comp, a.kind == 0 && !ts.mixed);
@@ -1305,12 +1486,12 @@ cudaError_t launch_gj8(const TableSrc& ts, const PropArgs& a, int num_sms, cudaS
             const int64_t full = cnt / wave * wave;
             PropArgs b = a;
             b.obj_hi = lo + full;
-            cudaError_t e = launch_gj8(ts, b, num_sms, s, block_override, kWalkTwoPlain, lane_ts);
+            cudaError_t e = launch_gj8(ts, b, num_sms, s, block_override, kWalkTwoPlain, lane_ts, lane64);
             if (e != cudaSuccess || full == cnt)
                 return e;
             PropArgs c = a;
             c.obj_lo = lo + full;
-            return launch_gj8(ts, c, num_sms, s, block_override, forced ? walk : 0, lane_ts);
+            return launch_gj8(ts, c, num_sms, s, block_override, forced ? walk : 0, lane_ts, lane64);
         }
     }
     if ((walk == kWalkLanes || walk == kWalkLanesTwo) && a.kind == 0 && lane_ts) {

@@ -298,28 +298,8 @@ template <class Team> struct KeepShared {
     __device__ __forceinline__ void sync() const { team.sync(); }
 };
 
-// Lanes per group as gravity_itrs_team takes them: P <= 32 lanes of a warp, or whole warps.
-template <bool WARPS> struct TeamOf;
-template <> struct TeamOf<false> {
-    using type = WarpTeam;
-};
-template <> struct TeamOf<true> {
-    using type = BlockTeam;
-};
-template <bool WARPS>
-__device__ __forceinline__ typename TeamOf<WARPS>::type make_team(int P, double* buf)
-{
-    const int l = (int)threadIdx.x % P;
-    if constexpr (WARPS) {
-        return BlockTeam { l, P, P / 32, 1 + (int)threadIdx.x / P, buf, 0 };
-    } else {
-        const int lane = (int)threadIdx.x & 31;
-        return WarpTeam { l, P, P == 32 ? 0xffffffffu : ((1u << P) - 1u) << (lane & ~(P - 1)) };
-    }
-}
-
 template <bool MIXED, bool WARPS, bool BATCH>
-__global__ void __launch_bounds__(384, 1) startup_rk8_team_kernel(TableSrc ts, StartupArgs a, int P)
+__global__ void __launch_bounds__(256, 1) startup_rk8_team_kernel(TableSrc ts, StartupArgs a, int P)
 {
     extern __shared__ __align__(128) uint8_t smem[];
     clear_counters(a);
@@ -429,7 +409,7 @@ __global__ void __launch_bounds__(256, 1) startup_eval_kernel(TableSrc ts, Start
 }
 
 template <bool MIXED, bool WARPS, bool BATCH>
-__global__ void __launch_bounds__(384, 1) startup_eval_team_kernel(TableSrc ts, StartupArgs a, int pass, int P)
+__global__ void __launch_bounds__(256, 1) startup_eval_team_kernel(TableSrc ts, StartupArgs a, int pass, int P)
 {
     extern __shared__ __align__(128) uint8_t smem[];
     const EvalItems items(a, pass);
@@ -619,8 +599,8 @@ template <class Kern> cudaError_t smem_of(Kern kernel, size_t bytes)
 }
 
 // Lanes per evaluation of `items` independent evaluations: the warps that hold a column per lane while
-// every SM has at most one such group, else the most lanes (<= 32) that leave one block of 384 threads
-// per SM; 0 where one evaluation per thread (plain kernels) is the better walk.
+// every SM has at most one such group, else the most lanes (<= 32) that leave one block of 256 threads
+// (255 registers: at 168 the walk waits on its table loads, 1.7 times as long) per SM; 0 where one evaluation per thread (plain kernels) is the better walk.
 struct TeamShape {
     int P = 0; // threads per group (0: plain kernels)
     bool warps = false;
@@ -637,7 +617,7 @@ TeamShape team_shape(int64_t items, int L, int num_sms)
     if (items > (int64_t)num_sms * 96)
         return t;
     t.P = 2;
-    while (t.P < 32 && items * 2 * t.P <= (int64_t)num_sms * 384)
+    while (t.P < 32 && items * 2 * t.P <= (int64_t)num_sms * 256)
         t.P *= 2;
     return t;
 }
@@ -645,11 +625,12 @@ TeamShape team_shape(int64_t items, int L, int num_sms)
 void team_grid(int64_t items, int P, int num_sms, int& block, unsigned& grid)
 {
     const int64_t per_sm = (items + num_sms - 1) / num_sms;
-    const int64_t groups = std::max<int64_t>(std::max(1, 32 / P), std::min<int64_t>(per_sm, 384 / P));
+    const int64_t groups = std::max<int64_t>(std::max(1, 32 / P), std::min<int64_t>(per_sm, 256 / P));
     block = (int)groups * P;
     grid = (unsigned)((items + groups - 1) / groups);
 }
 
+// The team kernels take the precision of the lane table, the others MIXED.
 template <bool MIXED, bool BATCH>
 cudaError_t launch_rk8(const TableSrc& plain, const TableSrc& lanes, const StartupArgs& a, int num_sms, cudaStream_t s)
 {
@@ -661,16 +642,17 @@ cudaError_t launch_rk8(const TableSrc& plain, const TableSrc& lanes, const Start
         team_grid(2 * a.n, t.P, num_sms, block, grid);
         const size_t bytes = stage_offset(lanes) + (size_t)(block / t.P) * (30 + (t.warps ? t.P / 4 : 0)) * 8;
         if (bytes <= max_smem_optin()) {
-            if (t.warps) {
-                if ((e = smem_of(startup_rk8_team_kernel<MIXED, true, BATCH>, bytes)) != cudaSuccess)
+            auto launch = [&](auto kernel) {
+                if ((e = smem_of(kernel, bytes)) != cudaSuccess)
                     return e;
-                startup_rk8_team_kernel<MIXED, true, BATCH><<<grid, block, bytes, s>>>(lanes, a, t.P);
-            } else {
-                if ((e = smem_of(startup_rk8_team_kernel<MIXED, false, BATCH>, bytes)) != cudaSuccess)
-                    return e;
-                startup_rk8_team_kernel<MIXED, false, BATCH><<<grid, block, bytes, s>>>(lanes, a, t.P);
-            }
-            return cudaGetLastError();
+                kernel<<<grid, block, bytes, s>>>(lanes, a, t.P);
+                return cudaGetLastError();
+            };
+            if (lanes.mixed)
+                return t.warps ? launch(startup_rk8_team_kernel<true, true, BATCH>)
+                               : launch(startup_rk8_team_kernel<true, false, BATCH>);
+            return t.warps ? launch(startup_rk8_team_kernel<false, true, BATCH>)
+                           : launch(startup_rk8_team_kernel<false, false, BATCH>);
         }
     }
     // two objects per thread where that still leaves a block of four warps per SM
@@ -701,16 +683,17 @@ cudaError_t launch_eval(const TableSrc& plain, const TableSrc& lanes, const Star
         unsigned grid;
         team_grid(items, t.P, num_sms, block, grid);
         const size_t bytes = stage_offset(lanes) + (t.warps ? (size_t)(block / t.P) * (t.P / 4) * 8 : 0);
-        if (t.warps) {
-            if ((e = smem_of(startup_eval_team_kernel<MIXED, true, BATCH>, bytes)) != cudaSuccess)
+        auto launch = [&](auto kernel) {
+            if ((e = smem_of(kernel, bytes)) != cudaSuccess)
                 return e;
-            startup_eval_team_kernel<MIXED, true, BATCH><<<grid, block, bytes, s>>>(lanes, a, pass, t.P);
-        } else {
-            if ((e = smem_of(startup_eval_team_kernel<MIXED, false, BATCH>, bytes)) != cudaSuccess)
-                return e;
-            startup_eval_team_kernel<MIXED, false, BATCH><<<grid, block, bytes, s>>>(lanes, a, pass, t.P);
-        }
-        return cudaGetLastError();
+            kernel<<<grid, block, bytes, s>>>(lanes, a, pass, t.P);
+            return cudaGetLastError();
+        };
+        if (lanes.mixed)
+            return t.warps ? launch(startup_eval_team_kernel<true, true, BATCH>)
+                           : launch(startup_eval_team_kernel<true, false, BATCH>);
+        return t.warps ? launch(startup_eval_team_kernel<false, true, BATCH>)
+                       : launch(startup_eval_team_kernel<false, false, BATCH>);
     }
     const size_t bytes = table_smem_bytes(plain);
     if (!BATCH && items >= (int64_t)num_sms * 384) {
