@@ -15,6 +15,11 @@ namespace {
 
 struct ScopedBufs {
     DevBuf b[12];
+    explicit ScopedBufs(const gpop_ctx* ctx)
+    {
+        for (DevBuf& x : b)
+            x.use(ctx->pool, true);
+    }
     ~ScopedBufs()
     {
         for (DevBuf& x : b)
@@ -77,12 +82,19 @@ gpop_status begin(gpop_ctx* ctx, gpop_propagator& p, const gpop_time* start, dou
     p.r = r;
     p.v = v;
     p.mixed = false;
+    for (DevBuf* b : { &p.own_state, &p.own_gen, &p.own_prop })
+        b->use(ctx->pool, true);
     return propagator_init(&p, s);
 }
 
 // Positions of the startup's stages and columns, their Jacobians and the startup tangents.
 struct StartupTangents {
     DevBuf stage_pos, col_pos, stage_jac, col_jac, out;
+    explicit StartupTangents(const gpop_ctx* ctx)
+    {
+        for (DevBuf* b : { &stage_pos, &col_pos, &stage_jac, &col_jac, &out })
+            b->use(ctx->pool, true);
+    }
     ~StartupTangents()
     {
         for (DevBuf* b : { &stage_pos, &col_pos, &stage_jac, &col_jac, &out })
@@ -177,12 +189,17 @@ gpop_status run_adjoint(gpop_ctx* ctx, gpop_propagator& p, int32_t steps, const 
     const int64_t U = (int64_t)step0.size(), n = p.n;
     struct Bufs {
         DevBuf rank, sweep, jac, offset, pos;
+        explicit Bufs(const gpop_ctx* ctx)
+        {
+            for (DevBuf* b : { &rank, &sweep, &jac, &offset, &pos })
+                b->use(ctx->pool, true);
+        }
         ~Bufs()
         {
             for (DevBuf* b : { &rank, &sweep, &jac, &offset, &pos })
                 b->release();
         }
-    } B;
+    } B(ctx);
     // ranks: units by their last seeded step, latest first
     std::vector<int> rank(2 * U); // unit, then object of each rank
     for (int64_t u = 0; u < U; ++u)
@@ -305,6 +322,8 @@ gpop_status run_adjoint(gpop_ctx* ctx, gpop_propagator& p, int32_t steps, const 
                 ~Free() { b.release(); }
             } free_rv { rv };
             const size_t bytes = (size_t)f.n * 3 * sizeof(double);
+            rv.use(ctx->pool, true);
+            q.own_state.use(ctx->pool, true);
             if ((e = rv.ensure(2 * bytes)) != cudaSuccess || (e = q.own_state.ensure(state_bytes(f.n))) != cudaSuccess)
                 return nomem(ctx, "startup tangents", e);
             q.ctx = ctx;
@@ -381,9 +400,9 @@ gpop_status gpop_stm(gpop_ctx* ctx, const gpop_time* start, double h, int32_t st
     cudaStream_t s = nullptr;
     for (int64_t lo = 0; lo < n; lo += kVarObjects) {
         const int64_t m = std::min(kVarObjects, n - lo);
-        ScopedBufs B;
+        ScopedBufs B(ctx);
         DevBuf &dr = B.b[0], &dv = B.b[1], &dphi = B.b[2], &pos = B.b[3], &jac = B.b[4], &sweep = B.b[5];
-        StartupTangents tan;
+        StartupTangents tan(ctx);
         gpop_propagator p;
         if ((st = upload(ctx, dr, r_in + 3 * lo, 3 * m, s)) != GPOP_OK || (st = upload(ctx, dv, v_in + 3 * lo, 3 * m, s)) != GPOP_OK
             || (st = begin(ctx, p, start, h, steps, m, dr.as<double>(), dv.as<double>(), s)) != GPOP_OK
@@ -464,10 +483,10 @@ gpop_status gpop_propagate_vjp(gpop_ctx* ctx, const gpop_time* start, double h, 
         return GPOP_OK;
     }
     cudaStream_t s = nullptr;
-    ScopedBufs B;
+    ScopedBufs B(ctx);
     DevBuf &dr = B.b[0], &dv = B.b[1], &dr0 = B.b[2], &dv0 = B.b[3], &ck = B.b[4], &traj = B.b[5],
            &dobj = B.b[6], &dstep = B.b[7], &dseed = B.b[8], &dgrad = B.b[9];
-    StartupTangents tan;
+    StartupTangents tan(ctx);
     if ((st = upload(ctx, dr, r_in, 3 * n, s)) != GPOP_OK || (st = upload(ctx, dv, v_in, 3 * n, s)) != GPOP_OK
         || (st = upload(ctx, dr0, r_in, 3 * n, s)) != GPOP_OK || (st = upload(ctx, dv0, v_in, 3 * n, s)) != GPOP_OK)
         return st;
@@ -535,8 +554,8 @@ gpop_status gpop_miss_gradient(gpop_ctx* ctx, const gpop_time* start, double h, 
     }
     const size_t traj_bytes = (size_t)steps * 3 * n * sizeof(double);
     cudaStream_t s = nullptr;
-    ScopedBufs B;
-    StartupTangents tan;
+    ScopedBufs B(ctx);
+    StartupTangents tan(ctx);
     DevBuf &dr = B.b[0], &dv = B.b[1], &dr0 = B.b[2], &dv0 = B.b[3], &ck = B.b[4],
            &traj = B.b[6], &dpairs = B.b[7], &units = B.b[8], &dseed = B.b[9], &out = B.b[10],
            &dgrad = B.b[11];

@@ -264,6 +264,8 @@ gpop_status gpop_create(const gpop_config* cfg_in, gpop_ctx** out)
     gpop_ctx* ctx = new (std::nothrow) gpop_ctx();
     if (!ctx)
         return GPOP_ERR_NOMEM;
+    for (DevBuf* b : { &ctx->state, &ctx->gen_m, &ctx->prop_m, &ctx->io_r, &ctx->io_v })
+        b->use(ctx->pool, false); // used on callers' streams: frees the pool when memory runs out, keeps nothing there
     ctx->cfg = cfg;
     ctx->data_dir = cfg.data_dir;
     ctx->cfg.data_dir = ctx->data_dir.c_str();
@@ -369,6 +371,7 @@ void gpop_destroy(gpop_ctx* ctx)
              &ctx->state, &ctx->gen_m, &ctx->prop_m, &ctx->gen_sec, &ctx->prop_sec, &ctx->io_r,
              &ctx->io_v })
         b->release();
+    ctx->pool->trim(true);
     delete ctx;
 }
 
@@ -442,6 +445,8 @@ gpop_status gpop_propagator_create(gpop_ctx* ctx, const gpop_time* start, double
     p->r = r_dev;
     p->v = v_dev;
     p->mixed = ctx->cfg.precision == GPOP_MIXED;
+    for (DevBuf* b : { &p->own_state, &p->own_gen, &p->own_prop })
+        b->use(ctx->pool, false);
     gpop_status st = propagator_init(p, nullptr);
     if (st != GPOP_OK) {
         delete p;

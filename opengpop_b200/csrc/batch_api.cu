@@ -390,6 +390,8 @@ static gpop_status run_batch(gpop_ctx* ctx, const gpop_request* reqs, int32_t n_
     BatchCache* bc = ctx->batch;
     if (!bc)
         return fail(ctx, GPOP_ERR_NOMEM, "batch cache");
+    for (DevBuf* b : { &bc->state, &bc->io, &bc->tables })
+        b->use(ctx->pool, false);
     const bool replay = bc->exec && bc->sig == sig;
     cudaStream_t s = ctx->batch_stream;
     if (!s && (e = cudaStreamCreateWithFlags(&ctx->batch_stream, cudaStreamNonBlocking)) != cudaSuccess)

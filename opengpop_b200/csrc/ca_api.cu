@@ -40,11 +40,15 @@ struct gpop_ca {
     // cumulative device time (s) of propagation, screen and refinement (CUDA events)
     double t_prop = 0, t_screen = 0, t_refine = 0;
 
-    ~gpop_ca()
+    template <class F> void each_buffer(F f)
     {
         for (DevBuf* b : { &r, &v, &bound, &base, &tiles, &min_d2, &min_step, &so, &nh, &mo, &traj_r,
                  &traj_v, &traj_a, &dist, &time, &pos_a, &pos_b, &cand, &count, &state, &gen_m, &prop_m })
-            b->release();
+            f(*b);
+    }
+    ~gpop_ca()
+    {
+        each_buffer([](DevBuf& b) { b.release(); });
     }
 };
 
@@ -175,6 +179,8 @@ cudaError_t resize_store(gpop_ca* ca, int cap)
 {
     const size_t row = (size_t)ca->n * 3 * sizeof(double);
     DevBuf nr, nv, na;
+    for (DevBuf* b : { &nr, &nv, &na })
+        b->use(ca->ctx->pool, true);
     cudaError_t e;
     if ((e = nr.ensure(row * cap)) == cudaSuccess && (e = nv.ensure(row * cap)) == cudaSuccess
         && (e = na.ensure(row * cap)) == cudaSuccess && ca->total_steps > 0) {
@@ -271,6 +277,7 @@ gpop_status gpop_ca_create(gpop_ctx* ctx, const gpop_time* start, double h, int6
     if (!ca)
         return fail(ctx, GPOP_ERR_NOMEM, "closest approach");
     ca->ctx = ctx;
+    ca->each_buffer([&](DevBuf& b) { b.use(ctx->pool, true); });
     ca->start = *start;
     ca->h = h;
     ca->n = n;
@@ -570,6 +577,8 @@ gpop_status gpop_ca_find(gpop_ca* ca, double threshold, gpop_ca_record* out, int
     if (k == 0)
         return GPOP_OK;
     DevBuf d_idx, d_rec;
+    d_idx.use(ctx->pool, true);
+    d_rec.use(ctx->pool, true);
     if ((e = d_idx.ensure(k * 8)) != cudaSuccess || (e = d_rec.ensure(k * 64)) != cudaSuccess) {
         d_idx.release();
         d_rec.release();
