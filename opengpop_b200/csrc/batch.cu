@@ -14,6 +14,7 @@
 #include "gj8_tables.cuh"
 #include "lanes.cuh"
 #include "startup.cuh"
+#include "team.cuh"
 
 #include <type_traits>
 
@@ -259,6 +260,44 @@ __global__ void __launch_bounds__(256, 1) batch_gj8_kernel(TableSrc ts, BatchArg
     }
 }
 
+// Objects of the longest requests, each by a team of warps with a lane per column (team.cuh) on SMs of their own:
+// a request's steps follow one another, so the longest one bounds the batch. 24 objects x 7,780 steps at 70x70,
+// 256 requests of one to 512 objects: 72 of 81 ms on warps of the persistent kernel (9.3 us per step), 38 here, the
+// call 57 with the other requests on more lanes. FP64 in mixed precision too: it is the faster one there.
+__global__ void __launch_bounds__(kTeamBlock, 1) batch_team_kernel(TableSrc ts, BatchArgs a, int P)
+{
+    extern __shared__ __align__(128) uint8_t smem[];
+    GravSmem g;
+    if (!bind_lane_table(smem, ts, a.err, g))
+        return;
+    double* hist = reinterpret_cast<double*>(smem + stage_offset(ts))
+        + (size_t)(threadIdx.x / P) * team_doubles(P, true);
+    int* item = reinterpret_cast<int*>(hist + team_doubles(P, true) - 1);
+    const auto team = make_team<true>(P, hist + 27);
+    for (;;) {
+        if (team.l == 0)
+            *item = atomicAdd(a.next_item + 1, 1);
+        team.sync();
+        const int i = *item;
+        team.sync(); // read by all before the next one is fetched
+        if (i >= a.n_team)
+            break;
+        const BatchItem it = a.team_items[i];
+        const BatchReq rq = a.reqs[it.req];
+        g.L = rq.L;
+        PropArgs p;
+        p.n = a.n_obj;
+        p.state = a.state;
+        p.h = rq.h;
+        p.ncorr = a.ncorr;
+        p.prop_m = rq.prop_m;
+        p.step_end = rq.steps + 1;
+        p.out_r = a.r_out;
+        p.out_v = a.v_out;
+        team_steps<false, true>(ts, g, p, team, rq.obj0 + it.first, P, hist, 0xffffffffu);
+    }
+}
+
 template <class K> static cudaError_t set_smem(K kernel, size_t bytes)
 {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
@@ -315,6 +354,17 @@ cudaError_t launch_batch_gj8(const TableSrc& lane_ts, const TableSrc& plain_ts, 
         return cudaSuccess;
     return lane_ts.mixed ? launch_batch_gj8_m<true>(lane_ts, plain_ts, a, blocks, block, s)
                          : launch_batch_gj8_m<false>(lane_ts, plain_ts, a, blocks, block, s);
+}
+
+cudaError_t launch_batch_teams(const TableSrc& lane64, const BatchArgs& a, int blocks, int teams, int lanes,
+    cudaStream_t s)
+{
+    const size_t bytes = stage_offset(lane64) + (size_t)teams * team_doubles(lanes, true) * sizeof(double);
+    cudaError_t e = set_smem(batch_team_kernel, bytes);
+    if (e != cudaSuccess)
+        return e;
+    batch_team_kernel<<<blocks, teams * lanes, bytes, s>>>(lane64, a, lanes);
+    return cudaGetLastError();
 }
 
 // ---- epoch tables of many requests: epoch e uses calendar cal[5 * epoch_req[e]] ----

@@ -35,7 +35,9 @@ struct BatchArgs {
     int n_req = 0;
     const BatchItem* items = nullptr;
     int n_items = 0;
-    int* next_item = nullptr; // work-queue head (zeroed before the launch)
+    int* next_item = nullptr; // work-queue heads, of items and of team items (zeroed before the launch)
+    const BatchItem* team_items = nullptr; // single objects of the longest requests (batch_team_kernel)
+    int n_team = 0;
     const int* obj_req = nullptr; // request of each flattened object (startup)
     int64_t n_obj = 0;
     int ncorr = 7;
@@ -57,6 +59,9 @@ cudaError_t launch_batch_startup(const TableSrc& lane_ts, const TableSrc& plain_
 // block.
 cudaError_t launch_batch_gj8(const TableSrc& lane_ts, const TableSrc& plain_ts, const BatchArgs& a,
     int blocks, int block, cudaStream_t s);
+// The team items, on `blocks` blocks of `teams` teams of `lanes` lanes. lane64: the FP64 lane-layout table.
+cudaError_t launch_batch_teams(const TableSrc& lane64, const BatchArgs& a, int blocks, int teams, int lanes,
+    cudaStream_t s);
 cudaError_t launch_frames_batch(const FrameData& fd, const int* cal, const int* epoch_req,
     const double* sec_args, int count, double* m_out, cudaStream_t s);
 

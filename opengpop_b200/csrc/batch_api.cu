@@ -21,6 +21,7 @@ namespace {
 // the two-object path needs the registers of 8 warps at most.
 constexpr int kWarpOptions[2] = { 4, 8 };
 inline int warp_index(int W) { return W == kWarpOptions[0] ? 0 : 1; }
+constexpr int kBatchTeamThreads = 256; // largest block of batch_team_kernel
 constexpr int kDegrees[4] = { 8, 20, 36, 70 };
 const double kNodesH[10] = { 0.0, 4.0 / 27.0, 2.0 / 9.0, 1.0 / 3.0, 1.0 / 2.0, 2.0 / 3.0, 1.0 / 6.0, 1.0, 5.0 / 6.0, 1.0 };
 
@@ -48,7 +49,7 @@ double eta(const gpop_ctx* ctx, int W, int L, int P)
         return 1.0 / (c0 + f * (c1 - c0));
     }
     const bool mixed = ctx->cfg.precision == GPOP_MIXED;
-    const double base70 = mixed ? 6.5e5 : 4.5e5; // object-steps/s per SM at 70x70, one lane
+    const double base70 = mixed ? 2.8e6 : 1.4e6; // object-steps/s per SM at 70x70, one lane
     const double cost = (terms(std::max(L, 2)) + 60.0) / (terms(70) + 60.0);
     return base70 / cost / (1.0 + 0.12 * lp) * (wi == 0 ? 0.75 : 1.0);
 }
@@ -83,7 +84,9 @@ inline double lpt_makespan(std::vector<std::pair<double, int64_t>>& groups, doub
 // Then every request whose work item outlasts the makespan bound -- the larger of the average warp
 // load and the shortest possible item of the longest request -- doubles its lanes while that
 // shortens the item -- except that a batch whose items fit one wave of warps keeps them in one
-// wave (lanes cost efficiency; a second wave of split items costs more). Measured on B200:
+// wave (lanes cost efficiency; a second wave of split items costs more); the longest items take its
+// places first (in the order of the requests, a 36x36 request ahead of a longer 70x70 one took them: 256
+// requests without their longest 460 ms, longest first 47). Measured on B200:
 // 4,096 uneven requests 8.7 s; one 65,536-object request at 70x70 keeps one lane per object
 // (136 M object-steps/s with the two-column walk on the plain table; 75 M with two lanes per
 // object and the one-column walk).
@@ -114,15 +117,23 @@ double choose_lanes(const std::vector<int64_t>& n, const std::vector<int>& steps
                 }
             const double bound = std::max(total / warps, crit);
             bool changed = false;
+            // the longest items first: they come before the others for the wave's places
+            std::priority_queue<std::pair<double, size_t>> longest;
             for (size_t r = 0; r < R; ++r)
-                while (steps[r] > 0 && lpo[r] < 32 && item_time(r, lpo[r]) > bound
-                    && item_time(r, 2 * lpo[r]) < item_time(r, lpo[r])
+                if (steps[r] > 0)
+                    longest.push({ item_time(r, lpo[r]), r });
+            while (!longest.empty() && longest.top().first > bound) {
+                const size_t r = longest.top().second;
+                longest.pop();
+                if (lpo[r] < 32 && item_time(r, 2 * lpo[r]) < item_time(r, lpo[r])
                     && (count > (int64_t)warps
                         || count - items_of(r, lpo[r]) + items_of(r, 2 * lpo[r]) <= (int64_t)warps)) {
                     count += items_of(r, 2 * lpo[r]) - items_of(r, lpo[r]);
                     lpo[r] *= 2;
                     changed = true;
+                    longest.push({ item_time(r, lpo[r]), r });
                 }
+            }
             if (!changed)
                 break;
         }
@@ -163,6 +174,8 @@ struct Plan {
     std::vector<BatchItem> items;
     double est = 0.0;
     int warps_per_sm = 8; // block shape of the persistent grid
+    std::vector<BatchItem> team_items; // objects that teams take (choose_teams)
+    int team_blocks = 0, teams_per_block = 0, team_lanes = 0;
 };
 
 // The plan: for each block shape (warps per SM), lanes per object and the simulated makespan with
@@ -208,6 +221,85 @@ Plan make_plan(const gpop_ctx* ctx, const std::vector<int64_t>& n, const std::ve
     for (auto& it : items)
         p.items.push_back(it.second);
     return p;
+}
+
+// Seconds per step of one object on a team with a lane per column (B200, FP64, one team per SM: 20x20 3.9 us, 36
+// 4.7, 50 5.4, 70 6.4; two per SM: 70 7.9), and of a work item on one warp with P lanes per object (70x70: 9.3
+// to 11 us with 32 lanes, 17 with 8, 91 with one; 20x20: 4.7 with 32, 13.6 with one).
+double team_step(int L, int teams_per_block) { return (L < 14 ? 2.1e-6 : 2.9e-6 + 5e-8 * L) * (teams_per_block > 1 ? 1.2 : 1.0); }
+double warp_step(int L, int P) { return 1.25 * team_step(L, 1) + 3.6e-8 * terms(std::max(L, 2)) / P * (P == 1 ? 1.5 : 1.0); }
+
+// Moves the objects of the longest requests from the items to teams while that shortens the batch. A request's
+// steps follow one another: in a batch with a few requests much longer than the mean load of a warp, these bound
+// it (256 requests, 24 objects x 7,780 steps at 70x70: 72 of 77 ms). Taken: the requests whose items last longest,
+// as long as the longest team, the longest item left and the load on the SMs left to the items together get
+// shorter by a tenth; up to one team per SM on a quarter of the SMs, then two on up to half.
+void choose_teams(const gpop_ctx* ctx, const std::vector<int64_t>& n, const std::vector<int>& steps,
+    const std::vector<int>& L, Plan& p)
+{
+    if (ctx->force_lpo > 0
+        || stage_offset(ctx->lane_table(false)) + kBatchTeamThreads * sizeof(double) > max_smem_optin())
+        return; // (a team needs less than a double per lane beside the table)
+    const size_t R = n.size();
+    std::vector<size_t> order;
+    double load = 0.0; // warp-seconds of the items
+    std::vector<double> req_load(R, 0.0);
+    for (size_t r = 0; r < R; ++r) {
+        if (steps[r] <= 0)
+            continue;
+        const int per = batch_item_objects(p.lpo[r]);
+        req_load[r] = (double)((n[r] + per - 1) / per) * steps[r] * p.warps_per_sm * per
+            / eta(ctx, p.warps_per_sm, L[r], p.lpo[r]);
+        load += req_load[r];
+        order.push_back(r);
+    }
+    std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t b) {
+        return steps[a] * warp_step(L[a], p.lpo[a]) > steps[b] * warp_step(L[b], p.lpo[b]);
+    });
+    auto span = [&](double team, size_t next, double items, int blocks) {
+        const double longest = next < order.size() ? steps[order[next]] * warp_step(L[order[next]], p.lpo[order[next]]) : 0.0;
+        return std::max(std::max(team, longest), items / ((double)p.warps_per_sm * (ctx->num_sms - blocks)));
+    };
+    double best = 0.9 * span(0.0, 0, load, 0);
+    size_t take = 0;
+    int64_t objects = 0;
+    int Lmax = 0;
+    for (size_t k = 0; k < order.size(); ++k) {
+        const size_t r = order[k];
+        objects += n[r];
+        if (objects > ctx->num_sms)
+            break;
+        load -= req_load[r];
+        Lmax = std::max(Lmax, L[r]);
+        const int lanes = (Lmax + 32) / 32 * 32, teams = objects > ctx->num_sms / 4 ? 2 : 1;
+        if (lanes * teams > kBatchTeamThreads)
+            break;
+        double team = 0.0;
+        for (size_t i = 0; i <= k; ++i)
+            team = std::max(team, steps[order[i]] * team_step(L[order[i]], teams));
+        const int blocks = (int)((objects + teams - 1) / teams);
+        const double t = span(team, k + 1, load, blocks);
+        if (t < best) {
+            best = t;
+            take = k + 1;
+            p.team_blocks = blocks;
+            p.teams_per_block = teams;
+            p.team_lanes = lanes;
+        }
+    }
+    if (take == 0)
+        return;
+    std::vector<int> rest = steps;
+    for (size_t k = 0; k < take; ++k) {
+        rest[order[k]] = 0;
+        for (int64_t i = 0; i < n[order[k]]; ++i)
+            p.team_items.push_back(BatchItem { (int)order[k], (int)i, 1 });
+    }
+    // the others by themselves: lanes for what is the longest now
+    Plan q = make_plan(ctx, n, rest, L);
+    p.lpo = q.lpo;
+    p.items = q.items;
+    p.warps_per_sm = q.warps_per_sm;
 }
 
 struct TableKey {
@@ -272,6 +364,14 @@ void destroy_batch_cache(gpop_ctx* ctx)
     if (ctx->batch_stream)
         cudaStreamDestroy(ctx->batch_stream);
     ctx->batch_stream = nullptr;
+    if (ctx->batch_side)
+        cudaStreamDestroy(ctx->batch_side);
+    ctx->batch_side = nullptr;
+    for (cudaEvent_t& ev : ctx->batch_event) {
+        if (ev)
+            cudaEventDestroy(ev);
+        ev = nullptr;
+    }
     if (ctx->batch_host)
         cudaFreeHost(ctx->batch_host);
     ctx->batch_host = nullptr;
@@ -305,6 +405,24 @@ gpop_status gpop_batch_plan(gpop_ctx* ctx, const gpop_request* reqs, int32_t n_r
 }
 
 } // extern "C"
+
+// The team launch on a second captured stream, and its end. Events and stream live as long as the context.
+static cudaError_t fork_teams(gpop_ctx* ctx, const BatchArgs& a, const Plan& plan, cudaStream_t s)
+{
+    cudaError_t e = cudaEventRecord(ctx->batch_event[0], s);
+    if (e == cudaSuccess)
+        e = cudaStreamWaitEvent(ctx->batch_side, ctx->batch_event[0], 0);
+    if (e == cudaSuccess)
+        e = launch_batch_teams(ctx->lane_table(false), a, plan.team_blocks, plan.teams_per_block, plan.team_lanes,
+            ctx->batch_side);
+    return e;
+}
+
+static cudaError_t join_teams(gpop_ctx* ctx, cudaStream_t s)
+{
+    const cudaError_t e = cudaEventRecord(ctx->batch_event[1], ctx->batch_side);
+    return e == cudaSuccess ? cudaStreamWaitEvent(s, ctx->batch_event[1], 0) : e;
+}
 
 // The batch proper, over requests that have passed request_problem.
 static gpop_status run_batch(gpop_ctx* ctx, const gpop_request* reqs, int32_t n_req)
@@ -352,6 +470,7 @@ static gpop_status run_batch(gpop_ctx* ctx, const gpop_request* reqs, int32_t n_
     if (N == 0)
         return GPOP_OK;
     Plan plan = make_plan(ctx, n, steps, L);
+    choose_teams(ctx, n, steps, L, plan);
     ctx->batch_warps = plan.warps_per_sm;
     // epoch table offsets (in matrices): [gen 80 | prop len] per table
     std::vector<int64_t> t_off(tables.size());
@@ -397,6 +516,11 @@ static gpop_status run_batch(gpop_ctx* ctx, const gpop_request* reqs, int32_t n_
     if (!s && (e = cudaStreamCreateWithFlags(&ctx->batch_stream, cudaStreamNonBlocking)) != cudaSuccess)
         return cuda_fail(ctx, e, "batch stream");
     s = ctx->batch_stream;
+    if (!ctx->batch_side && (e = cudaStreamCreateWithFlags(&ctx->batch_side, cudaStreamNonBlocking)) != cudaSuccess)
+        return cuda_fail(ctx, e, "batch stream");
+    for (cudaEvent_t& ev : ctx->batch_event)
+        if (!ev && (e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess)
+            return cuda_fail(ctx, e, "batch event");
     // ---- inputs: one pinned staging buffer [r0 | v0 | r_out | v_out] ----
     const size_t io_bytes = (size_t)N * 3 * 4 * sizeof(double);
     if ((e = bc->io.ensure(io_bytes)) != cudaSuccess)
@@ -435,10 +559,10 @@ static gpop_status run_batch(gpop_ctx* ctx, const gpop_request* reqs, int32_t n_
             || (e = bc->epoch_req.ensure((size_t)E * sizeof(int))) != cudaSuccess
             || (e = bc->cal.ensure(cal.size() * sizeof(int) + 4)) != cudaSuccess
             || (e = bc->reqs.ensure(n_req * sizeof(BatchReq))) != cudaSuccess
-            || (e = bc->items.ensure(std::max<size_t>(1, plan.items.size()) * sizeof(BatchItem))) != cudaSuccess
+            || (e = bc->items.ensure((plan.items.size() + plan.team_items.size()) * sizeof(BatchItem))) != cudaSuccess
             || (e = bc->obj_req.ensure((size_t)N * sizeof(int))) != cudaSuccess
             || (e = bc->state.ensure(state_bytes(N))) != cudaSuccess
-            || (e = bc->queue.ensure(sizeof(int))) != cudaSuccess)
+            || (e = bc->queue.ensure(2 * sizeof(int))) != cudaSuccess)
             return fail(ctx, GPOP_ERR_NOMEM, std::string("batch buffers: ") + cudaGetErrorString(e));
         for (size_t t = 0; t < tables.size(); ++t) {
             const TableKey& k = tables[t];
@@ -486,6 +610,9 @@ static gpop_status run_batch(gpop_ctx* ctx, const gpop_request* reqs, int32_t n_
             || (e = cudaMemcpyAsync(bc->items.p, plan.items.data(), plan.items.size() * sizeof(BatchItem),
                     cudaMemcpyHostToDevice, s))
                 != cudaSuccess
+            || (e = cudaMemcpyAsync(bc->items.as<BatchItem>() + plan.items.size(), plan.team_items.data(),
+                    plan.team_items.size() * sizeof(BatchItem), cudaMemcpyHostToDevice, s))
+                != cudaSuccess
             || (e = cudaMemcpyAsync(bc->obj_req.p, obj_req.data(), N * sizeof(int), cudaMemcpyHostToDevice, s))
                 != cudaSuccess
             || (e = cudaStreamSynchronize(s)) != cudaSuccess) // the host vectors go out of scope
@@ -498,6 +625,8 @@ static gpop_status run_batch(gpop_ctx* ctx, const gpop_request* reqs, int32_t n_
         a.items = bc->items.as<BatchItem>();
         a.n_items = (int)plan.items.size();
         a.next_item = bc->queue.as<int>();
+        a.team_items = a.items + plan.items.size();
+        a.n_team = (int)plan.team_items.size();
         a.obj_req = bc->obj_req.as<int>();
         a.n_obj = N;
         a.ncorr = ctx->cfg.n_corrections;
@@ -518,10 +647,16 @@ static gpop_status run_batch(gpop_ctx* ctx, const gpop_request* reqs, int32_t n_
         if (le == cudaSuccess)
             le = launch_batch_startup(ctx->lane_table(mixed), ctx->table(mixed), a, ctx->num_sms, s);
         if (le == cudaSuccess)
-            le = cudaMemsetAsync(bc->queue.p, 0, sizeof(int), s);
+            le = cudaMemsetAsync(bc->queue.p, 0, 2 * sizeof(int), s);
+        if (le == cudaSuccess && a.n_team > 0) // the teams beside the items, on blocks of their own
+            le = fork_teams(ctx, a, plan, s);
         if (le == cudaSuccess)
-            le = launch_batch_gj8(ctx->lane_table(mixed), ctx->table(mixed), a, ctx->num_sms,
+            le = launch_batch_gj8(ctx->lane_table(mixed), ctx->table(mixed), a, ctx->num_sms - plan.team_blocks,
                 32 * plan.warps_per_sm, s);
+        if (a.n_team > 0) {
+            const cudaError_t j = join_teams(ctx, s);
+            le = le == cudaSuccess ? j : le;
+        }
         e = cudaStreamEndCapture(s, &graph);
         if (le != cudaSuccess || e != cudaSuccess) {
             if (graph)
@@ -540,7 +675,8 @@ static gpop_status run_batch(gpop_ctx* ctx, const gpop_request* reqs, int32_t n_
     timer.mark(s);
     if ((e = cudaGraphLaunch(bc->exec, s)) != cudaSuccess)
         return cuda_fail(ctx, e, "batch graph launch");
-    ctx->launches += 2 + startup_launches(ctx->cfg.n_corrections);
+    ctx->launches += 1 + startup_launches(ctx->cfg.n_corrections) + (plan.items.empty() ? 0 : 1)
+        + (plan.team_items.empty() ? 0 : 1);
     timer.mark(s);
     if ((e = cudaMemcpyAsync(host + 6 * N, dio + 6 * N, (size_t)N * 6 * sizeof(double), cudaMemcpyDeviceToHost, s))
         != cudaSuccess)

@@ -187,7 +187,8 @@ struct gpop_ctx {
     std::shared_ptr<gpop::DevPool> pool = std::make_shared<gpop::DevPool>();
     // batched propagation: cached plan and graph, its stream and pinned staging buffer
     BatchCache* batch = nullptr;
-    cudaStream_t batch_stream = nullptr;
+    cudaStream_t batch_stream = nullptr, batch_side = nullptr;
+    cudaEvent_t batch_event[2] = {};
     void* batch_host = nullptr;
     size_t batch_host_cap = 0;
     // batched-kernel throughput (object-steps/s per SM) for the persistent grid's block shapes

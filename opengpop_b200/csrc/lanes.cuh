@@ -159,6 +159,7 @@ __device__ __forceinline__ void lane_sum4(double& a, double& b, double& c, doubl
 struct WarpTeam {
     int l, P;
     unsigned mask;
+    __device__ __forceinline__ int top() const { return P - 2; } // LanePowers
     __device__ __forceinline__ void sum4(double& a, double& b, double& c, double& d) const
     {
         lane_sum4(a, b, c, d, l, P, mask);
@@ -174,6 +175,7 @@ struct BlockTeam {
     int l, P, warps, bar;
     double* buf;
     mutable int half;
+    __device__ __forceinline__ int top() const { return (l | 31) - 1; } // of the warp: the first has the longest columns
     __device__ __forceinline__ void sync() const
     {
         asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(P) : "memory");
@@ -414,7 +416,7 @@ __device__ __forceinline__ void gravity_itrs_team(const GravSmem& gs, const Team
         u[k] = q * (z[k] * ri[k]);
         w[k] = q * q;
         G[k] = H[k] = J[k] = KK[k] = 0.0;
-        lp[k] = lane_powers(x[k] * ri[k], y[k] * ri[k], q, team.l, team.P - 2, team.P, team.P <= gs.L);
+        lp[k] = lane_powers(x[k] * ri[k], y[k] * ri[k], q, team.l, team.top(), team.P, team.P <= gs.L);
     }
     lane_walk<MIXED, K, PAIRS>(gs, team.l, team.P, gs.L, lp, u, w, G, H, J, KK);
 #pragma unroll
@@ -432,27 +434,11 @@ __device__ __forceinline__ void gravity_itrs_lk(const GravSmem& gs, int l, int P
     gravity_itrs_team<MIXED, K, PAIRS>(gs, WarpTeam { l, P, mask }, x, y, z, ax, ay, az);
 }
 
-template <bool MIXED>
-__device__ __forceinline__ void gravity_itrs_lanes(const GravSmem& gs, int l, int P, double x,
-    double y, double z, double& ax, double& ay, double& az, unsigned mask = 0xffffffffu)
-{
-    const double X[1] = { x }, Y[1] = { y }, Z[1] = { z };
-    double AX[1], AY[1], AZ[1];
-    gravity_itrs_lk<MIXED, 1>(gs, l, P, X, Y, Z, AX, AY, AZ, mask);
-    ax = AX[0];
-    ay = AY[0];
-    az = AZ[0];
-}
-
 // K objects: GCRS positions r[k] with the ITRS<-GCRS matrix M of gravity_gcrs.
 template <bool MIXED, int K, bool PAIRS = false, class Team = WarpTeam>
-__device__ __forceinline__ void gravity_gcrs_team(const GravSmem& gs, const Team& team,
-    const double* __restrict__ M, const double (&r)[K][3], double (&a)[K][3])
+__device__ __forceinline__ void gravity_gcrs_team(const GravSmem& gs, const Team& team, const double (&m)[9],
+    const double (&r)[K][3], double (&a)[K][3])
 {
-    double m[9];
-#pragma unroll
-    for (int i = 0; i < 9; ++i)
-        m[i] = __ldg(M + i);
     double px[K], py[K], pz[K], ax[K], ay[K], az[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) {
@@ -469,29 +455,22 @@ __device__ __forceinline__ void gravity_gcrs_team(const GravSmem& gs, const Team
     }
 }
 
-template <bool MIXED, int K, bool PAIRS = false>
-__device__ __forceinline__ void gravity_gcrs_lk(const GravSmem& gs, int l, int P, const double* __restrict__ M,
-    const double (&r)[K][3], double (&a)[K][3], unsigned mask)
-{
-    gravity_gcrs_team<MIXED, K, PAIRS>(gs, WarpTeam { l, P, mask }, M, r, a);
-}
-
-template <bool MIXED>
-__device__ __forceinline__ void gravity_gcrs_lanes(const GravSmem& gs, int l, int P,
-    const double* __restrict__ M, const double* r, double* a, unsigned mask = 0xffffffffu)
+template <bool MIXED, int K, bool PAIRS = false, class Team = WarpTeam>
+__device__ __forceinline__ void gravity_gcrs_team(const GravSmem& gs, const Team& team,
+    const double* __restrict__ M, const double (&r)[K][3], double (&a)[K][3])
 {
     double m[9];
 #pragma unroll
     for (int i = 0; i < 9; ++i)
         m[i] = __ldg(M + i);
-    const double px = m[0] * r[0] + m[1] * r[1] + m[2] * r[2];
-    const double py = m[3] * r[0] + m[4] * r[1] + m[5] * r[2];
-    const double pz = m[6] * r[0] + m[7] * r[1] + m[8] * r[2];
-    double ax, ay, az;
-    gravity_itrs_lanes<MIXED>(gs, l, P, px, py, pz, ax, ay, az, mask);
-    a[0] = m[0] * ax + m[3] * ay + m[6] * az;
-    a[1] = m[1] * ax + m[4] * ay + m[7] * az;
-    a[2] = m[2] * ax + m[5] * ay + m[8] * az;
+    gravity_gcrs_team<MIXED, K, PAIRS>(gs, team, m, r, a);
+}
+
+template <bool MIXED, int K, bool PAIRS = false>
+__device__ __forceinline__ void gravity_gcrs_lk(const GravSmem& gs, int l, int P, const double* __restrict__ M,
+    const double (&r)[K][3], double (&a)[K][3], unsigned mask)
+{
+    gravity_gcrs_team<MIXED, K, PAIRS>(gs, WarpTeam { l, P, mask }, M, r, a);
 }
 
 } // namespace gpop

@@ -9,6 +9,7 @@
 #include "gj8_tables.cuh"
 #include "integrator.cuh"
 #include "lanes.cuh"
+#include "team.cuh"
 #include "kernels.h"
 #include "startup.cuh"
 
@@ -104,7 +105,6 @@ struct ForceAnalytic {
     }
 };
 
-constexpr int kTeamBlock = 256; // largest block of gj8_team_kernel
 constexpr int kLanesBlock = 384; // threads per SM the lane walks are spread to
 
 // ---- table staging ----
@@ -645,14 +645,7 @@ __global__ void __launch_bounds__(K == 1 ? kOneObjectBlock : 256, 1) gj8_kernel(
     }
 }
 
-// ---- GJ8 step with a group of lanes per object (few objects) ----
-// Same step as gj8_kernel; the lanes of an object's group split its gravity columns (lanes.cuh, lane-layout
-// table) and hold identical state, and lane 0 stores. A group is P lanes of a warp, or (WARPS) whole warps
-// with a lane per column. The acceleration history lies in shared memory for the launch.
-// Bounds: the latency of an evaluation (one chain of FMAs per column, then a sum over the lanes), so what a
-// step needs besides is kept short: history and sums in shared memory, the next step's rotation prefetched.
-// Blocks of at most 256 threads: with 255 registers a step of one object on 32 lanes takes 9.2 us at 70x70
-// (FP64), with the 168 of 384 threads 16.9.
+// ---- GJ8 step with a group of lanes per object (few objects): team.cuh ----
 template <bool MIXED, bool WARPS>
 __global__ void __launch_bounds__(kTeamBlock, 1) gj8_team_kernel(TableSrc ts, PropArgs a, int P)
 {
@@ -660,8 +653,7 @@ __global__ void __launch_bounds__(kTeamBlock, 1) gj8_team_kernel(TableSrc ts, Pr
     GravSmem g;
     if (!bind_lane_table(smem, ts, a.err, g))
         return;
-    const int64_t n = a.n; // the state's stride; this launch runs objects [lo, hi)
-    const int64_t lo = a.obj_lo, hi = a.obj_hi < 0 ? n : a.obj_hi;
+    const int64_t lo = a.obj_lo, hi = a.obj_hi < 0 ? a.n : a.obj_hi; // this launch's objects
     const int in_block = (int)threadIdx.x / P;
     const int64_t obj = lo + (int64_t)blockIdx.x * (blockDim.x / P) + in_block;
     const int in_warp = (int)blockDim.x - (int)(threadIdx.x & ~31u); // the block's last warp may be partial
@@ -670,110 +662,7 @@ __global__ void __launch_bounds__(kTeamBlock, 1) gj8_team_kernel(TableSrc ts, Pr
         return; // whole groups leave: shuffles and barriers name the group only
     // per group: 27 doubles of history [slot][axis], then 8 per warp for the sums of a group of warps
     double* hist = reinterpret_cast<double*>(smem + stage_offset(ts)) + (size_t)in_block * team_doubles(P, WARPS);
-    const auto team = make_team<WARPS>(P, hist + 27);
-    const int l = team.l;
-    const bool lead = l == 0;
-    double* st = a.state + obj;
-    for (int i = l; i < 27; i += P)
-        hist[i] = st[(kHist + i) * n];
-    team.sync();
-    const double h = a.h;
-    double r[1][3], v[3], s[3], S[3];
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-        r[0][j] = st[(kR + j) * n];
-        v[j] = st[(kV + j) * n];
-        s[j] = st[(kSs + j) * n];
-        S[j] = st[(kSb + j) * n];
-    }
-    int ring0 = a.step_begin >= 5 ? (a.step_begin - 5) % 9 : 0;
-    for (int step = a.step_begin; step < a.step_end; ++step) {
-        double a8[1][3];
-        if (step <= 4) {
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                r[0][j] = st[(kRep + (step - 1) * 6 + j) * n];
-                v[j] = st[(kRep + (step - 1) * 6 + 3 + j) * n];
-                a8[0][j] = st[(kRepA + (step - 1) * 3 + j) * n];
-            }
-        } else {
-            const double* M = a.prop_m + (size_t)(step + 4) * 9;
-            if (l < 2 && step + 1 < a.step_end) // the next step's rotation
-                asm volatile("prefetch.global.L1 [%0];" ::"l"(M + 9 + 8 * l));
-            double s1[3], s2[3], prev[3], a7[3];
-#pragma unroll
-            for (int j = 0; j < 3; ++j) { // as gj8_kernel
-                double q[9];
-#pragma unroll
-                for (int c = 0; c < 9; ++c) {
-                    int slot = ring0 + c;
-                    slot -= slot >= 9 ? 9 : 0;
-                    q[c] = hist[slot * 3 + j];
-                }
-                double rt = 0.0, c1 = 0.0, c2 = 0.0;
-#pragma unroll
-                for (int c = 0; c < 9; ++c)
-                    rt = fma(q[c], c_GJ[9][c], rt);
-#pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    c1 = fma(q[c + 1], c_SA[8][c], c1);
-                    c2 = fma(q[c + 1], c_GJ[8][c], c2);
-                }
-                S[j] += s[j] + q[8] / 2;
-                r[0][j] = (rt + S[j]) * h * h;
-                s1[j] = c1;
-                s2[j] = c2;
-                prev[j] = s[j];
-                a7[j] = q[8];
-            }
-            bool fast = false;
-            for (int it = 0; it < a.ncorr; ++it) {
-                gravity_gcrs_team<MIXED, 1, !WARPS>(g, team, M, r, a8);
-                if (correct_position(ts.corr, h, it, a.ncorr, s2, S, a8[0], r[0], fast))
-                    break; // the same for the lanes of a group
-            }
-            if constexpr (!WARPS)
-                __syncwarp(warp); // groups that were done earlier wait: the warp's walks stay converged
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                s[j] = prev[j] + (a8[0][j] + a7[j]) / 2;
-                v[j] = h * (s1[j] + a8[0][j] * c_SA[8][8] + s[j]);
-            }
-            if (lead)
-#pragma unroll
-                for (int j = 0; j < 3; ++j)
-                    hist[ring0 * 3 + j] = a8[0][j];
-            team.sync(); // the ring write precedes the group's loads of the next step
-            ring0 = ring0 == 8 ? 0 : ring0 + 1;
-        }
-        if (lead) {
-            const int64_t t = step - a.traj_step0;
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                if (a.traj_r)
-                    a.traj_r[(t * 3 + j) * n + obj] = r[0][j];
-                if (a.traj_v)
-                    a.traj_v[(t * 3 + j) * n + obj] = v[j];
-                if (a.traj_a)
-                    a.traj_a[(t * 3 + j) * n + obj] = a8[0][j];
-            }
-        }
-    }
-    for (int i = l; i < 27; i += P)
-        st[(kHist + i) * n] = hist[i];
-    if (!lead)
-        return;
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-        st[(kR + j) * n] = r[0][j];
-        st[(kV + j) * n] = v[j];
-        st[(kSs + j) * n] = s[j];
-        st[(kSb + j) * n] = S[j];
-        if (a.out_r)
-            a.out_r[obj * 3 + j] = r[0][j];
-        if (a.out_v)
-            a.out_v[obj * 3 + j] = v[j];
-    }
+    team_steps<MIXED, WARPS>(ts, g, a, make_team<WARPS>(P, hist + 27), obj, P, hist, warp);
 }
 
 // ---- GJ8 step with P lanes per group of two objects ----
