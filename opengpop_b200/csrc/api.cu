@@ -1,6 +1,7 @@
 // api.cu -- C ABI: context life cycle, propagation, force model and integrator entry points.
 #include "common.cuh"
 #include "context.h"
+#include "frames.cuh"
 #include "gpop.h"
 
 #include <algorithm>
@@ -63,14 +64,12 @@ gpop_status build_epoch_tables(gpop_ctx* ctx, const gpop_time* start, double h, 
                 cudaMemcpyHostToDevice, s))
             != cudaSuccess)
         return cuda_fail(ctx, e, "uploading epoch arguments");
-    if ((e = launch_frames(ctx->frames, start->year, start->month, start->day, start->hour, start->min,
-             ctx->gen_sec.as<double>(), 80, gen_m.as<double>(), nullptr, s))
-            != cudaSuccess
-        || (e = launch_frames(ctx->frames, start->year, start->month, start->day, start->hour,
-                start->min, ctx->prop_sec.as<double>(), count, prop_m.as<double>(), nullptr, s))
-            != cudaSuccess)
+    const FrameRange gen_r { ctx->gen_sec.as<double>(), 80, gen_m.as<double>(), nullptr };
+    const FrameRange prop_r { ctx->prop_sec.as<double>(), count, prop_m.as<double>(), nullptr };
+    if ((e = launch_frames(ctx->frames, start->year, start->month, start->day, start->hour, start->min, gen_r, prop_r, s))
+        != cudaSuccess)
         return cuda_fail(ctx, e, "frame kernel");
-    ctx->launches += 2;
+    ctx->launches++;
     // the host vectors die here: wait for the (pageable, hence staged) copies to have been consumed
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess)
         return cuda_fail(ctx, e, "frame kernel");
@@ -318,6 +317,7 @@ gpop_status gpop_create(const gpop_config* cfg_in, gpop_ctx** out)
     nut.insert(nut.end(), ctx->md.lon1.begin(), ctx->md.lon1.end());
     nut.insert(nut.end(), ctx->md.obl0.begin(), ctx->md.obl0.end());
     nut.insert(nut.end(), ctx->md.obl1.begin(), ctx->md.obl1.end());
+    std::transform(nut.begin(), nut.end(), nut.begin(), frames::nutation_radians);
     std::vector<double> leap(ctx->md.leap_mjd);
     leap.insert(leap.end(), ctx->md.leap_val.begin(), ctx->md.leap_val.end());
     if ((e = ctx->t64.ensure(ctx->t64_bytes)) != cudaSuccess
@@ -650,7 +650,7 @@ gpop_status gpop_frame_matrices(gpop_ctx* ctx, const gpop_time* start, double h,
         e = cudaMemcpyAsync(ctx->prop_sec.p, args.data(), count * sizeof(double), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess)
         e = launch_frames(ctx->frames, start->year, start->month, start->day, start->hour, start->min,
-            ctx->prop_sec.as<double>(), count, m_dev, mjd_dev, s);
+            FrameRange { ctx->prop_sec.as<double>(), count, m_dev, mjd_dev }, FrameRange {}, s);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(s);
     if (e != cudaSuccess)

@@ -9,7 +9,7 @@
 #include "batch.cuh"
 #include "common.cuh"
 #include "corrector.cuh"
-#include "frames.cuh"
+#include "frames_block.cuh"
 #include "gravity.cuh"
 #include "gj8_tables.cuh"
 #include "lanes.cuh"
@@ -368,50 +368,12 @@ cudaError_t launch_batch_teams(const TableSrc& lane64, const BatchArgs& a, int b
 }
 
 // ---- epoch tables of many requests: epoch e uses calendar cal[5 * epoch_req[e]] ----
-__device__ __forceinline__ double warp_sum_b(double v)
+__global__ void __launch_bounds__(kFrameThreads) frames_batch_kernel(FrameData fd, const int* __restrict__ cal,
+    const int* __restrict__ epoch_req, const double* __restrict__ sec_args, double* __restrict__ m_out)
 {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-        v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
-__device__ double series_sum_b(const NutTerm* terms, int count, const double* F, int lane)
-{
-    double acc = 0.0;
-    for (int i = lane; i < count; i += 32)
-        acc += frames::nutation_term(terms[i], F);
-    return warp_sum_b(acc);
-}
-
-__global__ void __launch_bounds__(256) frames_batch_kernel(FrameData fd, const int* __restrict__ cal,
-    const int* __restrict__ epoch_req, const double* __restrict__ sec_args, int count,
-    double* __restrict__ m_out)
-{
-    const int e = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    const int lane = threadIdx.x & 31;
-    if (e >= count)
-        return;
+    const int e = (int)blockIdx.x;
     const int* c = cal + 5 * epoch_req[e];
-    const double mjd_utc = frames::calendar_to_mjd(c[0], c[1], c[2], c[3], c[4], sec_args[e]);
-    const EopRec eop = frames::eop_at(fd.eop, fd.n_eop, mjd_utc);
-    const double mjd_ut1 = mjd_utc + eop.ut1 / 86400.0;
-    const double mjd_tt
-        = mjd_utc + (frames::leap_at(fd.leap_mjd, fd.leap_val, fd.n_leap, mjd_utc) + frames::kTtTai) / 86400.0;
-    const double t = (mjd_tt - frames::kMjdJ2000) / 36525.0;
-    double F[14];
-    frames::fundamental_args(t, F);
-    const NutTerm* lon1 = fd.nut + fd.n_lon0;
-    const NutTerm* obl0 = lon1 + fd.n_lon1;
-    const NutTerm* obl1 = obl0 + fd.n_obl0;
-    const double dpsi = series_sum_b(fd.nut, fd.n_lon0, F, lane) + series_sum_b(lon1, fd.n_lon1, F, lane) * t;
-    const double deps = series_sum_b(obl0, fd.n_obl0, F, lane) + series_sum_b(obl1, fd.n_obl1, F, lane) * t;
-    if (lane == 0) {
-        double M[9];
-        frames::assemble(t, F, dpsi, deps, mjd_ut1, mjd_tt, eop, M);
-        for (int k = 0; k < 9; ++k)
-            m_out[(size_t)e * 9 + k] = M[k];
-    }
+    frames_epoch(fd, c[0], c[1], c[2], c[3], c[4], sec_args[e], m_out + (size_t)e * 9, nullptr);
 }
 
 cudaError_t launch_frames_batch(const FrameData& fd, const int* cal, const int* epoch_req,
@@ -419,9 +381,7 @@ cudaError_t launch_frames_batch(const FrameData& fd, const int* cal, const int* 
 {
     if (count <= 0)
         return cudaSuccess;
-    const int threads = 256;
-    const int blocks = (int)(((int64_t)count * 32 + threads - 1) / threads);
-    frames_batch_kernel<<<blocks, threads, 0, s>>>(fd, cal, epoch_req, sec_args, count, m_out);
+    frames_batch_kernel<<<count, kFrameThreads, 0, s>>>(fd, cal, epoch_req, sec_args, m_out);
     return cudaGetLastError();
 }
 

@@ -105,13 +105,24 @@ GPOP_HD void fundamental_args(double t, double* F)
     }
 }
 
-// One nutation term's contribution (eq. 5.35 summand; ref_sys_trans.cu:241-254).
+// One nutation term's contribution (eq. 5.35 summand; ref_sys_trans.cu:241-254), its coefficients in radians
+// (nutation_radians).
 GPOP_HD double nutation_term(const NutTerm& term, const double* F)
 {
     double arg = 0.0;
     for (int k = 13; k >= 0; --k)
         arg += F[k] * (double)term.args[k];
-    return term.sin_uas / kUasToRad * sin(arg) + term.cos_uas / kUasToRad * cos(arg);
+    double s, c;
+    sincos(arg, &s, &c);
+    return term.sin_uas * s + term.cos_uas * c;
+}
+
+// A term with its coefficients in radians instead of microarcseconds: the same quotients, formed once per table.
+inline NutTerm nutation_radians(NutTerm term)
+{
+    term.sin_uas /= kUasToRad;
+    term.cos_uas /= kUasToRad;
+    return term;
 }
 
 // IAU 2006 precession quantities eps_A, gamma-bar, phi-bar, psi-bar (eq. 5.40; :262-291).

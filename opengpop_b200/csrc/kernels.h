@@ -127,7 +127,15 @@ struct FrameData {
     const double* leap_val = nullptr;
     int n_leap = 0;
 };
-cudaError_t launch_frames(const FrameData& fd, int y, int mo, int d, int hh, int mi,
-    const double* sec_args, int count, double* m_out, double* mjd_out, cudaStream_t s);
+// Epochs of one output table: m_out[count][9], mjd_out[count] (may be NULL).
+struct FrameRange {
+    const double* sec_args = nullptr;
+    int count = 0;
+    double* m_out = nullptr;
+    double* mjd_out = nullptr;
+};
+// Two tables of one calendar in one launch (the second may be empty).
+cudaError_t launch_frames(const FrameData& fd, int y, int mo, int d, int hh, int mi, const FrameRange& a,
+    const FrameRange& b, cudaStream_t s);
 
 } // namespace gpop

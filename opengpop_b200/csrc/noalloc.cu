@@ -114,11 +114,9 @@ extern "C" gpop_status gpop_propagate_device_noalloc(gpop_ctx* ctx, const gpop_t
     epoch_args_kernel<<<(count + 255) / 256, 256, 0, s>>>(start->sec, h, count,
         (ctx->cfg.flags & GPOP_FIX_BACKWARD_RK8_EPOCH) != 0, scratch + kOffGenSec, scratch + kOffPropSec);
     if ((e = cudaGetLastError()) != cudaSuccess
-        || (e = launch_frames(ctx->frames, start->year, start->month, start->day, start->hour,
-                start->min, scratch + kOffGenSec, 80, scratch + kOffGen, nullptr, s))
-            != cudaSuccess
-        || (e = launch_frames(ctx->frames, start->year, start->month, start->day, start->hour,
-                start->min, scratch + kOffPropSec, count, scratch + kOffProp, nullptr, s))
+        || (e = launch_frames(ctx->frames, start->year, start->month, start->day, start->hour, start->min,
+                FrameRange { scratch + kOffGenSec, 80, scratch + kOffGen, nullptr },
+                FrameRange { scratch + kOffPropSec, count, scratch + kOffProp, nullptr }, s))
             != cudaSuccess)
         return cuda_fail(ctx, e, "epoch tables");
     const bool mixed = ctx->cfg.precision == GPOP_MIXED;
@@ -152,7 +150,7 @@ extern "C" gpop_status gpop_propagate_device_noalloc(gpop_ctx* ctx, const gpop_t
             != cudaSuccess)
             return cuda_fail(ctx, e, "GJ8 kernel");
     }
-    ctx->launches += 3 + startup_launches(ctx->cfg.n_corrections) + (steps + chunk - 1) / chunk;
+    ctx->launches += 2 + startup_launches(ctx->cfg.n_corrections) + (steps + chunk - 1) / chunk;
     unsigned word = 0;
     if ((e = cudaMemcpyAsync(&word, err, sizeof(unsigned), cudaMemcpyDeviceToHost, s)) != cudaSuccess
         || (e = cudaStreamSynchronize(s)) != cudaSuccess)
