@@ -45,13 +45,17 @@ def terms(L):
     return (L + 1) * (L + 2) // 2 - 3
 
 
+# gravity evaluations of a step: the corrector ends at its fixed point (corrector.cuh)
+EVALUATIONS = 2
+
+
 def flops_per_object_step(L=DEGREE):
-    return 7 * (24 * terms(L) + 15 * L + 60) + 500
+    return EVALUATIONS * (24 * terms(L) + 15 * L + 60) + 500
 
 
 def fp32_flops_per_object_step(L=DEGREE):
     # the mixed build runs the degree > 8 terms in FP32
-    return 7 * 24 * (terms(L) - terms(8))
+    return EVALUATIONS * 24 * (terms(L) - terms(8))
 
 
 # DRAM bytes (read + write) of one mixed GJ8 launch over 65,536 objects (the split block), from an
@@ -513,8 +517,8 @@ def run_adjoint(args, torch, G, dev):
     # one Jacobian and six tangent steps per object-step
     W = 24 * terms(DEGREE) + 15 * DEGREE + 60
     units = 2 * n_pairs
-    f_miss = units * steps * (2 * flops_per_object_step() + w_jac(DEGREE)) + units * 145 * w_jac(DEGREE)
-    f_stm = n_stm * steps * (flops_per_object_step() + w_jac(DEGREE) + 6 * 500) + n_stm * 145 * w_jac(DEGREE)
+    f_miss = units * steps * (flops_per_object_step() + w_jac(DEGREE)) + units * 89 * w_jac(DEGREE)
+    f_stm = n_stm * steps * (flops_per_object_step() + w_jac(DEGREE) + 6 * 500) + n_stm * 89 * w_jac(DEGREE)
     peak64 = _peaks(torch, dev, clocks)[0]
     cpu = None
     if not args.no_cpu_baseline:
