@@ -116,8 +116,9 @@ gpop_status gpop_propagator_step(gpop_propagator* p, int32_t steps, double* traj
     double* traj_a, void* stream);
 /* Steps taken so far. */
 int32_t gpop_propagator_steps_done(const gpop_propagator* p);
-/* No counterpart in the reference. The gravity walk the propagation calls take for n objects on a
- * GPU of num_sms SMs at the given precision: 1 = one object per thread, 2 = two objects per
+/* No counterpart in the reference. The walk without the column split for n objects on a GPU of num_sms
+ * SMs at the given precision, as GPOP_WALK_MODE names the walks (by default a call may take groups of
+ * warps or the columns over a block instead where they are faster): 1 = one object per thread, 2 = two objects per
  * thread, 3 = lanes per object, 4 = lanes per group of two objects (*lanes_out = the lanes for 3
  * and 4, else 1); -1 for invalid arguments. Host arithmetic only, no CUDA call. */
 int32_t gpop_walk_policy(int64_t n, int32_t num_sms, int32_t precision, int32_t* lanes_out);

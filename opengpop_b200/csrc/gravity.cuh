@@ -35,7 +35,8 @@ constexpr int kMixedSplit = 8; // highest degree kept in FP64 in the mixed mode
 // Two objects per thread walk the columns two at a time (two independent recursions per thread
 // hide each other's latency). Measured on B200, 65,536 objects at 70x70, with the corrector state
 // in shared memory: mixed 123.9 -> 139.4 M object-steps/s (pair unroll 4: 137.6, 8: 139.4, 12:
-// 139.0; three columns at a time 130.5, four 121.3), FP64 72.3 -> 73.8 M (pair unroll 2).
+// 139.0; three columns at a time 130.5, four 121.3), FP64 72.3 -> 73.8 M (pair unroll 2;
+// the column walk of few objects runs faster at 4, which all share).
 #ifndef GPOP_COLPAIR_UNROLL
 #define GPOP_COLPAIR_UNROLL 8
 #endif
