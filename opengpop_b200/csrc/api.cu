@@ -283,6 +283,8 @@ gpop_status gpop_create(const gpop_config* cfg_in, gpop_ctx** out)
         ctx->adjoint_store = (size_t)std::max(0L, atol(mb)) << 20;
     if (const char* ws = std::getenv("GPOP_TEST_FIRST_WAIT_SPINS"))
         ctx->first_wait_spins = (uint32_t)std::min(1L << 22, std::max(0L, atol(ws)));
+    if (const char* ww = std::getenv("GPOP_TEST_FIRST_WAIT_WARP"))
+        ctx->first_wait_spins = kWaitOneWarp | (uint32_t)std::min(31L, std::max(0L, atol(ww)));
     cudaError_t e = cudaSetDevice(cfg.device);
     if (e != cudaSuccess)
         return cuda_fail(ctx, e, "cudaSetDevice");

@@ -99,8 +99,7 @@ __global__ void __launch_bounds__(kBlock, 1) gj8_columns_kernel(TableSrc ts, Pro
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ unsigned need[2]; // sets with objects that are not done, for even and odd passes
     GravSmem g;
-    const bool ok = bind_lane_table(smem, ts, a.err, g);
-    if (!__syncthreads_and(ok)) // the block leaves as one: barriers follow
+    if (!bind_lane_table(smem, ts, a.err, g))
         return;
     const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t n = a.n, lo = a.obj_lo, hi = a.obj_hi < 0 ? n : a.obj_hi;

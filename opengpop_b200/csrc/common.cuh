@@ -15,6 +15,10 @@ enum : unsigned {
     kErrTmaUnfinished = 4u, // a staging copy had still not landed when its block gave up and left
 };
 
+// first_spins of stage_to_smem with this bit set: warp (first_spins without it) polls not once, the
+// others as usual (a test setting).
+constexpr uint32_t kWaitOneWarp = 1u << 31;
+
 // ---- bulk-copy (TMA, cp.async.bulk) staging of a read-only table into shared memory ----
 __device__ __forceinline__ uint32_t smem_u32(const void* p)
 {
@@ -23,13 +27,18 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p)
 
 // Copies `bytes` (multiple of 16, both addresses 16-byte aligned) from global to shared memory with
 // one elected thread issuing cp.async.bulk chunks that complete on an mbarrier. Every thread of the
-// block waits with a bounded spin of first_spins polls; when that runs out the block raises
-// kErrTmaTimeout and returns false after a second bounded wait for the copies still in flight
-// (kErrTmaUnfinished if they have not landed by then either: the caller's results are void).
+// block waits with a bounded spin of first_spins polls; a thread whose polls run out raises
+// kErrTmaTimeout and waits a second bounded time for the copies still in flight (kErrTmaUnfinished if
+// they have not landed by then either: the caller's results are void). The copy may land between the
+// last polls of two warps, so the answer is the block's: false in every thread as soon as one gave up.
+// A block that returns on it leaves as one, and no barrier or full-warp exchange behind it waits for
+// threads that have left. Every thread of the block makes the call.
 __device__ __forceinline__ bool stage_to_smem(void* smem_dst, const void* gsrc, uint32_t bytes,
     uint64_t* mbar, unsigned* err_word, uint32_t first_spins)
 {
     const uint32_t bar = smem_u32(mbar);
+    if (first_spins & kWaitOneWarp)
+        first_spins = (threadIdx.x >> 5) == (first_spins & ~kWaitOneWarp) ? 0u : 1u << 22;
     if (threadIdx.x == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -61,9 +70,9 @@ __device__ __forceinline__ bool stage_to_smem(void* smem_dst, const void* gsrc, 
         if (!done)
             __nanosleep(64);
     }
-    if (!done) {
-        if (threadIdx.x == 0)
-            atomicOr(err_word, kErrTmaTimeout);
+    const bool in_time = done != 0;
+    if (!in_time) {
+        atomicOr(err_word, kErrTmaTimeout);
         // give the copies in flight a second bounded window before the block leaves
         for (int it = 0; it < (1 << 22) && !done; ++it) {
             asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n"
@@ -74,11 +83,10 @@ __device__ __forceinline__ bool stage_to_smem(void* smem_dst, const void* gsrc, 
             if (!done)
                 __nanosleep(64);
         }
-        if (!done && threadIdx.x == 0)
+        if (!done)
             atomicOr(err_word, kErrTmaUnfinished);
-        return false;
     }
-    return true;
+    return __syncthreads_and(in_time) != 0;
 }
 
 // Stores and loads of per-thread values parked in shared memory across a long computation. The

@@ -172,7 +172,8 @@ struct gpop_ctx {
     size_t adjoint_store = (size_t)32 << 30;
     int walk_mode = 0; // GJ8 triangle walk (WalkMode; 0 = default)
     // first staging wait of every kernel (TableSrc::wait_spins); GPOP_TEST_FIRST_WAIT_SPINS, a
-    // test setting, lowers it so that a test can watch the wait give up
+    // test setting, lowers it so that a test can watch the wait give up, GPOP_TEST_FIRST_WAIT_WARP for one
+    // warp of each block alone
     uint32_t first_wait_spins = 1u << 22;
     // device-resident model data
     gpop::DevBuf t64, mixed, nut, eop, leap, err_word;

@@ -410,10 +410,7 @@ __global__ void __launch_bounds__(K == 1 ? kOneObjectBlock : 256, 1) gj8_kernel(
         "the split block carries two objects per thread");
     double* stage = nullptr;
     if constexpr (F::kTable) {
-        bool ok = bind_table<F::kMixed>(smem, ts, a.err, f.g);
-        if constexpr (SPLIT != kSplitNone)
-            ok = __syncthreads_and(ok); // the block leaves as one: barriers follow
-        if (!ok)
+        if (!bind_table<F::kMixed>(smem, ts, a.err, f.g))
             return;
         stage = reinterpret_cast<double*>(smem + stage_offset(ts)) + threadIdx.x;
     }
