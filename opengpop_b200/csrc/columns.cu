@@ -314,8 +314,9 @@ __global__ void __launch_bounds__(kBlock, 1) gj8_columns_kernel(TableSrc ts, Pro
                     const double x = __ldg(M + 0) * r[0] + __ldg(M + 1) * r[1] + __ldg(M + 2) * r[2];
                     const double y = __ldg(M + 3) * r[0] + __ldg(M + 4) * r[1] + __ldg(M + 5) * r[2];
                     const double z = __ldg(M + 6) * r[0] + __ldg(M + 7) * r[1] + __ldg(M + 8) * r[2];
+                    const double ri = inv_norm(x, y, z);
                     double ax, ay, az;
-                    assemble_itrs(g.gm, x, y, z, inv_norm(x, y, z), xs[j], xs[pad + j], xs[2 * pad + j], xs[3 * pad + j],
+                    assemble_itrs(central(g.gm, x, y, z, ri), x, y, z, ri, xs[j], xs[pad + j], xs[2 * pad + j], xs[3 * pad + j],
                         ax, ay, az);
                     a8[0] = __ldg(M + 0) * ax + __ldg(M + 3) * ay + __ldg(M + 6) * az;
                     a8[1] = __ldg(M + 1) * ax + __ldg(M + 4) * ay + __ldg(M + 7) * az;

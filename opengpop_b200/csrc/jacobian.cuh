@@ -169,7 +169,9 @@ __device__ __forceinline__ void gravity_jac_itrs(const GravSmem& gs, int l, int 
             dF[f][j] = F[f][1] * gq[j] + F[f][2] * ge[j] + F[f][3] * gc[j] + F[f][4] * gsn[j];
     // a = c (Lambda p^ - P), P = (J, K, H), Lambda = 1 + G + eps H, c = -GM / r^2
     const double Lambda = t.Gv + 1.0 + eps * t.Hv;
-    const double c = -gs.gm * (invr * invr);
+    const double e = norm_error(x, y, z, invr), c0 = -gs.gm * (invr * invr);
+    const double c = fma(c0, 1.5 * e, c0); // as central()
+    const double pe[3] = { fma(ph[0], e, ph[0]), fma(ph[1], e, ph[1]), fma(ph[2], e, ph[2]) }; // and of its p^ p^
     double dL[3];
 #pragma unroll
     for (int j = 0; j < 3; ++j)
@@ -180,8 +182,8 @@ __device__ __forceinline__ void gravity_jac_itrs(const GravSmem& gs, int l, int 
         a[i] = c * base;
 #pragma unroll
         for (int j = 0; j < 3; ++j)
-            Jm[i][j] = -2.0 * c * ph[j] * invr * base
-                + c * (dL[j] * ph[i] + Lambda * ((i == j ? 1.0 : 0.0) - ph[i] * ph[j]) * invr - dF[i + 1][j]);
+            Jm[i][j] = -2.0 * c * pe[j] * invr * base
+                + c * (dL[j] * ph[i] + Lambda * ((i == j ? 1.0 : 0.0) - ph[i] * pe[j]) * invr - dF[i + 1][j]);
     }
 }
 

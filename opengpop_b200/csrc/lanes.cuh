@@ -407,7 +407,7 @@ template <bool MIXED, int K, bool PAIRS = false, class Team = WarpTeam>
 __device__ __forceinline__ void gravity_itrs_team(const GravSmem& gs, const Team& team, const double (&x)[K],
     const double (&y)[K], const double (&z)[K], double (&ax)[K], double (&ay)[K], double (&az)[K])
 {
-    double ri[K], u[K], w[K], G[K], H[K], J[K], KK[K];
+    double ri[K], gr2[K], u[K], w[K], G[K], H[K], J[K], KK[K];
     LanePowers lp[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) {
@@ -415,6 +415,7 @@ __device__ __forceinline__ void gravity_itrs_team(const GravSmem& gs, const Team
         const double q = gs.radius * ri[k];
         u[k] = q * (z[k] * ri[k]);
         w[k] = q * q;
+        gr2[k] = central(gs.gm, x[k], y[k], z[k], ri[k]); // here it hides behind the walk
         G[k] = H[k] = J[k] = KK[k] = 0.0;
         lp[k] = lane_powers(x[k] * ri[k], y[k] * ri[k], q, team.l, team.top(), team.P, team.P <= gs.L);
     }
@@ -422,7 +423,7 @@ __device__ __forceinline__ void gravity_itrs_team(const GravSmem& gs, const Team
 #pragma unroll
     for (int k = 0; k < K; ++k) {
         team.sum4(G[k], H[k], J[k], KK[k]);
-        assemble_itrs(gs.gm, x[k], y[k], z[k], ri[k], G[k], H[k], J[k], KK[k], ax[k], ay[k], az[k]);
+        assemble_itrs(gr2[k], x[k], y[k], z[k], ri[k], G[k], H[k], J[k], KK[k], ax[k], ay[k], az[k]);
     }
 }
 

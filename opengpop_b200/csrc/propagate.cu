@@ -393,7 +393,8 @@ __device__ __forceinline__ void split_eval(const GravSmem& g, const double* __re
         const int64_t sl = slot(k, tau, obj[k]);
         const double x = X.get(0, sl), y = X.get(1, sl), z = X.get(2, sl);
         double ax, ay, az;
-        assemble_itrs(g.gm, x, y, z, inv_norm(x, y, z), X.get(8, sl) + hi.G[k], X.get(9, sl) + hi.H[k],
+        const double ri = inv_norm(x, y, z);
+        assemble_itrs(central(g.gm, x, y, z, ri), x, y, z, ri, X.get(8, sl) + hi.G[k], X.get(9, sl) + hi.H[k],
             X.get(10, sl) + hi.J[k], X.get(11, sl) + hi.K[k], ax, ay, az);
         a8[k][0] = m[0] * ax + m[3] * ay + m[6] * az;
         a8[k][1] = m[1] * ax + m[4] * ay + m[7] * az;

@@ -1749,3 +1749,22 @@ int32_t or_miss_fd(const void* dv, const or_time* st, double h, int32_t steps, i
 }
 
 } // extern "C"
+
+extern "C" void or_gravity_ld(const void* dv, int64_t n, const double* r, double* hi, double* lo)
+{
+    const Data& d = *static_cast<const Data*>(dv);
+#pragma omp parallel
+    {
+        GravScratchT<long double> gs(d);
+#pragma omp for
+        for (int64_t i = 0; i < n; ++i) {
+            const long double p[3] = { r[3 * i], r[3 * i + 1], r[3 * i + 2] };
+            long double a[3];
+            gravity_itrs(d, p, a, gs.P, gs.Cm, gs.Sm, gs.sums);
+            for (int j = 0; j < 3; ++j) {
+                hi[3 * i + j] = (double)a[j];
+                lo[3 * i + j] = (double)(a[j] - hi[3 * i + j]);
+            }
+        }
+    }
+}

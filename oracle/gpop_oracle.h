@@ -150,6 +150,10 @@ int32_t or_miss_fd(const void* data, const or_time* start, double h, int32_t ste
     int64_t n_pairs, const double* rA, const double* vA, const double* rB, const double* vB, double dr,
     double dv, double* miss, double* tca, double* grad, int32_t threads);
 
+/* ---- extended precision (long double), for the errors of 64-bit results ----
+ * Accelerations at Earth-fixed positions r (n x 3): each value as hi + lo. */
+void or_gravity_ld(const void* data, int64_t n, const double* r, double* hi, double* lo);
+
 #ifdef __cplusplus
 }
 #endif

@@ -1,0 +1,16 @@
+"""The oracle's extended-precision (long double) entry points: what the errors of 64-bit results are taken from."""
+import ctypes as C
+
+import numpy as np
+
+import oracle_api as O
+
+
+def gravity(data, r):
+    """Accelerations at Earth-fixed positions r [n, 3] as (hi, lo), hi + lo the value."""
+    r = O.f64(r)
+    hi, lo = np.zeros_like(r), np.zeros_like(r)
+    fn = O.lib().or_gravity_ld
+    fn.restype, fn.argtypes = None, [C.c_void_p, C.c_int64] + [C.c_void_p] * 3
+    fn(data.h, r.shape[0], O.ptr(r), O.ptr(hi), O.ptr(lo))
+    return hi, lo
