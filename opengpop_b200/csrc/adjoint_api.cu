@@ -87,29 +87,36 @@ gpop_status begin(gpop_ctx* ctx, gpop_propagator& p, const gpop_time* start, dou
     return propagator_init(&p, s);
 }
 
+constexpr size_t kPassBytes = (size_t)64 << 20; // Jacobians of plain startup passes held at once
+
 // Positions of the startup's stages and columns, their Jacobians and the startup tangents.
 struct StartupTangents {
-    DevBuf stage_pos, col_pos, stage_jac, col_jac, out;
+    DevBuf stage_pos, col_pos, pass_pos, stage_jac, col_jac, pass_jac, out;
+    int window = 1; // plain passes whose Jacobians are held at once
     explicit StartupTangents(const gpop_ctx* ctx)
     {
-        for (DevBuf* b : { &stage_pos, &col_pos, &stage_jac, &col_jac, &out })
+        for (DevBuf* b : { &stage_pos, &col_pos, &pass_pos, &stage_jac, &col_jac, &pass_jac, &out })
             b->use(ctx->pool, true);
     }
     ~StartupTangents()
     {
-        for (DevBuf* b : { &stage_pos, &col_pos, &stage_jac, &col_jac, &out })
+        for (DevBuf* b : { &stage_pos, &col_pos, &pass_pos, &stage_jac, &col_jac, &pass_jac, &out })
             b->release();
     }
     gpop_status reserve(gpop_ctx* ctx, gpop_propagator& p)
     {
         const size_t n = (size_t)p.n;
+        window = (int)std::min<size_t>(p.ncorr, std::max<size_t>(1, kPassBytes / (81 * n * 8)));
         cudaError_t e;
         if ((e = stage_pos.ensure(240 * n * 8)) != cudaSuccess || (e = col_pos.ensure(27 * n * 8)) != cudaSuccess
+            || (e = pass_pos.ensure((size_t)p.ncorr * 27 * n * 8)) != cudaSuccess
+            || (e = pass_jac.ensure((size_t)window * 81 * n * 8)) != cudaSuccess
             || (e = stage_jac.ensure(720 * n * 8)) != cudaSuccess || (e = col_jac.ensure(81 * n * 8)) != cudaSuccess
             || (e = out.ensure((size_t)kStartupTangents * 6 * n * 8)) != cudaSuccess)
             return nomem(ctx, "startup tangents", e);
         p.stage_pos = stage_pos.as<double>();
         p.col_pos = col_pos.as<double>();
+        p.pass_pos = pass_pos.as<double>();
         return GPOP_OK;
     }
     // after the startup of p has run
@@ -139,16 +146,33 @@ struct StartupTangents {
         t.col_jac = col_jac.as<double>();
         t.out = out.as<double>();
         if (e == cudaSuccess)
-            e = launch_startup_tangents(t, s);
+            e = launch_rk8_tangents(t, s);
+        ctx->launches += 3;
+        t.mark = pass_pos.as<double>();
+        t.pass_jac = pass_jac.as<double>();
+        j.frames = 9;
+        j.mark = t.mark;
+        j.jac = pass_jac.as<double>();
+        for (; t.pass_lo < p.ncorr && e == cudaSuccess; t.pass_lo = t.pass_hi) {
+            t.pass_hi = std::min(p.ncorr, t.pass_lo + window);
+            j.pos = pass_pos.as<double>() + (size_t)t.pass_lo * 27 * p.n;
+            j.items = 9 * (t.pass_hi - t.pass_lo);
+            j.total = j.items * p.n;
+            if ((e = launch_jac_points(ctx->table(false), j, ctx->num_sms, s)) == cudaSuccess)
+                e = launch_pass_tangents(t, s);
+            ctx->launches += 2;
+        }
+        if (e == cudaSuccess)
+            e = launch_corrector_tangents(t, s);
+        ctx->launches++;
         if (e != cudaSuccess)
             return cuda_fail(ctx, e, "startup tangents");
-        ctx->launches += 4;
         return GPOP_OK;
     }
 };
 
-// Forward run of the adjoint: the whole trajectory's positions in traj_r (and v, a when asked for), or,
-// with traj_r NULL, the GJ8 state after the startup and after every 64th step in ckpt.
+// Forward run of the adjoint: the whole trajectory's positions and accelerations in traj_r and traj_a (and v when
+// asked for), or, with traj_r NULL, the GJ8 state after the startup and after every 64th step in ckpt.
 gpop_status forward_run(gpop_ctx* ctx, gpop_propagator& p, int32_t steps, double* traj_r, double* traj_v,
     double* traj_a, DevBuf& ckpt, cudaStream_t s)
 {
@@ -182,7 +206,7 @@ gpop_status forward_run(gpop_ctx* ctx, gpop_propagator& p, int32_t steps, double
 // Reverse sweep over a forward run. step0: host copy of the units' first seeded step, obj_host of their
 // objects. Device: unit_obj, seed_step0, seeds, grad.
 gpop_status run_adjoint(gpop_ctx* ctx, gpop_propagator& p, int32_t steps, const double* r0, const double* v0,
-    const double* traj_r, const DevBuf& ckpt, StartupTangents& tan, const std::vector<int>& step0,
+    const double* traj_r, const double* traj_a, const DevBuf& ckpt, StartupTangents& tan, const std::vector<int>& step0,
     const std::vector<int>& obj_host, const int* unit_obj, const int* seed_step0, const double* seeds, double* grad,
     cudaStream_t s)
 {
@@ -259,9 +283,11 @@ gpop_status run_adjoint(gpop_ctx* ctx, gpop_propagator& p, int32_t steps, const 
             != cudaSuccess)
             return cuda_fail(ctx, e, "adjoint window");
         const double* pos = traj_r ? traj_r + (size_t)(lo - 1) * 3 * n : nullptr;
+        const double* acc = traj_r ? traj_a + (size_t)(lo - 1) * 3 * n : nullptr;
         if (!traj_r) { // run the window's segment again from its checkpoint
             const int seg = (lo - 1) / kCheckpointSteps, from = std::max(5, seg * kCheckpointSteps + 1);
-            if ((e = B.pos.ensure((size_t)(hi - from + 1) * 3 * n * sizeof(double))) != cudaSuccess)
+            const size_t rows = (size_t)(hi - from + 1) * 3 * n;
+            if ((e = B.pos.ensure(2 * rows * sizeof(double))) != cudaSuccess)
                 return nomem(ctx, "adjoint segment", e);
             const size_t ck = (size_t)kCheckpointArrays * n;
             if ((e = cudaMemcpyAsync(p.state->as<double>() + (size_t)kSs * n, ckpt.as<double>() + (size_t)seg * ck,
@@ -269,14 +295,17 @@ gpop_status run_adjoint(gpop_ctx* ctx, gpop_propagator& p, int32_t steps, const 
                 != cudaSuccess)
                 return cuda_fail(ctx, e, "checkpoint restore");
             p.done = from - 1;
-            const gpop_status st = propagator_step(&p, hi - from + 1, B.pos.as<double>(), nullptr, nullptr, s);
+            const gpop_status st
+                = propagator_step(&p, hi - from + 1, B.pos.as<double>(), nullptr, B.pos.as<double>() + rows, s);
             if (st != GPOP_OK)
                 return st;
             pos = B.pos.as<double>() + (size_t)(lo - from) * 3 * n;
+            acc = pos + rows;
         }
         JacPoints j;
         j.n = n;
         j.pos = pos;
+        j.acc = acc;
         j.M = p.prop_m->as<double>() + (size_t)(lo + 4) * 9;
         j.items = (int)offset.size();
         j.offset = B.offset.as<int64_t>();
@@ -408,10 +437,10 @@ gpop_status gpop_stm(gpop_ctx* ctx, const gpop_time* start, double h, int32_t st
             || (st = begin(ctx, p, start, h, steps, m, dr.as<double>(), dv.as<double>(), s)) != GPOP_OK
             || (st = tan.reserve(ctx, p)) != GPOP_OK)
             return st;
-        const int window = (int)std::min<int64_t>(steps, std::max<int64_t>(1, (int64_t)(kWindowBytes / 96) / m));
+        const int window = (int)std::min<int64_t>(steps, std::max<int64_t>(1, (int64_t)(kWindowBytes / 120) / m));
         cudaError_t e;
         if ((e = dphi.ensure(36 * m * sizeof(double))) != cudaSuccess
-            || (e = pos.ensure((size_t)window * 3 * m * sizeof(double))) != cudaSuccess
+            || (e = pos.ensure((size_t)window * 6 * m * sizeof(double))) != cudaSuccess
             || (e = jac.ensure((size_t)window * 9 * m * sizeof(double))) != cudaSuccess
             || (e = sweep.ensure((size_t)kStmSweep * 6 * m * sizeof(double))) != cudaSuccess)
             return nomem(ctx, "STM buffers", e);
@@ -433,11 +462,13 @@ gpop_status gpop_stm(gpop_ctx* ctx, const gpop_time* start, double h, int32_t st
             a.step_hi = done + w;
             a.last = a.step_hi >= steps;
             if (w > 0) {
-                if ((st = propagator_step(&p, w, pos.as<double>(), nullptr, nullptr, s)) != GPOP_OK)
+                double* acc = pos.as<double>() + (size_t)window * 3 * m;
+                if ((st = propagator_step(&p, w, pos.as<double>(), nullptr, acc, s)) != GPOP_OK)
                     return st;
                 JacPoints j;
                 j.n = j.width = m;
                 j.pos = pos.as<double>();
+                j.acc = acc;
                 j.M = p.prop_m->as<double>() + (size_t)(a.step_lo + 4) * 9;
                 j.items = w;
                 j.total = (int64_t)w * m;
@@ -490,15 +521,17 @@ gpop_status gpop_propagate_vjp(gpop_ctx* ctx, const gpop_time* start, double h, 
     if ((st = upload(ctx, dr, r_in, 3 * n, s)) != GPOP_OK || (st = upload(ctx, dv, v_in, 3 * n, s)) != GPOP_OK
         || (st = upload(ctx, dr0, r_in, 3 * n, s)) != GPOP_OK || (st = upload(ctx, dv0, v_in, 3 * n, s)) != GPOP_OK)
         return st;
-    // the positions of every step when they fit, else checkpoints
-    const size_t traj_bytes = (size_t)steps * 3 * n * sizeof(double);
+    // the positions and accelerations of every step when they fit, else checkpoints
+    const size_t rows = (size_t)steps * 3 * n, traj_bytes = 2 * rows * sizeof(double);
     const bool store = traj_bytes <= ctx->adjoint_store && traj.ensure(traj_bytes) == cudaSuccess;
     if (!store)
         cudaGetLastError(); // a failed allocation
     gpop_propagator p;
     if ((st = begin(ctx, p, start, h, steps, n, dr.as<double>(), dv.as<double>(), s)) != GPOP_OK
         || (n <= kVarObjects && (st = tan.reserve(ctx, p)) != GPOP_OK)
-        || (st = forward_run(ctx, p, steps, store ? traj.as<double>() : nullptr, nullptr, nullptr, ck, s)) != GPOP_OK)
+        || (st = forward_run(ctx, p, steps, store ? traj.as<double>() : nullptr, nullptr,
+                store ? traj.as<double>() + rows : nullptr, ck, s))
+            != GPOP_OK)
         return st;
     // seeds on the final state: node 0 at the last step
     std::vector<int> obj(n), step0(n, steps);
@@ -519,8 +552,8 @@ gpop_status gpop_propagate_vjp(gpop_ctx* ctx, const gpop_time* start, double h, 
     if ((e = cudaMemcpyAsync(dobj.p, obj.data(), n * sizeof(int), cudaMemcpyHostToDevice, s)) != cudaSuccess
         || (e = cudaMemcpyAsync(dstep.p, step0.data(), n * sizeof(int), cudaMemcpyHostToDevice, s)) != cudaSuccess)
         return cuda_fail(ctx, e, "seed upload");
-    if ((st = run_adjoint(ctx, p, steps, dr0.as<double>(), dv0.as<double>(), store ? traj.as<double>() : nullptr, ck,
-             tan, step0, obj, dobj.as<int>(), dstep.as<int>(), dseed.as<double>(), dgrad.as<double>(), s))
+    if ((st = run_adjoint(ctx, p, steps, dr0.as<double>(), dv0.as<double>(), store ? traj.as<double>() : nullptr,
+             store ? traj.as<double>() + rows : nullptr, ck, tan, step0, obj, dobj.as<int>(), dstep.as<int>(), dseed.as<double>(), dgrad.as<double>(), s))
         != GPOP_OK)
         return st;
     std::vector<double> g(6 * n);
@@ -602,7 +635,7 @@ gpop_status gpop_miss_gradient(gpop_ctx* ctx, const gpop_time* start, double h, 
     if ((e = cudaMemcpy(step0.data(), pa.seed_step0, U * sizeof(int), cudaMemcpyDeviceToHost)) != cudaSuccess)
         return cuda_fail(ctx, e, "pair approach kernel");
     std::copy(pairs, pairs + U, obj.begin());
-    if ((st = run_adjoint(ctx, p, steps, dr0.as<double>(), dv0.as<double>(), tr, ck, tan, step0, obj, pa.unit_obj,
+    if ((st = run_adjoint(ctx, p, steps, dr0.as<double>(), dv0.as<double>(), tr, tr + 2 * tn, ck, tan, step0, obj, pa.unit_obj,
              pa.seed_step0, pa.seeds, dgrad.as<double>(), s))
         != GPOP_OK)
         return st;

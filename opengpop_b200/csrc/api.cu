@@ -177,6 +177,7 @@ gpop_status propagator_step(gpop_propagator* p, int steps, double* traj_r, doubl
     a.v0 = p->v;
     a.stage_pos = p->stage_pos;
     a.col_pos = p->col_pos;
+    a.pass_pos = p->pass_pos;
     if (!p->started) {
         if ((e = launch_startup(ts, a, ctx->num_sms, s, &lane_ts, &lane64)) != cudaSuccess)
             return cuda_fail(ctx, e, "startup kernel");

@@ -255,8 +255,9 @@ struct gpop_propagator {
     int done = 0;
     bool started = false;
     bool mixed = false;
-    double* stage_pos = nullptr; // StartupArgs::stage_pos, col_pos (variational equations)
+    double* stage_pos = nullptr; // StartupArgs::stage_pos, col_pos, pass_pos (variational equations)
     double* col_pos = nullptr;
+    double* pass_pos = nullptr;
     gpop::DevBuf own_state, own_gen, own_prop;
     gpop::DevBuf *state = &own_state, *gen_m = &own_gen, *prop_m = &own_prop;
     ~gpop_propagator()

@@ -53,8 +53,9 @@ struct PropArgs {
     const double* r0 = nullptr;
     const double* v0 = nullptr;
     double* out27[5] = { nullptr, nullptr, nullptr, nullptr, nullptr };
-    double* stage_pos = nullptr; // StartupArgs::stage_pos, col_pos
+    double* stage_pos = nullptr; // StartupArgs::stage_pos, col_pos, pass_pos
     double* col_pos = nullptr;
+    double* pass_pos = nullptr;
     // GJ8 range and outputs
     int step_begin = 1, step_end = 1; // steps [begin, end), 1-based
     double* traj_r = nullptr; // [steps][3][n], indexed by step - traj_step0

@@ -1032,6 +1032,7 @@ cudaError_t launch_startup(const TableSrc& ts, const PropArgs& a, int num_sms, c
         b.err = a.err;
         b.stage_pos = a.stage_pos;
         b.col_pos = a.col_pos;
+        b.pass_pos = a.pass_pos;
         // few objects: the FP64 table, as their steps (step_walk)
         return launch_startup_gravity(ts, lane64 && 2 * a.n <= 4 * (int64_t)num_sms ? *lane64 : *lane_ts, b, num_sms, s);
     }

@@ -456,9 +456,14 @@ template <bool BATCH> __global__ void __launch_bounds__(128) startup_correct_ker
     const size_t n = (size_t)a.n;
     int* flags = reinterpret_cast<int*>(a.state + (size_t)kSflag * n);
     int flag = flags[o];
-    if (flag & kFlagDone)
-        return;
     double* st = a.state + o;
+    double* before = a.pass_pos ? a.pass_pos + (size_t)it * 27 * n + o : nullptr;
+    if (flag & kFlagDone) { // the passes left repeat the last one
+        if (before && !(flag & kFlagFast))
+            for (int i = 0; i < 27; ++i)
+                before[i * n] = st[(kSr + i) * n];
+        return;
+    }
     const double h = source<BATCH>(a, o, 0).h;
     double acc[9][3], pos[9][3], v4[3];
     for (int c = 0; c < 9; ++c)
@@ -540,6 +545,11 @@ template <bool BATCH> __global__ void __launch_bounds__(128) startup_correct_ker
                         st[(kHist + c * 3 + j) * n] = ac[c][j];
         }
     }
+    if (before && !(flag & kFlagFast))
+        for (int i = 0; i < 27; ++i)
+            before[i * n] = pos[i / 3][i % 3];
+    else if (before && it == 0)
+        before[0] = __longlong_as_double(0x7ff8000000000000ll);
     for (int j = 0; j < 3; ++j) {
         for (int c = 0; c < 9; ++c)
             if (c != 4)

@@ -23,9 +23,11 @@ struct StartupArgs {
     bool check = false; // raise kErrBadInput for states gravity cannot take
     unsigned* err = nullptr;
     // for the variational equations (may be NULL): positions of the 80 RK8 stages, in the order of gen_m,
-    // and of the nine columns at the end, [.][3][n]
+    // and of the nine columns at the end, [.][3][n]; of the columns in front of every corrector pass,
+    // [ncorr][9][3][n], for objects that take the plain passes (NaN in the first value of the others)
     double* stage_pos = nullptr;
     double* col_pos = nullptr;
+    double* pass_pos = nullptr;
 };
 
 // plain: the plain table, lanes: the lane-layout table of the same precision.

@@ -3,9 +3,13 @@
 //
 // Tangents and adjoints are the derivatives of the discrete map of the forward propagation (startup, GJ8
 // steps: gpu_propagator.cu:28-119) with one simplification: the Jacobian of a step's corrector passes is
-// taken once, at the step's position (the corrector converges, so the passes' iterates differ by far less
-// than the truncation error); the startup's columns likewise. Forward tangents and the reverse sweep make
-// the same choice, so they are exact transposes of each other.
+// taken once, at the position of the last evaluation (the corrector converges, so the passes' iterates differ by
+// far less than the truncation error); of the startup's passes likewise where they converge, else in front of each
+// (pass_tangent_kernel). Forward tangents and the reverse sweep make the same choice, so they are exact transposes of
+// each other. With few passes the last evaluation is not at the step's position: found from its acceleration
+// (evaluation_point). Transition matrices of 40 steps of 120 s against differences in long double, largest error of a
+// block with 1, 2 and 3 passes: with one Jacobian per step and column at the last positions 7e-7, 9e-9 and 2e-10,
+// with those of the evaluations 1.1e-13, 7e-10 and 7e-13.
 //
 // The Jacobians depend on the positions alone, not on the tangents. So the forward propagation runs with
 // the propagation's own kernels and keeps its positions (per step, and of the startup's 80 stages and nine
@@ -48,6 +52,35 @@ __device__ __forceinline__ bool bind_plain64(uint8_t* smem, const TableSrc& ts, 
 
 } // namespace
 
+// Moves r to where gravity, with Jacobian J, is larger by d. False, with r as it was, where that is at rounding
+// (2^-46 of r: a converged corrector, some 1e-15) or not near. J has no trace, so it is far from singular.
+__device__ __forceinline__ bool evaluation_point(const double (&J)[3][3], const double (&d)[3], double (&r)[3])
+{
+    double x[3], c0[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) { // cofactors of column j
+        const int k = (j + 1) % 3, l = (j + 2) % 3;
+        double c[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            c[i] = J[(i + 1) % 3][k] * J[(i + 2) % 3][l] - J[(i + 2) % 3][k] * J[(i + 1) % 3][l];
+        x[j] = c[0] * d[0] + c[1] * d[1] + c[2] * d[2];
+        if (j == 0)
+            for (int i = 0; i < 3; ++i)
+                c0[i] = c[i];
+    }
+    const double det = fabs(c0[0] * J[0][0] + c0[1] * J[1][0] + c0[2] * J[2][0]);
+    const double move = fmax(fmax(fabs(x[0]), fabs(x[1])), fabs(x[2]));
+    const double size = fmax(fmax(fabs(r[0]), fabs(r[1])), fabs(r[2])) * det;
+    if (!(move > 0x1p-46 * size) || !(move < 0x1p-4 * size))
+        return false;
+    const double inv = 1.0 / (c0[0] * J[0][0] + c0[1] * J[1][0] + c0[2] * J[2][0]);
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+        r[j] = fma(x[j], inv, r[j]);
+    return true;
+}
+
 // ---- Jacobians of many points ----
 __global__ void __launch_bounds__(256, 1) jac_points_kernel(TableSrc ts, JacPoints a)
 {
@@ -74,11 +107,25 @@ __global__ void __launch_bounds__(256, 1) jac_points_kernel(TableSrc ts, JacPoin
             u = t - i * a.width;
         }
         const int64_t o = a.obj ? a.obj[u] : u;
+        if (a.mark && isnan(a.mark[o]))
+            continue;
+        const double* M = a.M + (size_t)(a.frames ? i % a.frames : i) * 9;
         double r[3], acc[3], J[3][3];
 #pragma unroll
         for (int j = 0; j < 3; ++j)
             r[j] = a.pos[(i * 3 + j) * a.n + o];
-        gravity_jac_gcrs<false>(g, 0, 1, a.M + (size_t)i * 9, r, acc, J, 0u);
+#pragma unroll 1
+        for (int it = 0;; ++it) {
+            gravity_jac_gcrs<false>(g, 0, 1, M, r, acc, J, 0u);
+            if (!a.acc || it == 4)
+                break;
+            double d[3];
+#pragma unroll
+            for (int j = 0; j < 3; ++j)
+                d[j] = a.acc[(i * 3 + j) * a.n + o] - acc[j];
+            if (!evaluation_point(J, d, r))
+                break;
+        }
 #pragma unroll
         for (int k = 0; k < 9; ++k)
             a.jac[(int64_t)k * a.total + t] = J[k / 3][k % 3];
@@ -152,35 +199,39 @@ __global__ void __launch_bounds__(128) rk8_tangent_kernel(StartupTangentArgs a)
     }
 }
 
-// The mid-corrector's passes of direction dir, with one Jacobian per column: out slots 0..26 the
-// accelerations, 27..32 s and S of column 8, 33..44 and 45..56 positions and velocities of columns 5..8.
-__global__ void __launch_bounds__(128) corrector_tangent_kernel(StartupTangentArgs a)
-{
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= 6 * a.n)
-        return;
-    const int64_t n = a.n, o = t % n;
-    const int dir = (int)(t / n);
-    double* out = a.out + (int64_t)dir * n + o;
-    auto slot = [&](int k) -> double& { return out[(int64_t)k * 6 * n]; };
+// The mid-corrector of direction dir. Position tangents of the columns in out slots 0..26 become, at the end, those
+// of the accelerations; 27..32 s and S of column 8, 33..44 and 45..56 positions and velocities of columns 5..8.
+struct ColumnTangents {
+    double* out;
+    int64_t stride;
     double dr[9][3], da[9][3], r4[3], v4[3];
-    for (int c = 0; c < 9; ++c)
-        for (int j = 0; j < 3; ++j)
-            dr[c][j] = slot(c * 3 + j);
-    for (int j = 0; j < 3; ++j) {
-        r4[j] = dir == j ? 1.0 : 0.0;
-        v4[j] = dir == 3 + j ? 1.0 : 0.0;
-    }
-    auto accel = [&](int c) {
-        double J[3][3];
-        load_jac(a.col_jac, 9 * n, (int64_t)c * n + o, J);
-        mul(J, dr[c], da[c]);
-    };
-    for (int c = 0; c < 9; ++c)
-        accel(c);
     PassResult p;
-    for (int it = 0; it < a.ncorr; ++it) {
-        corrector_pass(a.h, da, r4, v4, p);
+    __device__ __forceinline__ ColumnTangents(const StartupTangentArgs& a, int64_t t)
+        : out(a.out + t)
+        , stride(6 * a.n)
+    {
+        const int dir = (int)(t / a.n);
+        for (int c = 0; c < 9; ++c)
+            for (int j = 0; j < 3; ++j)
+                dr[c][j] = slot(c * 3 + j);
+        for (int j = 0; j < 3; ++j) {
+            r4[j] = dir == j ? 1.0 : 0.0;
+            v4[j] = dir == 3 + j ? 1.0 : 0.0;
+        }
+    }
+    __device__ __forceinline__ double& slot(int k) const { return out[(int64_t)k * stride]; }
+    __device__ __forceinline__ void accelerations(const double* jac, int64_t total, int64_t n, int64_t first)
+    {
+        for (int c = 0; c < 9; ++c) {
+            double J[3][3];
+            load_jac(jac, total, first + (int64_t)c * n, J);
+            mul(J, dr[c], da[c]);
+        }
+    }
+    // a pass; whether it left every position as it was
+    __device__ __forceinline__ bool pass(double h)
+    {
+        corrector_pass(h, da, r4, v4, p);
         bool same = true;
         for (int c = 0; c < 9; ++c) {
             if (c == 4)
@@ -189,21 +240,64 @@ __global__ void __launch_bounds__(128) corrector_tangent_kernel(StartupTangentAr
                 same = same && same_bits(dr[c][j], p.r[c][j]);
                 dr[c][j] = p.r[c][j];
             }
-            accel(c);
         }
+        return same;
+    }
+    __device__ __forceinline__ void put_end(const double (&x)[9][3]) const
+    {
+        for (int j = 0; j < 3; ++j) {
+            for (int c = 0; c < 9; ++c)
+                slot(c * 3 + j) = x[c][j];
+            slot(27 + j) = p.s8[j];
+            slot(30 + j) = p.S8[j];
+            for (int k = 0; k < 4; ++k) {
+                slot(33 + k * 3 + j) = dr[5 + k][j];
+                slot(45 + k * 3 + j) = p.v[k][j];
+            }
+        }
+    }
+};
+
+// Passes of the objects that take them one by one (few passes, long steps), each with the Jacobians in front of it.
+__global__ void __launch_bounds__(128) pass_tangent_kernel(StartupTangentArgs a)
+{
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= 6 * a.n)
+        return;
+    const int64_t n = a.n, o = t % n;
+    if (isnan(a.mark[o]))
+        return;
+    ColumnTangents q(a, t);
+    for (int it = a.pass_lo; it < a.pass_hi; ++it) {
+        q.accelerations(a.pass_jac, (int64_t)(a.pass_hi - a.pass_lo) * 9 * n, n, (int64_t)(it - a.pass_lo) * 9 * n + o);
+        q.pass(a.h);
+    }
+    q.put_end(q.dr);
+}
+
+// The end: the accelerations at the last positions, behind the passes of the others, which have converged: one
+// Jacobian per column serves them all.
+__global__ void __launch_bounds__(128) corrector_tangent_kernel(StartupTangentArgs a)
+{
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= 6 * a.n)
+        return;
+    const int64_t n = a.n, o = t % n;
+    ColumnTangents q(a, t);
+    q.accelerations(a.col_jac, 9 * n, n, o);
+    if (!isnan(a.mark[o])) {
+        for (int c = 0; c < 9; ++c)
+            for (int j = 0; j < 3; ++j)
+                q.slot(c * 3 + j) = q.da[c][j];
+        return;
+    }
+    for (int it = 0; it < a.ncorr; ++it) {
+        const bool same = q.pass(a.h);
+        q.accelerations(a.col_jac, 9 * n, n, o);
         if (same) // every further pass repeats this one
             break;
     }
-    for (int j = 0; j < 3; ++j) {
-        for (int c = 0; c < 9; ++c)
-            slot(c * 3 + j) = da[c][j];
-        slot(27 + j) = p.s8[j];
-        slot(30 + j) = p.S8[j];
-        for (int k = 0; k < 4; ++k) {
-            slot(33 + k * 3 + j) = dr[5 + k][j];
-            slot(45 + k * 3 + j) = p.v[k][j];
-        }
-    }
+    q.put_end(q.da);
 }
 
 // ---- forward variational equations: steps [step_lo, step_hi] of every (direction, object) ----
@@ -576,11 +670,20 @@ cudaError_t launch_jac_points(const TableSrc& plain64, const JacPoints& a, int n
     return cudaGetLastError();
 }
 
-cudaError_t launch_startup_tangents(const StartupTangentArgs& a, cudaStream_t s)
+cudaError_t launch_rk8_tangents(const StartupTangentArgs& a, cudaStream_t s)
 {
-    if (a.n <= 0)
-        return cudaSuccess;
     rk8_tangent_kernel<<<(unsigned)((12 * a.n + 127) / 128), 128, 0, s>>>(a);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_pass_tangents(const StartupTangentArgs& a, cudaStream_t s)
+{
+    pass_tangent_kernel<<<(unsigned)((6 * a.n + 127) / 128), 128, 0, s>>>(a);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_corrector_tangents(const StartupTangentArgs& a, cudaStream_t s)
+{
     corrector_tangent_kernel<<<(unsigned)((6 * a.n + 127) / 128), 128, 0, s>>>(a);
     return cudaGetLastError();
 }

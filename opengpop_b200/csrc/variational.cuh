@@ -14,10 +14,15 @@ constexpr int kCheckpointArrays = 33; // s, S and the 9-slot history (state arra
 // Jacobians at many positions: item i (a step, an RK8 stage, a column) of object o lies at
 // pos[(i 3 + j) n + o] in the frame M[i 9 ..]. Entry t of the result, 9 arrays of `total`, is item i's
 // u-th object (obj[u], or u): t = i width + u, or offset[i] + u where the items hold fewer and fewer.
+// With acc (laid out as pos) the Jacobian is taken where gravity is acc, next to pos: the positions of a step are
+// those after its last corrector pass, its acceleration that of the evaluation before.
 struct JacPoints {
     int64_t n = 0; // stride of the positions
     const double* pos = nullptr;
+    const double* acc = nullptr;
     const double* M = nullptr;
+    int frames = 0; // M of item i is that of i % frames (0: of i)
+    const double* mark = nullptr; // [n]: objects with NaN here are left out (may be NULL)
     int64_t width = 0;
     int items = 0;
     const int64_t* offset = nullptr; // [items], ascending
@@ -36,7 +41,12 @@ struct StartupTangentArgs {
     double h = 0;
     int ncorr = 7;
     const double* stage_jac = nullptr; // 9 arrays of 80 n, stages in the order of gen_m
-    const double* col_jac = nullptr; // 9 arrays of 9 n
+    const double* col_jac = nullptr; // 9 arrays of 9 n, at the columns' last positions
+    const double* mark = nullptr; // [n] StartupArgs::pass_pos: NaN where the passes have converged
+    // passes [pass_lo, pass_hi) of the other objects: Jacobians at the columns in front of each, 9 arrays of
+    // (pass_hi - pass_lo) 9 n
+    const double* pass_jac = nullptr;
+    int pass_lo = 0, pass_hi = 0;
     double* out = nullptr;
 };
 
@@ -106,7 +116,11 @@ struct PairArgs {
 };
 
 cudaError_t launch_jac_points(const TableSrc& plain64, const JacPoints& a, int num_sms, cudaStream_t s);
-cudaError_t launch_startup_tangents(const StartupTangentArgs& a, cudaStream_t s);
+// Of the startup, in this order: the RK8 chains, the plain corrector passes (in as many windows as their Jacobians
+// come in), the end.
+cudaError_t launch_rk8_tangents(const StartupTangentArgs& a, cudaStream_t s);
+cudaError_t launch_pass_tangents(const StartupTangentArgs& a, cudaStream_t s);
+cudaError_t launch_corrector_tangents(const StartupTangentArgs& a, cudaStream_t s);
 cudaError_t launch_stm_sweep(const StmArgs& a, cudaStream_t s);
 cudaError_t launch_adjoint_sweep(const AdjSweepArgs& a, cudaStream_t s);
 cudaError_t launch_adjoint_finish(const AdjFinishArgs& a, cudaStream_t s);

@@ -1768,3 +1768,25 @@ extern "C" void or_gravity_ld(const void* dv, int64_t n, const double* r, double
         }
     }
 }
+
+extern "C" void or_stm_ld(const void* dv, const or_time* st, double h, int32_t steps, int32_t ncorr, int64_t n,
+    const double* r0, const double* v0, double* phi)
+{
+    using LD = long double;
+    const Force f = make_force(dv, OR_FORCE_GRAVITY, st, h, steps, 0);
+#pragma omp parallel for schedule(dynamic, 1)
+    for (int64_t job = 0; job < 6 * n; ++job) {
+        const int64_t i = job / 6;
+        const int k = (int)(job % 6);
+        const LD d = k < 3 ? 100.0L : 0.1L, off[4] = { d, -d, 2 * d, -2 * d };
+        LD x[6], y[4][6];
+        for (int q = 0; q < 4; ++q) {
+            for (int j = 0; j < 6; ++j)
+                x[j] = (j < 3 ? r0[3 * i + j] : v0[3 * i + j - 3]) + (j == k ? off[q] : 0.0L);
+            propagate_one<LD>(f, steps, ncorr, x, x + 3, n, i, nullptr, nullptr, nullptr, y[q], y[q] + 3);
+        }
+        for (int j = 0; j < 6; ++j)
+            phi[(i * 6 + j) * 6 + k]
+                = (double)((8 * (y[0][j] - y[1][j]) - (y[2][j] - y[3][j])) / (12 * d));
+    }
+}
