@@ -250,9 +250,14 @@ gpop_status run_adjoint(gpop_ctx* ctx, gpop_propagator& p, int32_t steps, const 
     a.first = true;
     int hi = U > 0 ? last(rank[0]) : 0;
     int64_t cnt = 0; // ranks that take part at the present step
-    if (hi < 5 && (e = launch_adjoint_sweep(a, s)) != cudaSuccess) // nothing to sweep: zero adjoints
-        return cuda_fail(ctx, e, "adjoint kernel");
+    if (hi < 5) { // nothing to sweep: zero adjoints
+        if ((e = launch_adjoint_sweep(a, s)) != cudaSuccess)
+            return cuda_fail(ctx, e, "adjoint kernel");
+        ctx->launches++;
+    }
     const size_t limit = std::max<size_t>(kWindowBytes / 72, (size_t)U);
+    int held = -1; // segment whose positions and accelerations, `rows` doubles each, are in B.pos
+    size_t rows = 0;
     while (hi >= 5) {
         const int floor_step = traj_r ? 5 : std::max(5, (hi - 1) / kCheckpointSteps * kCheckpointSteps + 1);
         // ranks per step from hi down, as many steps as the Jacobians' budget takes
@@ -284,21 +289,24 @@ gpop_status run_adjoint(gpop_ctx* ctx, gpop_propagator& p, int32_t steps, const 
             return cuda_fail(ctx, e, "adjoint window");
         const double* pos = traj_r ? traj_r + (size_t)(lo - 1) * 3 * n : nullptr;
         const double* acc = traj_r ? traj_a + (size_t)(lo - 1) * 3 * n : nullptr;
-        if (!traj_r) { // run the window's segment again from its checkpoint
+        if (!traj_r) {
             const int seg = (lo - 1) / kCheckpointSteps, from = std::max(5, seg * kCheckpointSteps + 1);
-            const size_t rows = (size_t)(hi - from + 1) * 3 * n;
-            if ((e = B.pos.ensure(2 * rows * sizeof(double))) != cudaSuccess)
-                return nomem(ctx, "adjoint segment", e);
-            const size_t ck = (size_t)kCheckpointArrays * n;
-            if ((e = cudaMemcpyAsync(p.state->as<double>() + (size_t)kSs * n, ckpt.as<double>() + (size_t)seg * ck,
-                     ck * sizeof(double), cudaMemcpyDeviceToDevice, s))
-                != cudaSuccess)
-                return cuda_fail(ctx, e, "checkpoint restore");
-            p.done = from - 1;
-            const gpop_status st
-                = propagator_step(&p, hi - from + 1, B.pos.as<double>(), nullptr, B.pos.as<double>() + rows, s);
-            if (st != GPOP_OK)
-                return st;
+            if (seg != held) { // its first window, which ends where the segment does: run it from its checkpoint
+                rows = (size_t)(hi - from + 1) * 3 * n;
+                if ((e = B.pos.ensure(2 * rows * sizeof(double))) != cudaSuccess)
+                    return nomem(ctx, "adjoint segment", e);
+                const size_t ck = (size_t)kCheckpointArrays * n;
+                if ((e = cudaMemcpyAsync(p.state->as<double>() + (size_t)kSs * n,
+                         ckpt.as<double>() + (size_t)seg * ck, ck * sizeof(double), cudaMemcpyDeviceToDevice, s))
+                    != cudaSuccess)
+                    return cuda_fail(ctx, e, "checkpoint restore");
+                p.done = from - 1;
+                const gpop_status st
+                    = propagator_step(&p, hi - from + 1, B.pos.as<double>(), nullptr, B.pos.as<double>() + rows, s);
+                if (st != GPOP_OK)
+                    return st;
+                held = seg;
+            }
             pos = B.pos.as<double>() + (size_t)(lo - from) * 3 * n;
             acc = pos + rows;
         }
