@@ -255,7 +255,7 @@ gpop_status run_adjoint(gpop_ctx* ctx, gpop_propagator& p, int32_t steps, const 
             return cuda_fail(ctx, e, "adjoint kernel");
         ctx->launches++;
     }
-    const size_t limit = std::max<size_t>(kWindowBytes / 72, (size_t)U);
+    size_t limit = std::max<size_t>(kWindowBytes / 72, (size_t)U);
     int held = -1; // segment whose positions and accelerations, `rows` doubles each, are in B.pos
     size_t rows = 0;
     while (hi >= 5) {
@@ -274,15 +274,20 @@ gpop_status run_adjoint(gpop_ctx* ctx, gpop_propagator& p, int32_t steps, const 
             width.push_back(c);
             --lo;
         }
-        cnt = width.back();
         std::vector<int64_t> offset(width.size()); // ascending steps
         int64_t at = 0;
         for (size_t i = 0; i < width.size(); ++i) {
             offset[i] = at;
             at += width[width.size() - 1 - i];
         }
-        if ((e = B.jac.ensure(9 * total * sizeof(double))) != cudaSuccess
-            || (e = B.offset.ensure(offset.size() * sizeof(int64_t))) != cudaSuccess)
+        e = B.jac.ensure(9 * total * sizeof(double));
+        if (e == cudaErrorMemoryAllocation && width.size() > 1) { // fewer steps at once
+            cudaGetLastError();
+            limit = total / 2;
+            continue;
+        }
+        cnt = width.back();
+        if (e != cudaSuccess || (e = B.offset.ensure(offset.size() * sizeof(int64_t))) != cudaSuccess)
             return nomem(ctx, "adjoint Jacobians", e);
         if ((e = cudaMemcpyAsync(B.offset.p, offset.data(), offset.size() * sizeof(int64_t), cudaMemcpyHostToDevice, s))
             != cudaSuccess)
@@ -390,6 +395,64 @@ gpop_status run_adjoint(gpop_ctx* ctx, gpop_propagator& p, int32_t steps, const 
     return check_device_errors(ctx, s);
 }
 
+// The vector-Jacobian product of checked arguments, from the stored trajectory or from checkpoints.
+gpop_status run_vjp(gpop_ctx* ctx, const gpop_time* start, double h, int32_t steps, int64_t n, const double* r_in,
+    const double* v_in, const double* r_bar, const double* v_bar, bool store, double* grad_r0, double* grad_v0)
+{
+    cudaStream_t s = nullptr;
+    gpop_status st;
+    cudaError_t e;
+    ScopedBufs B(ctx);
+    DevBuf &dr = B.b[0], &dv = B.b[1], &dr0 = B.b[2], &dv0 = B.b[3], &ck = B.b[4], &traj = B.b[5],
+           &dobj = B.b[6], &dstep = B.b[7], &dseed = B.b[8], &dgrad = B.b[9];
+    StartupTangents tan(ctx);
+    if ((st = upload(ctx, dr, r_in, 3 * n, s)) != GPOP_OK || (st = upload(ctx, dv, v_in, 3 * n, s)) != GPOP_OK
+        || (st = upload(ctx, dr0, r_in, 3 * n, s)) != GPOP_OK || (st = upload(ctx, dv0, v_in, 3 * n, s)) != GPOP_OK)
+        return st;
+    const size_t rows = (size_t)steps * 3 * n;
+    if (store && (e = traj.ensure(2 * rows * sizeof(double))) != cudaSuccess)
+        return nomem(ctx, "trajectory", e);
+    gpop_propagator p;
+    if ((st = begin(ctx, p, start, h, steps, n, dr.as<double>(), dv.as<double>(), s)) != GPOP_OK
+        || (n <= kVarObjects && (st = tan.reserve(ctx, p)) != GPOP_OK)
+        || (st = forward_run(ctx, p, steps, store ? traj.as<double>() : nullptr, nullptr,
+                store ? traj.as<double>() + rows : nullptr, ck, s))
+            != GPOP_OK)
+        return st;
+    // seeds on the final state: node 0 at the last step
+    std::vector<int> obj(n), step0(n, steps);
+    std::vector<double> seeds((size_t)n * 27, 0.0);
+    for (int64_t o = 0; o < n; ++o) {
+        obj[o] = (int)o;
+        for (int j = 0; j < 3; ++j) {
+            seeds[o * 27 + j] = r_bar ? r_bar[o * 3 + j] : 0.0;
+            seeds[o * 27 + 3 + j] = v_bar ? v_bar[o * 3 + j] : 0.0;
+        }
+    }
+    if ((e = dobj.ensure(n * sizeof(int))) != cudaSuccess || (e = dstep.ensure(n * sizeof(int))) != cudaSuccess
+        || (e = dgrad.ensure(6 * n * sizeof(double))) != cudaSuccess)
+        return fail(ctx, GPOP_ERR_NOMEM, std::string("adjoint buffers: ") + cudaGetErrorString(e));
+    if ((st = upload(ctx, dseed, seeds.data(), seeds.size(), s)) != GPOP_OK)
+        return st;
+    if ((e = cudaMemcpyAsync(dobj.p, obj.data(), n * sizeof(int), cudaMemcpyHostToDevice, s)) != cudaSuccess
+        || (e = cudaMemcpyAsync(dstep.p, step0.data(), n * sizeof(int), cudaMemcpyHostToDevice, s)) != cudaSuccess)
+        return cuda_fail(ctx, e, "seed upload");
+    if ((st = run_adjoint(ctx, p, steps, dr0.as<double>(), dv0.as<double>(), store ? traj.as<double>() : nullptr,
+             store ? traj.as<double>() + rows : nullptr, ck, tan, step0, obj, dobj.as<int>(),
+             dstep.as<int>(), dseed.as<double>(), dgrad.as<double>(), s))
+        != GPOP_OK)
+        return st;
+    std::vector<double> g(6 * n);
+    if ((e = cudaMemcpy(g.data(), dgrad.p, 6 * n * sizeof(double), cudaMemcpyDeviceToHost)) != cudaSuccess)
+        return cuda_fail(ctx, e, "gradient download");
+    for (int64_t o = 0; o < n; ++o)
+        for (int j = 0; j < 3; ++j) {
+            grad_r0[o * 3 + j] = g[o * 6 + j];
+            grad_v0[o * 3 + j] = g[o * 6 + 3 + j];
+        }
+    return GPOP_OK;
+}
+
 } // namespace
 
 extern "C" {
@@ -445,13 +508,18 @@ gpop_status gpop_stm(gpop_ctx* ctx, const gpop_time* start, double h, int32_t st
             || (st = begin(ctx, p, start, h, steps, m, dr.as<double>(), dv.as<double>(), s)) != GPOP_OK
             || (st = tan.reserve(ctx, p)) != GPOP_OK)
             return st;
-        const int window = (int)std::min<int64_t>(steps, std::max<int64_t>(1, (int64_t)(kWindowBytes / 120) / m));
+        int window = (int)std::min<int64_t>(steps, std::max<int64_t>(1, (int64_t)(kWindowBytes / 120) / m));
         cudaError_t e;
         if ((e = dphi.ensure(36 * m * sizeof(double))) != cudaSuccess
-            || (e = pos.ensure((size_t)window * 6 * m * sizeof(double))) != cudaSuccess
-            || (e = jac.ensure((size_t)window * 9 * m * sizeof(double))) != cudaSuccess
             || (e = sweep.ensure((size_t)kStmSweep * 6 * m * sizeof(double))) != cudaSuccess)
             return nomem(ctx, "STM buffers", e);
+        while ((e = pos.ensure((size_t)window * 6 * m * sizeof(double))) != cudaSuccess
+            || (e = jac.ensure((size_t)window * 9 * m * sizeof(double))) != cudaSuccess) {
+            if (e != cudaErrorMemoryAllocation || window == 1)
+                return nomem(ctx, "STM buffers", e);
+            cudaGetLastError(); // fewer steps at once
+            window /= 2;
+        }
         int done = std::min(steps, 4);
         if ((st = propagator_step(&p, done, nullptr, nullptr, nullptr, s)) != GPOP_OK || (st = tan.make(ctx, p, s)) != GPOP_OK)
             return st;
@@ -521,58 +589,17 @@ gpop_status gpop_propagate_vjp(gpop_ctx* ctx, const gpop_time* start, double h, 
         }
         return GPOP_OK;
     }
-    cudaStream_t s = nullptr;
-    ScopedBufs B(ctx);
-    DevBuf &dr = B.b[0], &dv = B.b[1], &dr0 = B.b[2], &dv0 = B.b[3], &ck = B.b[4], &traj = B.b[5],
-           &dobj = B.b[6], &dstep = B.b[7], &dseed = B.b[8], &dgrad = B.b[9];
-    StartupTangents tan(ctx);
-    if ((st = upload(ctx, dr, r_in, 3 * n, s)) != GPOP_OK || (st = upload(ctx, dv, v_in, 3 * n, s)) != GPOP_OK
-        || (st = upload(ctx, dr0, r_in, 3 * n, s)) != GPOP_OK || (st = upload(ctx, dv0, v_in, 3 * n, s)) != GPOP_OK)
-        return st;
-    // the positions and accelerations of every step when they fit, else checkpoints
-    const size_t rows = (size_t)steps * 3 * n, traj_bytes = 2 * rows * sizeof(double);
-    const bool store = traj_bytes <= ctx->adjoint_store && traj.ensure(traj_bytes) == cudaSuccess;
-    if (!store)
-        cudaGetLastError(); // a failed allocation
-    gpop_propagator p;
-    if ((st = begin(ctx, p, start, h, steps, n, dr.as<double>(), dv.as<double>(), s)) != GPOP_OK
-        || (n <= kVarObjects && (st = tan.reserve(ctx, p)) != GPOP_OK)
-        || (st = forward_run(ctx, p, steps, store ? traj.as<double>() : nullptr, nullptr,
-                store ? traj.as<double>() + rows : nullptr, ck, s))
-            != GPOP_OK)
-        return st;
-    // seeds on the final state: node 0 at the last step
-    std::vector<int> obj(n), step0(n, steps);
-    std::vector<double> seeds((size_t)n * 27, 0.0);
-    for (int64_t o = 0; o < n; ++o) {
-        obj[o] = (int)o;
-        for (int j = 0; j < 3; ++j) {
-            seeds[o * 27 + j] = r_bar ? r_bar[o * 3 + j] : 0.0;
-            seeds[o * 27 + 3 + j] = v_bar ? v_bar[o * 3 + j] : 0.0;
-        }
+    // the positions and accelerations of every step when they fit, else checkpoints: also where memory runs out
+    // behind them
+    const size_t traj_bytes = (size_t)6 * steps * n * sizeof(double);
+    st = GPOP_ERR_NOMEM;
+    if (traj_bytes <= ctx->adjoint_store)
+        st = run_vjp(ctx, start, h, steps, n, r_in, v_in, r_bar, v_bar, true, grad_r0, grad_v0);
+    if (st == GPOP_ERR_NOMEM) {
+        cudaGetLastError();
+        st = run_vjp(ctx, start, h, steps, n, r_in, v_in, r_bar, v_bar, false, grad_r0, grad_v0);
     }
-    cudaError_t e;
-    if ((e = dobj.ensure(n * sizeof(int))) != cudaSuccess || (e = dstep.ensure(n * sizeof(int))) != cudaSuccess
-        || (e = dgrad.ensure(6 * n * sizeof(double))) != cudaSuccess)
-        return fail(ctx, GPOP_ERR_NOMEM, std::string("adjoint buffers: ") + cudaGetErrorString(e));
-    if ((st = upload(ctx, dseed, seeds.data(), seeds.size(), s)) != GPOP_OK)
-        return st;
-    if ((e = cudaMemcpyAsync(dobj.p, obj.data(), n * sizeof(int), cudaMemcpyHostToDevice, s)) != cudaSuccess
-        || (e = cudaMemcpyAsync(dstep.p, step0.data(), n * sizeof(int), cudaMemcpyHostToDevice, s)) != cudaSuccess)
-        return cuda_fail(ctx, e, "seed upload");
-    if ((st = run_adjoint(ctx, p, steps, dr0.as<double>(), dv0.as<double>(), store ? traj.as<double>() : nullptr,
-             store ? traj.as<double>() + rows : nullptr, ck, tan, step0, obj, dobj.as<int>(), dstep.as<int>(), dseed.as<double>(), dgrad.as<double>(), s))
-        != GPOP_OK)
-        return st;
-    std::vector<double> g(6 * n);
-    if ((e = cudaMemcpy(g.data(), dgrad.p, 6 * n * sizeof(double), cudaMemcpyDeviceToHost)) != cudaSuccess)
-        return cuda_fail(ctx, e, "gradient download");
-    for (int64_t o = 0; o < n; ++o)
-        for (int j = 0; j < 3; ++j) {
-            grad_r0[o * 3 + j] = g[o * 6 + j];
-            grad_v0[o * 3 + j] = g[o * 6 + 3 + j];
-        }
-    return GPOP_OK;
+    return st;
 }
 
 gpop_status gpop_miss_gradient(gpop_ctx* ctx, const gpop_time* start, double h, int32_t steps, int64_t n,
