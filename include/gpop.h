@@ -116,13 +116,22 @@ gpop_status gpop_propagator_step(gpop_propagator* p, int32_t steps, double* traj
     double* traj_a, void* stream);
 /* Steps taken so far. */
 int32_t gpop_propagator_steps_done(const gpop_propagator* p);
-/* No counterpart in the reference. The walk without the column split for n objects on a GPU of num_sms
- * SMs at the given precision, as GPOP_WALK_MODE names the walks (by default a call may take groups of
- * warps or the columns over a block instead where they are faster): 1 = one object per thread, 2 = two objects per
+/* No counterpart in the reference. The gravity walk the propagation calls take for n objects on a GPU of num_sms
+ * SMs at the given precision and degree, when none is forced (GPOP_WALK_MODE) and the sums are not compensated:
+ * 1 = one object per thread, 2 = two objects per thread (in the split block where gpop_split_block says so), 3 =
+ * lanes per object (*lanes_out of them: up to 32 of a warp, or whole warps), 5 = two objects per thread in plain
+ * blocks (above 512 objects per SM: whole waves of these, then the walk of the rest), 6 = columns over the warps
+ * of a block; *lanes_out = 1 but for 3. *fp64_out: whether the terms are those of the FP64 table (always in FP64; in
+ * mixed precision for few objects, where it is the faster one). -1 for invalid arguments. Both outputs may be NULL.
+ * Host arithmetic only, no CUDA call. */
+int32_t gpop_step_walk(int64_t n, int32_t num_sms, int32_t precision, int32_t degree, int32_t* lanes_out,
+    int32_t* fp64_out);
+/* No counterpart in the reference. The walk of n objects among those GPOP_WALK_MODE names, which compensated sums
+ * take by default (1 or 2; others see gpop_step_walk): 1 = one object per thread, 2 = two objects per
  * thread, 3 = lanes per object, 4 = lanes per group of two objects (*lanes_out = the lanes for 3
  * and 4, else 1); -1 for invalid arguments. Host arithmetic only, no CUDA call. */
 int32_t gpop_walk_policy(int64_t n, int32_t num_sms, int32_t precision, int32_t* lanes_out);
-/* No counterpart in the reference. Where the walk is two objects per thread: the owner warps of
+/* No counterpart in the reference. Where the walk is two objects per thread (2 of gpop_step_walk): the owner warps of
  * the split block it launches (8 warps per SM, of which the owners carry the objects and the
  * others walk the low gravity columns of the owners' objects), 5 to 7 when each SM carries 5 to 7
  * sets of 64 objects and the degree is above 8; 0 for the plain block. -1 for invalid arguments.

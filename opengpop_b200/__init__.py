@@ -37,7 +37,7 @@ EXPORTS = (
     "gpop_startup_init", "gpop_startup_correct", "gpop_gj8_predict", "gpop_gj8_correct",
     "gpop_matrix_column", "gpop_gj8_coefficients", "gpop_gravity", "gpop_frame_matrices",
     "gpop_ca_create", "gpop_ca_create_analytic", "gpop_ca_create_external", "gpop_ca_append", "gpop_ca_propagate", "gpop_ca_find", "gpop_ca_pairs", "gpop_ca_num_pairs",
-    "gpop_ca_set_rows", "gpop_ca_pair_range", "gpop_ca_reserve", "gpop_walk_policy", "gpop_split_block", "gpop_ca_trajectory", "gpop_ca_device_seconds", "gpop_ca_destroy",
+    "gpop_ca_set_rows", "gpop_ca_pair_range", "gpop_ca_reserve", "gpop_walk_policy", "gpop_step_walk", "gpop_split_block", "gpop_ca_trajectory", "gpop_ca_device_seconds", "gpop_ca_destroy",
 )
 
 
@@ -132,6 +132,7 @@ def load_library(path=LIB_PATH):
         "gpop_ca_set_rows": (i32, [_VP, i64, i64]),
         "gpop_ca_reserve": (i32, [_VP, i32]),
         "gpop_walk_policy": (i32, [i64, i32, i32, C.POINTER(i32)]),
+        "gpop_step_walk": (i32, [i64, i32, i32, i32, C.POINTER(i32), C.POINTER(i32)]),
         "gpop_split_block": (i32, [i64, i32, i32]),
         "gpop_ca_pair_range": (i32, [_VP, C.POINTER(i64), C.POINTER(i64)]),
         "gpop_ca_trajectory": (i32, [_VP] * 4 + [C.POINTER(i32)]),
@@ -147,11 +148,13 @@ def load_library(path=LIB_PATH):
 
 
 WALKS = {1: "one object per thread", 2: "two objects per thread", 3: "lanes",
-         4: "lanes per group of two objects"}
+         4: "lanes per group of two objects", 5: "two objects per thread, plain blocks",
+         6: "columns over a block's warps"}
 
 
 def walk_policy(n, num_sms=148, precision=FP64):
-    """(walk, lanes per object) the propagation takes for n objects (gpop_walk_policy)."""
+    """(walk, lanes per object) for n objects among the walks GPOP_WALK_MODE names, which compensated sums take
+    by default (gpop_walk_policy); step_walk is what other propagations take."""
     lanes = C.c_int32()
     w = load_library().gpop_walk_policy(int(n), int(num_sms), int(precision), C.byref(lanes))
     if w < 0:
@@ -159,8 +162,18 @@ def walk_policy(n, num_sms=148, precision=FP64):
     return w, lanes.value
 
 
+def step_walk(n, num_sms=148, precision=FP64, degree=70):
+    """(walk, lanes per object, whether of the FP64 table) the propagation takes for n objects (gpop_step_walk)."""
+    lanes, fp64 = C.c_int32(), C.c_int32()
+    w = load_library().gpop_step_walk(int(n), int(num_sms), int(precision), int(degree), C.byref(lanes),
+                                      C.byref(fp64))
+    if w < 0:
+        raise GpopError(1, "invalid arguments to gpop_step_walk")
+    return w, lanes.value, bool(fp64.value)
+
+
 def split_block(n, num_sms=148, degree=70):
-    """Owner warps of the split block two objects per thread take for n objects (0: a plain
+    """Owner warps of the split block two objects per thread (walk 2) take for n objects (0: a plain
     block; gpop_split_block)."""
     s = load_library().gpop_split_block(int(n), int(num_sms), int(degree))
     if s < 0:

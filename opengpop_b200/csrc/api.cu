@@ -481,6 +481,31 @@ int32_t gpop_walk_policy(int64_t n, int32_t num_sms, int32_t precision, int32_t*
     return walk;
 }
 
+int32_t gpop_step_walk(int64_t n, int32_t num_sms, int32_t precision, int32_t degree, int32_t* lanes_out,
+    int32_t* fp64_out)
+{
+    if (n <= 0 || num_sms <= 0 || degree < 0 || (precision != GPOP_FP64 && precision != GPOP_MIXED))
+        return -1;
+    const StepWalk w = step_walk(n, num_sms, degree, precision == GPOP_MIXED);
+    const bool team = w.kind == StepWalk::kTeam;
+    if (lanes_out)
+        *lanes_out = team ? w.P : 1;
+    if (fp64_out)
+        *fp64_out = precision == GPOP_FP64 || (team && w.fp64);
+    switch (w.kind) {
+    case StepWalk::kTeam:
+        return kWalkLanes;
+    case StepWalk::kColumns:
+        return 6;
+    case StepWalk::kOne:
+        return kWalkOneObject;
+    case StepWalk::kTwo:
+        return kWalkTwoObjects;
+    default:
+        return kWalkTwoPlain;
+    }
+}
+
 int32_t gpop_split_block(int64_t n, int32_t num_sms, int32_t degree)
 {
     if (n <= 0 || num_sms <= 0 || degree < 0)

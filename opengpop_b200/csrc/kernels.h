@@ -92,14 +92,24 @@ cudaError_t launch_startup(const TableSrc& ts, const PropArgs& a, int num_sms, c
 enum WalkMode : int {
     kWalkOneObject = 1, kWalkTwoObjects = 2, kWalkLanes = 3, kWalkLanesTwo = 4, kWalkTwoPlain = 5
 };
+// The walk of cnt objects' steps under gravity when none is forced (propagate.cu): P lanes per object of a team
+// (of the FP64 table where fp64), the columns over a block's warps, one or two objects per thread. More than 512
+// objects per SM run as whole waves of kTwoPlain and then as the walk of the rest.
+struct StepWalk {
+    enum Kind { kTeam, kColumns, kOne, kTwo, kTwoPlain } kind = kTwo;
+    int P = 1;
+    bool fp64 = false;
+};
+StepWalk step_walk(int64_t cnt, int num_sms, int L, bool mixed);
 // Lanes per object (1..32, a power of 2): the most that keep n objects in one wave of blocks of at
 // most 384 threads, one per SM.
 int lanes_per_object(int64_t n, int num_sms);
 // Lanes per group of two objects (a power of 2 up to 32) where the default walk carries two objects
 // per lane group, 0 elsewhere.
 int lane_pair_lanes(int64_t n, int num_sms, bool fp64_gravity);
-// The walk launch_gj8 takes for n objects when none is forced (lanes: a lane-layout table is at
-// hand and the force is the gravity model; fp64_gravity: the FP64 build of it).
+// The walk launch_gj8 takes for n objects when none is forced and step_walk does not apply: analytic forces and
+// compensated sums (lanes: a lane-layout table is at hand and the force is the gravity model; fp64_gravity: the FP64
+// build of it). Its bands were measured among the walks of WalkMode.
 int default_walk(int64_t n, int num_sms, bool lanes, bool fp64_gravity);
 // Owner warps of the split block two objects per thread take for n objects (0: a plain block).
 int split_owner_warps(int64_t n, int num_sms, int L);

@@ -1287,12 +1287,7 @@ static cudaError_t launch_lanes_range(const TableSrc& lt, const PropArgs& a0, in
 //         128: 1 3.8 / 4.5, 2p 5.8 / 6.1             320: 2p 7.4 / 7.5, 1 8.2 / 9.6
 // With up to four objects per SM the FP64 table is the faster one in mixed precision too (1 object: 7.2 against
 // 9.1 us): a chain of FP64 terms and one of FP32 terms take turns there.
-struct StepWalk {
-    enum Kind { kTeam, kColumns, kOne, kTwo, kTwoPlain } kind = kTwo;
-    int P = 1;
-    bool fp64 = false;
-};
-static StepWalk step_walk(int64_t cnt, int num_sms, int L, bool mixed)
+StepWalk step_walk(int64_t cnt, int num_sms, int L, bool mixed)
 {
     StepWalk w;
     const int64_t o = (cnt + num_sms - 1) / num_sms;
