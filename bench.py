@@ -341,7 +341,7 @@ def run_batch(args, torch, G, dev):
     if not args.no_tune:
         ctx.tune()
     tune_s = time.perf_counter() - t0
-    lpo, est = ctx.batch_plan(reqs)
+    lanes, on_team, est = ctx.batch_run_plan(reqs)
     sampler = ClockSampler(torch.cuda.current_device())
     for _ in range(args.warmup):
         ctx.propagate_batch(reqs)
@@ -380,7 +380,9 @@ def run_batch(args, torch, G, dev):
                          % (len(all_reqs), SEED),
              "object_steps_per_batch": osteps_all, "l2": "inputs (and state) larger than L2",
              "parallelism": "replicas" if world == 1 else "requests over %d ranks (LPT)" % world,
-             "lanes_per_object_histogram": np.bincount(lpo, minlength=33)[[1, 2, 4, 8, 16, 32]].tolist(),
+             "lanes_per_object_histogram":
+                 np.bincount(lanes[~on_team], minlength=33)[[1, 2, 4, 8, 16, 32]].tolist(),
+             "requests_on_teams": int(on_team.sum()),
              "planner_estimate_s": est, "tune_s": tune_s},
             {"n_gpus": world, "scaling": "strong",
              "ms_per_step": 1e3 * t,

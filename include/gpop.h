@@ -188,11 +188,18 @@ gpop_status gpop_propagate_batch(gpop_ctx* ctx, const gpop_request* reqs, int32_
  * its status for every request that was to run. */
 gpop_status gpop_propagate_batch_status(gpop_ctx* ctx, const gpop_request* reqs, int32_t n_req,
     int32_t* status);
-/* The batch plan: lanes per object chosen for each request and the estimated makespan (s). The
+/* The plan of a batch on the persistent grid alone, before its longest requests move to teams
+ * (gpop_batch_run_plan): lanes per object chosen for each request and the estimated makespan (s). The
  * planner also picks the block shape of the persistent grid (4 or 8 warps per SM), the one with the
  * shorter simulated makespan; gpop_batch_warps_per_sm gives the last planned batch's. */
 gpop_status gpop_batch_plan(gpop_ctx* ctx, const gpop_request* reqs, int32_t n_req,
     int32_t* lanes_per_object, double* est_seconds);
+/* No counterpart in the reference. The plan gpop_propagate_batch runs: on_team[i] = 1 for the requests whose objects
+ * run on teams of warps, on blocks of their own beside the persistent grid; lanes_per_object[i] = the lanes of
+ * the team, or of the request's work items on the SMs left (any value for a request without steps); the planner's
+ * estimate of the makespan (s). Outputs may be NULL. */
+gpop_status gpop_batch_run_plan(gpop_ctx* ctx, const gpop_request* reqs, int32_t n_req,
+    int32_t* lanes_per_object, int32_t* on_team, double* est_seconds);
 /* No counterpart in the reference. Warps per SM (the block shape) of the last planned batch. */
 int32_t gpop_batch_warps_per_sm(const gpop_ctx* ctx);
 /* Device time (s, CUDA events) of the last gpop_propagate_batch launch: frames, startup and the

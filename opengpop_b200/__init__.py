@@ -31,7 +31,7 @@ EXPORTS = (
     "gpop_gravity_degree", "gpop_kernel_launches", "gpop_propagate", "gpop_propagate_device",
     "gpop_propagate_device_noalloc", "gpop_propagate_trajectory", "gpop_propagator_create", "gpop_propagator_step",
     "gpop_propagator_steps_done", "gpop_propagator_destroy", "gpop_propagate_analytic",
-    "gpop_propagate_batch", "gpop_propagate_batch_status", "gpop_batch_plan", "gpop_batch_warps_per_sm", "gpop_tune", "gpop_batch_device_seconds", "gpop_gravity_jacobian", "gpop_stm", "gpop_propagate_vjp",
+    "gpop_propagate_batch", "gpop_propagate_batch_status", "gpop_batch_plan", "gpop_batch_run_plan", "gpop_batch_warps_per_sm", "gpop_tune", "gpop_batch_device_seconds", "gpop_gravity_jacobian", "gpop_stm", "gpop_propagate_vjp",
     "gpop_miss_gradient", "gpop_sample_states", "gpop_startup", "gpop_corrector_unit",
     "gpop_predict_unit", "gpop_finalize_correction_unit", "gpop_rk8_stage", "gpop_rk8_finish",
     "gpop_startup_init", "gpop_startup_correct", "gpop_gj8_predict", "gpop_gj8_correct",
@@ -106,6 +106,7 @@ def load_library(path=LIB_PATH):
         "gpop_propagate_batch": (i32, [_VP, _VP, i32]),
         "gpop_propagate_batch_status": (i32, [_VP, _VP, i32, _VP]),
         "gpop_batch_plan": (i32, [_VP, _VP, i32, _VP, C.POINTER(f64)]),
+        "gpop_batch_run_plan": (i32, [_VP, _VP, i32, _VP, _VP, C.POINTER(f64)]),
         "gpop_tune": (i32, [_VP, C.c_char_p]),
         "gpop_batch_warps_per_sm": (i32, [_VP]),
         "gpop_batch_device_seconds": (f64, [_VP]),
@@ -367,12 +368,24 @@ class Context:
         return load_library().gpop_batch_warps_per_sm(self._h)
 
     def batch_plan(self, reqs):
+        """(lanes per object, estimated seconds) of the persistent grid alone, before the longest requests move to
+        teams (gpop_batch_plan); batch_run_plan is what runs."""
         arr, keep = self._requests(reqs)
         lpo = np.zeros(len(reqs), np.int32)
         est = C.c_double()
         self._check(load_library().gpop_batch_plan(self._h, arr, len(reqs),
                                                    lpo.ctypes.data_as(_VP), C.byref(est)))
         return lpo, est.value
+
+    def batch_run_plan(self, reqs):
+        """(lanes per object, whether on a team, estimated seconds) as propagate_batch runs the requests
+        (gpop_batch_run_plan)."""
+        arr, keep = self._requests(reqs)
+        lanes, team = np.zeros(len(reqs), np.int32), np.zeros(len(reqs), np.int32)
+        est = C.c_double()
+        self._check(load_library().gpop_batch_run_plan(self._h, arr, len(reqs), lanes.ctypes.data_as(_VP),
+                                                       team.ctypes.data_as(_VP), C.byref(est)))
+        return lanes, team.astype(bool), est.value
 
     @property
     def batch_device_seconds(self):

@@ -175,6 +175,7 @@ struct Plan {
     double est = 0.0;
     int warps_per_sm = 8; // block shape of the persistent grid
     std::vector<BatchItem> team_items; // objects that teams take (choose_teams)
+    std::vector<char> on_team; // per request (empty: none)
     int team_blocks = 0, teams_per_block = 0, team_lanes = 0;
 };
 
@@ -239,7 +240,7 @@ void choose_teams(const gpop_ctx* ctx, const std::vector<int64_t>& n, const std:
 {
     if (ctx->force_lpo > 0
         || stage_offset(ctx->lane_table(false)) + kBatchTeamThreads * sizeof(double) > max_smem_optin())
-        return; // (a team needs less than a double per lane beside the table)
+        return; // (beside the table a team takes 28 doubles and 8 per warp, a block of them 104 at most)
     const size_t R = n.size();
     std::vector<size_t> order;
     double load = 0.0; // warp-seconds of the items
@@ -262,6 +263,7 @@ void choose_teams(const gpop_ctx* ctx, const std::vector<int64_t>& n, const std:
     };
     double best = 0.9 * span(0.0, 0, load, 0);
     size_t take = 0;
+    double team_time = 0.0;
     int64_t objects = 0;
     int Lmax = 0;
     for (size_t k = 0; k < order.size(); ++k) {
@@ -282,6 +284,7 @@ void choose_teams(const gpop_ctx* ctx, const std::vector<int64_t>& n, const std:
         if (t < best) {
             best = t;
             take = k + 1;
+            team_time = team;
             p.team_blocks = blocks;
             p.teams_per_block = teams;
             p.team_lanes = lanes;
@@ -290,15 +293,19 @@ void choose_teams(const gpop_ctx* ctx, const std::vector<int64_t>& n, const std:
     if (take == 0)
         return;
     std::vector<int> rest = steps;
+    p.on_team.assign(R, 0);
     for (size_t k = 0; k < take; ++k) {
         rest[order[k]] = 0;
+        p.on_team[order[k]] = 1;
         for (int64_t i = 0; i < n[order[k]]; ++i)
             p.team_items.push_back(BatchItem { (int)order[k], (int)i, 1 });
     }
-    // the others by themselves: lanes for what is the longest now
+    // the others by themselves: lanes for what is the longest now. With the warps of all SMs: counting those of the
+    // teams' SMs out keeps items on fewer lanes (256 requests: 57.2 -> 64.8 ms).
     Plan q = make_plan(ctx, n, rest, L);
     p.lpo = q.lpo;
     p.items = q.items;
+    p.est = std::max(team_time, q.est);
     p.warps_per_sm = q.warps_per_sm;
 }
 
@@ -381,8 +388,7 @@ void destroy_batch_cache(gpop_ctx* ctx)
 
 extern "C" {
 
-gpop_status gpop_batch_plan(gpop_ctx* ctx, const gpop_request* reqs, int32_t n_req,
-    int32_t* lanes_per_object, double* est_seconds)
+static gpop_status plan_batch(gpop_ctx* ctx, const gpop_request* reqs, int32_t n_req, bool teams, Plan& p)
 {
     if (!ctx)
         return GPOP_ERR_INVALID_ARG;
@@ -396,9 +402,40 @@ gpop_status gpop_batch_plan(gpop_ctx* ctx, const gpop_request* reqs, int32_t n_r
         steps[i] = reqs[i].steps;
         L[i] = (reqs[i].degree > 0 && reqs[i].degree < ctx->md.degree) ? reqs[i].degree : ctx->md.degree;
     }
-    Plan p = make_plan(ctx, n, steps, L);
+    p = make_plan(ctx, n, steps, L);
+    if (teams)
+        choose_teams(ctx, n, steps, L, p);
+    return GPOP_OK;
+}
+
+gpop_status gpop_batch_plan(gpop_ctx* ctx, const gpop_request* reqs, int32_t n_req,
+    int32_t* lanes_per_object, double* est_seconds)
+{
+    Plan p;
+    const gpop_status st = plan_batch(ctx, reqs, n_req, false, p);
+    if (st != GPOP_OK)
+        return st;
     if (lanes_per_object)
         std::copy(p.lpo.begin(), p.lpo.end(), lanes_per_object);
+    if (est_seconds)
+        *est_seconds = p.est;
+    return GPOP_OK;
+}
+
+gpop_status gpop_batch_run_plan(gpop_ctx* ctx, const gpop_request* reqs, int32_t n_req,
+    int32_t* lanes_per_object, int32_t* on_team, double* est_seconds)
+{
+    Plan p;
+    const gpop_status st = plan_batch(ctx, reqs, n_req, true, p);
+    if (st != GPOP_OK)
+        return st;
+    for (int32_t i = 0; i < n_req; ++i) {
+        const bool team = !p.on_team.empty() && p.on_team[i];
+        if (lanes_per_object)
+            lanes_per_object[i] = team ? p.team_lanes : p.lpo[i];
+        if (on_team)
+            on_team[i] = team;
+    }
     if (est_seconds)
         *est_seconds = p.est;
     return GPOP_OK;
