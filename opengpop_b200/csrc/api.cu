@@ -179,9 +179,8 @@ gpop_status propagator_step(gpop_propagator* p, int steps, double* traj_r, doubl
     a.col_pos = p->col_pos;
     a.pass_pos = p->pass_pos;
     if (!p->started) {
-        if ((e = launch_startup(ts, a, ctx->num_sms, s, &lane_ts, &lane64)) != cudaSuccess)
+        if ((e = launch_startup(ts, a, ctx->num_sms, s, &lane_ts, &lane64, &ctx->launches)) != cudaSuccess)
             return cuda_fail(ctx, e, "startup kernel");
-        ctx->launches += p->kind == GPOP_FORCE_GRAVITY ? startup_launches(p->ncorr) : 1;
         p->started = true;
     }
     a.traj_r = traj_r;

@@ -81,9 +81,10 @@ size_t max_smem_optin();
 // Kernels of the startup pipeline: the RK8 chains, their columns, two per corrector pass, the end.
 inline int startup_launches(int ncorr) { return 3 + 2 * ncorr; }
 // Startup of a.n objects. Gravity with the state and the lane-layout table at hand runs the pipeline of
-// startup.cu; analytic forces, compensated sums and the unit entry point one thread per object.
+// startup.cu; analytic forces, compensated sums and the unit entry point one thread per object. launches (may be
+// NULL): the kernels launched are added.
 cudaError_t launch_startup(const TableSrc& ts, const PropArgs& a, int num_sms, cudaStream_t s,
-    const TableSrc* lane_ts = nullptr, const TableSrc* lane64 = nullptr);
+    const TableSrc* lane_ts = nullptr, const TableSrc* lane64 = nullptr, int64_t* launches = nullptr);
 // How many objects a GJ8 thread carries through the gravity triangle walk (0 = by problem size).
 // kWalkLanes: P lanes per object split the gravity columns (few objects; P from lanes_per_object).
 // kWalkLanesTwo: P lanes per group of two objects (P from lane_pair_lanes, else 2), the default

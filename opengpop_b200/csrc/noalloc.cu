@@ -136,7 +136,7 @@ extern "C" gpop_status gpop_propagate_device_noalloc(gpop_ctx* ctx, const gpop_t
     a.err = err;
     a.r0 = r_dev;
     a.v0 = v_dev;
-    if ((e = launch_startup(ts, a, ctx->num_sms, s, &lane_ts, &lane64)) != cudaSuccess)
+    if ((e = launch_startup(ts, a, ctx->num_sms, s, &lane_ts, &lane64, &ctx->launches)) != cudaSuccess)
         return cuda_fail(ctx, e, "startup kernel");
     const int chunk = ctx->steps_per_launch;
     for (int b = 1; b <= steps; b += chunk) {
@@ -150,7 +150,7 @@ extern "C" gpop_status gpop_propagate_device_noalloc(gpop_ctx* ctx, const gpop_t
             != cudaSuccess)
             return cuda_fail(ctx, e, "GJ8 kernel");
     }
-    ctx->launches += 2 + startup_launches(ctx->cfg.n_corrections) + (steps + chunk - 1) / chunk;
+    ctx->launches += 2 + (steps + chunk - 1) / chunk;
     unsigned word = 0;
     if ((e = cudaMemcpyAsync(&word, err, sizeof(unsigned), cudaMemcpyDeviceToHost, s)) != cudaSuccess
         || (e = cudaStreamSynchronize(s)) != cudaSuccess)

@@ -1011,12 +1011,15 @@ template <class K> static cudaError_t set_smem(K kernel, size_t bytes)
 }
 
 cudaError_t launch_startup(const TableSrc& ts, const PropArgs& a, int num_sms, cudaStream_t s,
-    const TableSrc* lane_ts, const TableSrc* lane64)
+    const TableSrc* lane_ts, const TableSrc* lane64, int64_t* launches)
 {
     if (a.n <= 0)
         return cudaSuccess;
-    if (a.kind == 0 && a.state && lane_ts && !a.out27[0] && a.ncorr >= 1 && a.ncorr <= kStartupCounters
-        && !(ts.mixed && (a.flags & kFlagMixedCompensated))) {
+    const bool pipeline = a.kind == 0 && a.state && lane_ts && !a.out27[0] && a.ncorr >= 1 && a.ncorr <= kStartupCounters
+        && !(ts.mixed && (a.flags & kFlagMixedCompensated));
+    if (launches)
+        *launches += pipeline ? startup_launches(a.ncorr) : 1;
+    if (pipeline) {
         StartupArgs b;
         b.n = a.n;
         b.h = a.h;
