@@ -1790,3 +1790,23 @@ extern "C" void or_stm_ld(const void* dv, const or_time* st, double h, int32_t s
                 = (double)((8 * (y[0][j] - y[1][j]) - (y[2][j] - y[3][j])) / (12 * d));
     }
 }
+
+extern "C" void or_propagate_ld(const void* dv, const or_time* st, double h, int32_t steps, int32_t ncorr, int64_t n,
+    const double* r0, const double* v0, double* rf, double* vf)
+{
+    using LD = long double;
+    const Force f = make_force(dv, OR_FORCE_GRAVITY, st, h, steps, 0);
+#pragma omp parallel for schedule(dynamic, 1)
+    for (int64_t i = 0; i < n; ++i) {
+        LD x[6], y[6];
+        for (int j = 0; j < 3; ++j) {
+            x[j] = r0[3 * i + j];
+            x[3 + j] = v0[3 * i + j];
+        }
+        propagate_one<LD>(f, steps, ncorr, x, x + 3, n, i, nullptr, nullptr, nullptr, y, y + 3);
+        for (int j = 0; j < 3; ++j) {
+            rf[3 * i + j] = (double)y[j];
+            vf[3 * i + j] = (double)y[3 + j];
+        }
+    }
+}

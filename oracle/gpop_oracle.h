@@ -153,6 +153,9 @@ int32_t or_miss_fd(const void* data, const or_time* start, double h, int32_t ste
 /* ---- extended precision (long double), for the errors of 64-bit results ----
  * Accelerations at Earth-fixed positions r (n x 3): each value as hi + lo. */
 void or_gravity_ld(const void* data, int64_t n, const double* r, double* hi, double* lo);
+/* Final states of the propagation of n objects under gravity, rounded to double. */
+void or_propagate_ld(const void* data, const or_time* start, double h, int32_t steps, int32_t ncorr, int64_t n,
+    const double* r0, const double* v0, double* rf, double* vf);
 /* State transition matrices [n][6][6] of the propagation with its ncorr passes, by fourth-order central
  * differences (100 m and 0.1 m/s, twice these; rounding and remainder near 1e-14 of a block). */
 void or_stm_ld(const void* data, const or_time* start, double h, int32_t steps, int32_t ncorr, int64_t n,

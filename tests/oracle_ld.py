@@ -25,3 +25,14 @@ def stm(data, start, h, steps, r, v, ncorr=7):
     fn.argtypes = [C.c_void_p, C.POINTER(O.OrTime), C.c_double, C.c_int32, C.c_int32, C.c_int64] + [C.c_void_p] * 3
     fn(data.h, C.byref(O.tstruct(start)), h, steps, ncorr, r.shape[0], O.ptr(r), O.ptr(v), O.ptr(phi))
     return phi
+
+
+def propagate(data, start, h, steps, r, v, ncorr=7):
+    """Final positions and velocities [n, 3] of the propagation with ncorr passes, rounded to double."""
+    r, v = O.f64(r), O.f64(v)
+    rf, vf = np.zeros_like(r), np.zeros_like(r)
+    fn = O.lib().or_propagate_ld
+    fn.restype = None
+    fn.argtypes = [C.c_void_p, C.POINTER(O.OrTime), C.c_double, C.c_int32, C.c_int32, C.c_int64] + [C.c_void_p] * 4
+    fn(data.h, C.byref(O.tstruct(start)), h, steps, ncorr, r.shape[0], O.ptr(r), O.ptr(v), O.ptr(rf), O.ptr(vf))
+    return rf, vf
