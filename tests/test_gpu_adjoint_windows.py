@@ -37,3 +37,19 @@ def test_one_run_per_segment():
         assert (np.abs(a - b).max(axis=1) <= 1e-9 * np.abs(b).max(axis=1)).all()
     assert np.isfinite(gr).all() and np.isfinite(gv).all()
 
+
+
+def test_matrices_in_pieces():
+    import opengpop_b200 as G
+    from opengpop_b200 import orbits
+    n, steps = 65536 + 300, 12
+    r, v = orbits.mixed_population(n, seed=9)
+    pick = np.array([0, 1, 65535, 65536, n - 1])  # on either side of the pieces
+    ctx = G.Context(gravity_degree=8)
+    got = ctx.stm(START, 30.0, steps, r, v)
+    few = ctx.stm(START, 30.0, steps, r[pick], v[pick])
+    ctx.close()
+    for a, b in zip(got, few):  # other kernels for other counts, as above
+        a, b = a[pick].reshape(len(pick), -1), b.reshape(len(pick), -1)
+        assert (np.abs(a - b).max(axis=1) <= 1e-9 * np.abs(b).max(axis=1)).all()
+    assert all(np.isfinite(x).all() for x in got)
