@@ -195,7 +195,7 @@ gpop_status propagator_step(gpop_propagator* p, int steps, double* traj_r, doubl
         const bool last = a.step_end == end;
         a.out_r = last ? p->r : nullptr;
         a.out_v = last ? p->v : nullptr;
-        if ((e = launch_gj8(ts, a, ctx->num_sms, s, ctx->block_override, ctx->walk_mode, &lane_ts,
+        if ((e = launch_gj8(ts, a, ctx->num_sms, s, ctx->walk_mode, &lane_ts,
                  &lane64))
             != cudaSuccess)
             return cuda_fail(ctx, e, "GJ8 kernel");

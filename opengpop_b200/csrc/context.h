@@ -166,7 +166,6 @@ struct gpop_ctx {
     gpop::ColumnPlan plan64, plan_mixed;
     int num_sms = 148;
     int steps_per_launch = 64;
-    int block_override = 0; // GJ8 block size chosen by the tuner (0 = default policy)
     // largest trajectory (bytes) the adjoint keeps whole; above, segments are run again from checkpoints
     // (GPOP_ADJOINT_STORE_MB, read when a context is made)
     size_t adjoint_store = (size_t)32 << 30;

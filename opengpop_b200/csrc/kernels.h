@@ -116,7 +116,7 @@ int default_walk(int64_t n, int num_sms, bool lanes, bool fp64_gravity);
 int split_owner_warps(int64_t n, int num_sms, int L);
 // lane_ts: the lane-layout table of the same precision (NULL: no lane-split walk), lane64: the FP64 one.
 cudaError_t launch_gj8(const TableSrc& ts, const PropArgs& a, int num_sms, cudaStream_t s,
-    int block_override = 0, int walk = 0, const TableSrc* lane_ts = nullptr, const TableSrc* lane64 = nullptr);
+    int walk = 0, const TableSrc* lane_ts = nullptr, const TableSrc* lane64 = nullptr);
 // The same steps with the columns split over the warps of one block per SM (columns.cu): at most 512
 // objects per SM, degree >= 2.
 cudaError_t launch_gj8_columns(const TableSrc& lane_ts, const PropArgs& a, int num_sms, cudaStream_t s);

@@ -145,7 +145,7 @@ extern "C" gpop_status gpop_propagate_device_noalloc(gpop_ctx* ctx, const gpop_t
         const bool last = a.step_end == steps + 1;
         a.out_r = last ? r_dev : nullptr;
         a.out_v = last ? v_dev : nullptr;
-        if ((e = launch_gj8(ts, a, ctx->num_sms, s, ctx->block_override, ctx->walk_mode, &lane_ts,
+        if ((e = launch_gj8(ts, a, ctx->num_sms, s, ctx->walk_mode, &lane_ts,
                  &lane64))
             != cudaSuccess)
             return cuda_fail(ctx, e, "GJ8 kernel");

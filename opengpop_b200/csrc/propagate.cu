@@ -1092,12 +1092,12 @@ int split_owner_warps(int64_t n, int num_sms, int L)
 
 template <class F, int K>
 static cudaError_t launch_gj8_k(F f, const TableSrc& ts, const PropArgs& a, int num_sms,
-    cudaStream_t s, int block_override, bool split = true)
+    cudaStream_t s, bool split = true)
 {
     const int64_t cnt = (a.obj_hi < 0 ? a.n : a.obj_hi) - a.obj_lo; // objects of this launch
     if constexpr (K == 2 && F::kTable) {
         if constexpr (!F::kComp) {
-            const int S = block_override > 0 || !split ? 0 : split_owner_warps(cnt, num_sms, ts.L);
+            const int S = !split ? 0 : split_owner_warps(cnt, num_sms, ts.L);
             if (S > 0) {
                 PropArgs b = a;
                 b.split_owners = S;
@@ -1127,10 +1127,6 @@ static cudaError_t launch_gj8_k(F f, const TableSrc& ts, const PropArgs& a, int 
     }
     const int64_t threads = (cnt + K - 1) / K;
     LaunchShape ls = pick_shape(threads, K == 1 ? kOneObjectBlock : 256, num_sms);
-    if (block_override > 0) {
-        ls.block = block_override;
-        ls.grid = (int)((threads + block_override - 1) / block_override);
-    }
     if constexpr (F::kTable) {
         // the corrector state is parked in shared memory when it fits beside the table
         const size_t staged = stage_offset(ts) + (size_t)kStageDoubles * K * 8 * ls.block;
@@ -1154,11 +1150,11 @@ static cudaError_t launch_gj8_k(F f, const TableSrc& ts, const PropArgs& a, int 
 
 template <class F>
 static cudaError_t launch_gj8_f(F f, const TableSrc& ts, const PropArgs& a, int num_sms,
-    cudaStream_t s, int block_override, int walk)
+    cudaStream_t s, int walk)
 {
     if (walk == kWalkTwoObjects || walk == kWalkTwoPlain)
-        return launch_gj8_k<F, 2>(f, ts, a, num_sms, s, block_override, walk == kWalkTwoObjects);
-    return launch_gj8_k<F, 1>(f, ts, a, num_sms, s, block_override);
+        return launch_gj8_k<F, 2>(f, ts, a, num_sms, s, walk == kWalkTwoObjects);
+    return launch_gj8_k<F, 1>(f, ts, a, num_sms, s);
 }
 
 // The most lanes that keep every object in one wave of blocks of at most kLanesBlock threads,
@@ -1327,14 +1323,14 @@ StepWalk step_walk(int64_t cnt, int num_sms, int L, bool mixed)
 }
 
 cudaError_t launch_gj8(const TableSrc& ts, const PropArgs& a, int num_sms, cudaStream_t s,
-    int block_override, int walk, const TableSrc* lane_ts, const TableSrc* lane64)
+    int walk, const TableSrc* lane_ts, const TableSrc* lane64)
 {
     // objects [lo, hi) of the n the state holds
     const int64_t lo = a.obj_lo, hi = a.obj_hi < 0 ? a.n : a.obj_hi, cnt = hi - lo;
     if (cnt <= 0 || lo < 0 || hi > a.n || a.step_end <= a.step_begin)
         return cudaSuccess;
     const bool forced = walk > 0;
-    if (walk <= 0 && a.kind == 0 && lane_ts && block_override <= 0
+    if (walk <= 0 && a.kind == 0 && lane_ts
         && !(ts.mixed && (a.flags & kFlagMixedCompensated))) {
         const StepWalk w = step_walk(cnt, num_sms, ts.L, ts.mixed);
         switch (w.kind) {
@@ -1360,10 +1356,10 @@ cudaError_t launch_gj8(const TableSrc& ts, const PropArgs& a, int num_sms, cudaS
         ForceGravity<true, true> f {};
         f.gen_m = a.gen_m;
         f.prop_m = a.prop_m;
-        return launch_gj8_f(f, ts, a, num_sms, s, block_override,
+        return launch_gj8_f(f, ts, a, num_sms, s,
             walk == kWalkTwoObjects || walk == kWalkTwoPlain ? walk : kWalkOneObject);
     }
-    if (walk == kWalkTwoObjects && a.kind == 0 && block_override <= 0) {
+    if (walk == kWalkTwoObjects && a.kind == 0) {
         // More objects than one wave of 8 warps per SM holds at two per thread: whole waves of
         // 256-thread blocks, then the rest with the walk its own size takes (100,000 objects ran as
         // two waves of 169-thread blocks, 6 warps per SM spread 2-2-1-1).
@@ -1372,12 +1368,12 @@ cudaError_t launch_gj8(const TableSrc& ts, const PropArgs& a, int num_sms, cudaS
             const int64_t full = cnt / wave * wave;
             PropArgs b = a;
             b.obj_hi = lo + full;
-            cudaError_t e = launch_gj8(ts, b, num_sms, s, block_override, kWalkTwoPlain, lane_ts, lane64);
+            cudaError_t e = launch_gj8(ts, b, num_sms, s, kWalkTwoPlain, lane_ts, lane64);
             if (e != cudaSuccess || full == cnt)
                 return e;
             PropArgs c = a;
             c.obj_lo = lo + full;
-            return launch_gj8(ts, c, num_sms, s, block_override, forced ? walk : 0, lane_ts, lane64);
+            return launch_gj8(ts, c, num_sms, s, forced ? walk : 0, lane_ts, lane64);
         }
     }
     if ((walk == kWalkLanes || walk == kWalkLanesTwo) && a.kind == 0 && lane_ts) {
@@ -1418,15 +1414,15 @@ cudaError_t launch_gj8(const TableSrc& ts, const PropArgs& a, int num_sms, cudaS
             ForceGravity<true> f {};
             f.gen_m = a.gen_m;
             f.prop_m = a.prop_m;
-            return launch_gj8_f(f, ts, a, num_sms, s, block_override, walk);
+            return launch_gj8_f(f, ts, a, num_sms, s, walk);
         }
         ForceGravity<false> f {};
         f.gen_m = a.gen_m;
         f.prop_m = a.prop_m;
-        return launch_gj8_f(f, ts, a, num_sms, s, block_override, walk);
+        return launch_gj8_f(f, ts, a, num_sms, s, walk);
     }
     ForceAnalytic f { a.kind, a.h };
-    return launch_gj8_f(f, ts, a, num_sms, s, block_override, walk);
+    return launch_gj8_f(f, ts, a, num_sms, s, walk);
 }
 
 cudaError_t launch_gravity(const TableSrc& ts, int64_t n, const double* r, const double* m9,
