@@ -39,8 +39,8 @@ METRIC = "object-steps/s @70x70: mixed vs FP64 at <=1 m/7 d err; conj pairs/s"
 UNIT = "object-steps/s"
 
 # Algorithmic work (FMA = 2 flops): gravity evaluation W(L) = 24 T(L) + 15 L + 60, T(L) the number
-# of (n, m) terms with 2 <= n <= L; an object-step is 7 distinct evaluations plus ~500 flops of
-# GJ8 predictor/corrector arithmetic.
+# of (n, m) terms with 2 <= n <= L; an object-step is EVALUATIONS of them plus ~500 flops of GJ8
+# predictor/corrector arithmetic.
 def terms(L):
     return (L + 1) * (L + 2) // 2 - 3
 
@@ -59,9 +59,9 @@ def fp32_flops_per_object_step(L=DEGREE):
 
 
 # DRAM bytes (read + write) of one mixed GJ8 launch over 65,536 objects (the split block), from an
-# ncu capture (dram__bytes_read.sum 20.66 MB, dram__bytes_write.sum 0;
-# profiles/gj8_kernels_65536obj_70x70.md).
-MIXED_GJ8_DRAM_BYTES = 20.66e6
+# ncu capture (dram__bytes_read.sum 39.50 MB, dram__bytes_write.sum 0;
+# profiles/step_startup_screen_kernels.md).
+MIXED_GJ8_DRAM_BYTES = 39.50e6
 
 
 def env_int(k, d):
@@ -513,10 +513,9 @@ def run_adjoint(args, torch, G, dev):
     launches = ctx.kernel_launches - launches0
     ctx.close()
     tm, ts = float(np.mean(t_miss)), float(np.mean(t_stm))
-    # work of the miss-gradient call: forward propagation of 2 n_pairs objects, then per unit
-    # (pair side) a recomputed forward pass (7 W + 500 per step), the reverse pass (one Jacobian
-    # per step) and the tangent startup (145 Jacobian evaluations); of the STM: the primal step,
-    # one Jacobian and six tangent steps per object-step
+    # work of the miss-gradient call: forward propagation of 2 n_pairs objects, per unit (pair side) one
+    # Jacobian per step for the reverse pass and 89 of the startup (80 RK8 stages, nine columns); of the
+    # STM: the primal step, one Jacobian and six tangent steps per object-step
     W = 24 * terms(DEGREE) + 15 * DEGREE + 60
     units = 2 * n_pairs
     f_miss = units * steps * (flops_per_object_step() + w_jac(DEGREE)) + units * 89 * w_jac(DEGREE)
@@ -528,8 +527,8 @@ def run_adjoint(args, torch, G, dev):
         cpu = {"value": rate, "unit": "pairs/s", "cores": cores, "kind": "port", "sample": desc}
     ach = f_miss / tm / 1e12
     _common(args, "miss-distance gradients/s (adjoint, FP64)", n_pairs / tm, "pairs/s", "f64",
-            {"workload": "%d LEO pairs (seed %d), 70x70, 30 s, %d steps (24 h), checkpoint every 64 "
-                         "steps; %d STMs over the same span" % (n_pairs, SEED, steps, n_stm)},
+            {"workload": "%d LEO pairs (seed %d), 70x70, 30 s, %d steps (24 h), trajectory "
+                         "stored; %d STMs over the same span" % (n_pairs, SEED, steps, n_stm)},
             {"ms_per_step": 1e3 * tm,
              "stm": {"value": n_stm * steps / ts, "unit": "object-steps/s (with 6x6 STM)",
                      "seconds": ts, "roofline_frac": (f_stm / ts / 1e12) / peak64 if peak64 else None},
@@ -537,8 +536,8 @@ def run_adjoint(args, torch, G, dev):
                      "d2h_bytes_per_step": n_pairs * 14 * 8, "call": "gpop_miss_gradient"},
              "roofline": {"bound": "fp64", "achieved": ach, "peak": peak64, "unit": "TFLOP/s",
                           "frac": ach / peak64 if peak64 else None, "traffic": None,
-                          "per_unit": "per unit-step 2 (7 W + 500) + W_J, W(70) = %d, "
-                                      "W_J(70) = %d flops" % (W, w_jac(DEGREE))},
+                          "per_unit": "per unit-step %d W + 500 + W_J, W(70) = %d, "
+                                      "W_J(70) = %d flops" % (EVALUATIONS, W, w_jac(DEGREE))},
              "cpu_baseline": cpu, "clocks": clocks, "gpu_launches": launches})
     return 0
 
@@ -911,7 +910,7 @@ def main():
                          "traffic": MIXED_GJ8_DRAM_BYTES,
                          "traffic_note": "a stated constant, not measured in this run: dram "
                                          "read+write bytes of one launch of this kernel from an "
-                                         "ncu capture (65,536 objects, 4-step launch; the state "
+                                         "ncu capture (65,536 objects, 8-step launch; the state "
                                          "is read once per launch, later steps hit L2); "
                                          "algorithmic state bytes per launch %d" % (600 * n),
                          "peak_note": "not in MEASURED_PEAKS.json (HBM and bf16 only): SMs x "

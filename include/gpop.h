@@ -213,8 +213,8 @@ gpop_status gpop_tune(gpop_ctx* ctx, const char* cache_path);
 
 /* ---- variational equations and adjoint (FP64; the reference has no counterpart) ----
  * Derivatives of the discrete propagation map of gpop_propagate in FP64 (RK8 startup + GJ8 with
- * the context's corrector passes, gravity at every iterate), with respect to the initial GCRS
- * state x0 = (r0, v0). Host buffers. */
+ * the context's corrector passes), with respect to the initial GCRS state x0 = (r0, v0): exact through the
+ * startup; a step's passes with one Jacobian, at the position of its last evaluation. Host buffers. */
 /* Gravity acceleration (a_dev may be NULL) and its Jacobian jac_dev [n][3][3] = d a_i / d r_j at
  * GCRS positions r_dev [n][3] with frame matrix frame9_dev (as gpop_gravity; NULL = identity).
  * FP64, device buffers. */
@@ -224,9 +224,10 @@ gpop_status gpop_gravity_jacobian(gpop_ctx* ctx, int64_t n, const double* r_dev,
  * stm[i][j] = d x_N,i / d x0_j with x = (r, v); r_out, v_out (may be NULL) = the final state. */
 gpop_status gpop_stm(gpop_ctx* ctx, const gpop_time* start, double h, int32_t steps, int64_t n,
     const double* r_in, const double* v_in, double* r_out, double* v_out, double* stm_out);
-/* Vector-Jacobian product by the adjoint (reverse) sweep, GJ8 state checkpointed every 64
- * steps: grad_r0, grad_v0 [n][3] = d(sum r_bar . r_N + v_bar . v_N) / d(r0, v0). r_bar or v_bar
- * may be NULL (zero). */
+/* Vector-Jacobian product by the adjoint (reverse) sweep: grad_r0, grad_v0 [n][3] = d(sum r_bar . r_N +
+ * v_bar . v_N) / d(r0, v0). r_bar or v_bar may be NULL (zero). The sweep goes over the stored trajectory (48 bytes
+ * per object and step) up to 32 GB, another limit by GPOP_ADJOINT_STORE_MB when the context is made; above it, or
+ * where the device's memory does not take it, GJ8 states are kept every 64 steps and the segments run again. */
 gpop_status gpop_propagate_vjp(gpop_ctx* ctx, const gpop_time* start, double h, int32_t steps,
     int64_t n, const double* r_in, const double* v_in, const double* r_bar, const double* v_bar,
     double* grad_r0, double* grad_v0);

@@ -5,7 +5,7 @@
 // eight totals of an object are added through shared memory, and the thread that owns the object assembles
 // the acceleration and corrects. So
 // - a table entry is read once per warp and broadcast to 64 objects (lanes that walk different columns read
-//   one entry each, and shared memory is what they wait on);
+//   one entry each);
 // - all warps have the same work whatever the number of objects (two objects per thread fill 8 warps at 512
 //   objects per SM only, and at 64 objects per SM one);
 // - a set whose objects are all done takes no part in the next corrector pass.
@@ -14,10 +14,13 @@
 // An object's corrector state lies in shared memory for up to 64 objects per block, else in its state arrays
 // (L2): nothing of it is held through the walks, which have the registers to themselves.
 //
-// Bounds: the FP64 (mixed: FMA) pipe. Measured on B200, 70x70 FP64 / mixed, us per step against the best of the other
-// walks: 2,368 objects 18.6 / 15.3 (24.7 / 19.4), 9,472: 40.6 / 25.1 (51.5 / 42.0), 18,944: 78.7 / 45.7
-// (91 / 66), 37,888: 152 / 87 (156 / 96); two evaluations of a set take 70,500 of its 80,300 cycles, the FP64
-// pipe 72 % busy in them. From 6 sets on, two objects per thread are as good or better: no barriers there.
+// Bounds: dependent FMAs with two warps per scheduler, then the FP64 (mixed: FMA) pipe. Captured at 70x70, FP64: 17
+// objects per SM (the pair's lanes) FP64 pipe 52 % busy, shared-memory loads 37 % of their port, waits per issued
+// instruction 1.35 on fixed latency, 0.87 at barriers, 0.70 on the pipe; 64 and 128 per SM 62 % and 63 %, 46 %, 1.3,
+// 0.3 to 0.5, 0.85; mixed at 128 per SM FMA pipe 30 %, 40 %. Measured on B200, 70x70 FP64 / mixed, us per step
+// against the best of the other walks: 2,368 objects 18.6 / 15.3 (24.7 / 19.4), 9,472: 40.6 / 25.1 (51.5 / 42.0),
+// 18,944: 78.7 / 45.7 (91 / 66), 37,888: 152 / 87 (156 / 96); two evaluations of a set take 70,500 of its 80,300
+// cycles. From 6 sets on, two objects per thread are as good or better: no barriers there.
 #include "common.cuh"
 #include "corrector.cuh"
 #include "gj8_tables.cuh"

@@ -58,9 +58,10 @@ struct CorrJacobian {
 // Bounds a propagation (every other cost is per evaluation). Evaluations of a step by a warp of 64
 // objects, which waits for the slowest: 7 as the method states them; 4.0 when passes end on equal
 // bits alone (LEO and the mixed population at 30 s; 4.5 at 60 s); 2.7 with the central term for J
-// and eight last bits for `near`; 2.0 with J2 and `near` as here. Position error after 1,500 steps of
-// 30 s against an 80-bit propagation, rms of 24 LEO objects: 1.00e-6 m with seven passes, 0.98e-6 m
-// with this rule (60 s, 1,440 steps: 1.99e-6 and 1.49e-6). 18,501 objects, 240 steps, FP64, the call:
+// and eight last bits for `near`; 2.0 with J2 and `near` as here. Position error against a long double
+// propagation, rms of 160 LEO objects after 1,000 steps, seven passes / this rule: 10 s 2.49e-7 / 2.23e-7 m, 30 s
+// 5.35e-7 / 5.77e-7, 60 s 1.13e-6 / 1.05e-6 (the sums of rounded accelerations; such figures scatter by 6 %; the
+// tests hold them to the oracle's seven passes). 18,501 objects, 240 steps, FP64, the call:
 // 85.6 -> 30.2 ms; 65,536 mixed, 320 steps: 147.2 -> 54.5 ms.
 //
 // it, ncorr: this pass and the passes of the method. fast: kept by the caller between the passes of

@@ -2,7 +2,7 @@
 // (lane l of P takes m = l, l + P, ...); the per-object sums are added with warp shuffles among
 // the lanes named by `mask` (the whole warp, or the object's aligned group of P lanes), so every
 // lane of the object ends with the same result. Used where one object per thread leaves
-// the GPU idle: long single requests of a batch and the variational/adjoint kernels. The tables
+// the GPU idle: calls with few objects, long requests of a batch, Jacobians of few points. The tables
 // are in the lane layout (build_lane_blob), so the lanes' simultaneous reads of different columns
 // fall in different shared-memory banks.
 #pragma once

@@ -105,7 +105,7 @@ struct ForceAnalytic {
     }
 };
 
-constexpr int kLanesBlock = 384; // threads per SM the lane walks are spread to
+constexpr int kLanesBlock = 384; // threads per SM the forced lane walk is spread to (lanes_per_object)
 
 // ---- table staging ----
 size_t table_smem_bytes(const TableSrc& ts) { return 128 + (size_t)ts.bytes; }
@@ -1157,11 +1157,9 @@ static cudaError_t launch_gj8_f(F f, const TableSrc& ts, const PropArgs& a, int 
     return launch_gj8_k<F, 1>(f, ts, a, num_sms, s);
 }
 
-// The most lanes that keep every object in one wave of blocks of at most kLanesBlock threads,
-// so that the lane kernel runs with the registers of its 384-thread variant: fewer lanes with
-// more registers beat more lanes with 128 (B200, 70x70, FP64 / mixed M object-steps/s: 2,048
-// objects 19.0 / 26.1 against 16.2 / 21.2 with 512-thread blocks; 4,096: 25.6 / 36.1 against
-// 21.8 / 33.6; 9,472: 31.6 / 49.4 against 29.6 / 46.5; 16,000: 42.2 / 63.7 against 30.2 / 53.1).
+// The most lanes that keep every object within kLanesBlock threads per SM. Of a forced lane walk (GPOP_WALK_MODE=3)
+// only: default calls take step_walk's lanes. The kernel's blocks have at most 256 threads (kTeamBlock), so at 257
+// to 384 threads per SM a forced walk runs in two waves; the count is kept as gpop_walk_policy reports it.
 int lanes_per_object(int64_t n, int num_sms)
 {
     int P = 1;
@@ -1181,7 +1179,8 @@ int lanes_per_object(int64_t n, int num_sms)
 //          8,000: 62.4 (8) / 44.3      9,472: 69.5 (8) / 50.0    12,000: 59.4 (4) / 50.9
 //         18,944: 88.3 (4) / 73.0     20,000: 73.5 (4) / 68.4
 //                                     outside: 2,048: 29.5 (16) / 29.0; 24,000: 76.0 (2) / 81.8
-// P is the most lanes whose groups fit one wave of 8 warps per SM, doubled once, up to 8 lanes,
+// (Seven evaluations per step, as the method states them; default calls take the walks of step_walk, and this one
+// is forced with GPOP_WALK_MODE=4.) P is the most lanes whose groups fit one wave of 8 warps per SM, doubled once, up to 8 lanes,
 // when the groups still fit one and a half waves (FP64) or 1.2 waves (mixed); the groups past one
 // wave run in a second launch with more lanes. Before the staging, FP64 12,000 objects ran at 41.6
 // with 8 lanes against 38.7 with 4, and 6,000 at 34.4 with 8 against 31.4 with 16; staged, mixed
@@ -1200,7 +1199,8 @@ int lane_pair_lanes(int64_t n, int num_sms, bool fp64_gravity)
     return P;
 }
 
-// Default walk (measured on B200 at 70x70, LEO objects, mixed / FP64 M object-steps/s):
+// Walk among those of WalkMode where step_walk does not apply (compensated sums, analytic forces): the lines below
+// were measured with seven evaluations per step (B200, 70x70, LEO objects, mixed / FP64 M object-steps/s):
 // - up to 128 objects per SM, lanes (P from lanes_per_object, blocks of at most 384 threads):
 //   18,900 objects 74.7 / 49.4 against 65.0 / 47.0 with two lanes per pair of objects; 9,472:
 //   49.4 / 31.6 against 34.0 / 20.8 with two objects per thread;

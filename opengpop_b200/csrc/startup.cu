@@ -13,7 +13,8 @@
 //   reach it, so two rounds of evaluations serve for seven: 93 evaluations per object instead of 145.
 // Bounds: the gravity walk for many objects, its latency times 45 for few. Measured on B200 at 70x70, the
 // whole startup, one thread per object (65,536: the split block) -> here: 1 object FP64 5.88 -> 0.19 ms;
-// 18,501 FP64 7.8 -> 4.0 ms; 65,536 mixed 14.1 -> 6.3 ms.
+// 18,501 FP64 7.8 -> 4.0 ms; 65,536 mixed 14.1 -> 6.3 ms. Captured, RK8 chains of 18,501 objects, FP64 at one per
+// thread (3.2 ms): shared-memory loads at 91 % of their port, FP64 pipe 62 % busy.
 #include "common.cuh"
 #include "corrector.cuh"
 #include "gj8_tables.cuh"
